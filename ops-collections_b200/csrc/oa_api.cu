@@ -70,7 +70,7 @@ struct b2co_oa_table {
     uint64_t stage_keys = 0;
     cudaStream_t pipe[kHostSlots] = {};
     cudaEvent_t ev[kHostSlots + 1] = {};  // per-stream completion, then the caller's start
-    uint32_t find_lanes = 0, find_items = 0;
+    uint32_t find_lanes = 0, find_items = 0;  // lookup shape; 0: chosen by table size and batch (oa_inst.cuh)
 };
 
 namespace {
@@ -92,42 +92,6 @@ int check_batch(uint64_t n)
 }
 
 cudaStream_t cs(b2co_stream s) { return reinterpret_cast<cudaStream_t>(s); }
-
-// Default lookup shape per layout; b2co_oa_set_find_shape overrides it per table.
-// Tables at most this large (about 2.5 times the 126 MB L2) are served mostly
-// from L2, and the keys in flight per warp set their rate: measured on int64
-// tables, two-lane lookups beat four-lane ones by 1.39x at 70 MB, 1.17x at 130 MB
-// and 1.21x at 260 MB and lose by 8% at 520 MB; one-lane-per-key writes win by
-// 1.7x at 70 and 130 MB and 1.45x at 260 MB and lose by 11% at 520 MB.
-constexpr uint64_t kSmallTableBytes = uint64_t(320) << 20;
-
-uint64_t table_bytes(b2co_oa_table const* t)
-{
-    return uint64_t(t->capacity) * slot_bytes(t->desc.key_bytes, t->desc.value_bytes);
-}
-bool small_table(b2co_oa_table const* t) { return table_bytes(t) <= kSmallTableBytes; }
-
-// Writes to small tables run one lane per key (the reference's scan as
-// written); larger tables take the cooperative default.
-void default_write_shape(b2co_oa_table* t) { t->args.write_shape = small_table(t) ? (1u << 8) | 1u : 0u; }
-
-void default_shape(b2co_oa_table* t)
-{
-    if (t->desc.bucket_size == 1) {
-        t->find_lanes = 1;  // a one-slot window needs no cooperation
-        t->find_items = 4;
-    } else {
-        // keys staged per warp, keys that probe on past their first window
-        // queued and followed a pass at a time; four lanes per window (a 64-byte
-        // row of 16-byte slots per load) with two windows in flight, or two
-        // lanes and one window for 4-byte slots and for small tables (measured
-        // best per layout and size, see kSmallTableBytes)
-        uint32_t const sb = slot_bytes(t->desc.key_bytes, t->desc.value_bytes);
-        bool const narrow = sb <= 4 || small_table(t);
-        t->find_lanes = narrow ? 2 : 4;
-        t->find_items = (narrow ? 1 : 2) | kShapeDeferred;
-    }
-}
 
 unsigned int* status_word(b2co_oa_table* t) { return reinterpret_cast<unsigned int*>(t->d_counters + 2); }
 
@@ -259,8 +223,6 @@ int b2co_oa_create_ex(b2co_oa_desc const* d, uint64_t requested, bool clear, b2c
     t->ops = oa_ops_for(d->key_bytes, d->value_bytes, d->key_kind);
     t->capacity = cap;
     cudaGetDevice(&t->device);
-    default_shape(t);
-    default_write_shape(t);
 
     uint32_t nb = uint32_t(cap / d->bucket_size);
     ProbeParams& p = t->args.probe;
@@ -274,7 +236,8 @@ int b2co_oa_create_ex(b2co_oa_desc const* d, uint64_t requested, bool clear, b2c
     t->args.empty_value = d->value_bytes ? t->desc.empty_value_bits : 0;
     t->args.erased_key = t->desc.erased_key_bits;
 
-    cudaError_t e = cudaMalloc(&t->args.slots, cap * slot_bytes(d->key_bytes, d->value_bytes));
+    // whole 32-byte sectors: kernels read the sectors that a window covers
+    cudaError_t e = cudaMalloc(&t->args.slots, (cap * slot_bytes(d->key_bytes, d->value_bytes) + 31) / 32 * 32);
     // counters: [failed, assigned, status word]
     if (e == cudaSuccess) e = cudaMalloc(&t->d_counters, 3 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemset(t->d_counters, 0, 3 * sizeof(unsigned long long));
@@ -658,7 +621,7 @@ int b2co_oa_set_find_shape(b2co_oa_table* t, uint32_t lanes, uint32_t items)
 {
     if (int st = check_table(t)) return st;
     if (lanes == 0 && items == 0) {
-        default_shape(t);
+        t->find_lanes = t->find_items = 0;
         return B2CO_OK;
     }
     if (lanes != 1 && lanes != 2 && lanes != 4 && lanes != 8) return fail(B2CO_EINVAL, "lanes must be 1, 2, 4 or 8");
@@ -673,7 +636,7 @@ int b2co_oa_set_write_shape(b2co_oa_table* t, uint32_t lanes, uint32_t keys_per_
 {
     if (int st = check_table(t)) return st;
     if (lanes == 0 && keys_per_tile == 0) {
-        default_write_shape(t);
+        t->args.write_shape = 0;
         return B2CO_OK;
     }
     if (lanes != 1 && lanes != 2 && lanes != 4 && lanes != 8) return fail(B2CO_EINVAL, "lanes must be 1, 2, 4 or 8");

@@ -28,22 +28,9 @@
 // bounded number of times), so no kernel can spin.
 #pragma once
 
-#include "oa_kernels.cuh"
+#include "oa_sector.cuh"
 
 namespace b2co {
-
-enum { kInsPlain = 0, kInsAssign = 1, kInsIafRace = 2, kInsIafPlace = 3 };
-
-// Outputs of one insert-family launch (only the mode's fields are used).
-struct InsOut {
-    unsigned long long* counters;  // plain/assign: [failed, assigned] or NULL (async)
-    void* found;                   // race: payload found or inserted
-    uint8_t* inserted;             // race: 1 = this input inserted the key
-    uint32_t* pos;                 // place: slot of every input (kNoSlot = failed)
-    uint32_t* newbits;             // place: slots claimed by this batch
-    uint32_t* owner;               // place: claiming input of each claimed slot (claim_bit 0 only)
-    uint32_t claim_bit;            // place: flag OR-ed into pos[] of the claiming input (0 = none)
-};
 
 // Coherent window loads (L2, never a stale L1 line) with the 64-byte fill hint.
 __device__ __forceinline__ uint32_t ld_win(uint32_t const* p)
@@ -389,8 +376,8 @@ __global__ void __launch_bounds__(256, kWriteMinBlocks<Q>) k_insert_win(__grid_c
     while (count > 0) follow();
     if constexpr (MODE == kInsPlain || MODE == kInsAssign) {
         if (o.counters) {
-            warp_add_counter(o.counters, failed);
-            if (MODE == kInsAssign) warp_add_counter(o.counters + 1, assigned);
+            block_add_counter(o.counters, failed);
+            if (MODE == kInsAssign) block_add_counter(o.counters + 1, assigned);
         }
     }
 }

@@ -10,6 +10,36 @@
 
 namespace b2co {
 
+// Which kernels a table takes by default (no shape set), by measurement with
+// half-full tables and 50% hits on one B200 (both kernels, same box):
+//
+// Lookups.  The one-lane sector kernel (oa_sector.cuh) asks L2 for a window
+// sector by sector.  Where most sectors are in L2 that is the cheapest form, but
+// HBM serves about 37 G missed requests a second however many are in flight, so
+// on large tables the tiled kernels, which ask for a window in one or two
+// requests, win.  16 M queries, sector / 2 lanes / 4 lanes x 2 in Gkeys/s:
+//   16-byte slots: 40 MB 70 / 66 / 42, 120 MB 47 / 40 / 33, 220 MB 38 / 34 / 31, 300 MB 26 / 33 / 30
+//   8-byte slots:  20 MB 97 / 83 / 51, 160 MB 57 / 50 / 35, 300 MB 36 / 46 / 33
+//   4-byte slots:  40 MB 72 / 93 / 59: two lanes read such a window in fewer instructions
+// A small batch is bound by the length of its chain of loads, not by requests,
+// whatever the table: on a 1 GB table, sector / 4 lanes x 2 take 4.8 / 6.9 us for
+// 16,384 keys, 8.9 / 10.1 for 65,536 and 13.6 / 12.1 for 131,072.
+constexpr uint64_t kSectorFindBytes = uint64_t(224) << 20;
+constexpr uint32_t kSectorFindKeys = 3u << 15;
+// Two lanes and one window in flight against four and two: 34 / 31 at 220 MB,
+// 33 / 30 at 300 MB, 27 / 29 at 520 MB.
+constexpr uint64_t kNarrowFindBytes = uint64_t(320) << 20;
+// Writes.  The same trade with a CAS or a store behind every window, sector / 4
+// lanes in Gpairs/s: Insert 300 MB 18.9 / 15.8, 400 MB 14.9 / 15.7; InsertOrAssign of
+// present keys 220 MB 22.5 / 19.4, 300 MB 17.9 / 18.8.
+constexpr uint64_t kSectorInsertBytes = uint64_t(352) << 20;
+constexpr uint64_t kSectorAssignBytes = uint64_t(256) << 20;
+// Threads per block of the sector kernels: a batch that does not fill the GPU is
+// spread over more SMs in smaller blocks (an SM takes its windows' requests one
+// after the other): 1,000 keys take 3.8 us in blocks of 64 and 4.8 in blocks of 256.
+constexpr uint32_t kSpreadKeys = 1u << 17;
+inline uint32_t sector_block(uint32_t n) { return n <= kSpreadKeys ? 64 : 256; }
+
 template <class S>
 struct OaImpl {
     static constexpr uint32_t kBlock = 256;
@@ -45,9 +75,37 @@ struct OaImpl {
         return check_launch("clear kernel");
     }
 
-    // Whether the insert family runs one key per lane (the scan of
-    // open_addressing_ref_impl.h:489-532 as written) instead of a tile per window.
-    static bool per_key_writes(OaArgs const& a, int B) { return B == 1 || (a.write_shape >> 8) == 1; }
+    static uint64_t table_bytes(OaArgs const& a) { return uint64_t(a.probe.capacity) * S::bytes; }
+
+    // Whether the insert family runs one key per lane (oa_sector.cuh) instead of
+    // a tile per window (oa_insert.cuh).
+    static bool sector_writes(OaArgs const& a, int B, int mode)
+    {
+        uint32_t const lanes = a.write_shape >> 8;
+        return B == 1 || lanes == 1 ||
+               (lanes == 0 && table_bytes(a) <= (mode == kInsAssign ? kSectorAssignBytes : kSectorInsertBytes));
+    }
+
+    template <int B, int MODE>
+    static int launch_sector_write(OaArgs const& a, void const* pairs, uint8_t const* stencil, uint32_t n,
+                                   InsOut const& o, cudaStream_t s)
+    {
+        auto k = k_insert_sector<S, B, MODE>;
+        uint32_t const block = sector_block(n);
+        k<<<grid_for((void const*)k, block, n, block), block, 0, s>>>(a, pairs, stencil, n, o);
+        return check_launch("insert kernel");
+    }
+
+    // A write of one mode: the sector kernel, or the table's cooperative shape.
+    template <int B, int MODE>
+    static int write(OaArgs const& a, void const* pairs, uint8_t const* stencil, uint32_t n, InsOut const& o,
+                     cudaStream_t s)
+    {
+        if constexpr (B > 1) {
+            if (!sector_writes(a, B, MODE)) return launch_write<B, MODE>(a, pairs, stencil, n, o, s);
+        }
+        return launch_sector_write<B, MODE>(a, pairs, stencil, n, o, s);
+    }
 
     // Cooperative-window write kernel (oa_insert.cuh) of the table's shape.
     template <int B, int MODE>
@@ -74,17 +132,10 @@ struct OaImpl {
     {
         return with_b(b, [&](auto bc) {
             constexpr int B = decltype(bc)::value;
-            if constexpr (B > 1) {
-                if (!per_key_writes(a, B)) {
-                    InsOut o{};
-                    o.counters = counters;
-                    return assign ? launch_write<B, kInsAssign>(a, pairs, stencil, n, o, s)
-                                  : launch_write<B, kInsPlain>(a, pairs, stencil, n, o, s);
-                }
-            }
-            auto k = assign ? k_insert<S, B, true> : k_insert<S, B, false>;
-            k<<<grid_for((void const*)k, kBlock, n, kBlock), kBlock, 0, s>>>(a, pairs, stencil, n, counters);
-            return check_launch("insert kernel");
+            InsOut o{};
+            o.counters = counters;
+            return assign ? write<B, kInsAssign>(a, pairs, stencil, n, o, s)
+                          : write<B, kInsPlain>(a, pairs, stencil, n, o, s);
         });
     }
 
@@ -104,17 +155,10 @@ struct OaImpl {
     {
         return with_b(b, [&](auto bc) {
             constexpr int B = decltype(bc)::value;
-            if constexpr (B > 1) {
-                if (!per_key_writes(a, B)) {
-                    InsOut o{};
-                    o.found = found;
-                    o.inserted = inserted;
-                    return launch_write<B, kInsIafRace>(a, pairs, nullptr, n, o, s);
-                }
-            }
-            auto k = k_iaf_race<S, B>;
-            k<<<grid_for((void const*)k, kBlock, n, kBlock), kBlock, 0, s>>>(a, pairs, found, inserted, n);
-            return check_launch("insert_and_find kernel");
+            InsOut o{};
+            o.found = found;
+            o.inserted = inserted;
+            return write<B, kInsIafRace>(a, pairs, nullptr, n, o, s);
         });
     }
 
@@ -127,23 +171,12 @@ struct OaImpl {
             // batch, then shared with later inputs of the batch (`dup`)
             uint32_t* dup = newbits + (uint64_t(a.probe.capacity) + 31) / 32;
             uint32_t const claim_bit = a.probe.capacity < kClaimBit ? kClaimBit : 0u;  // slot indices below 2^31 - 1
-            bool placed = false;
-            if constexpr (B > 1) {
-                if (!per_key_writes(a, B)) {
-                    InsOut o{};
-                    o.pos = pos;
-                    o.newbits = newbits;
-                    o.owner = owner;
-                    o.claim_bit = claim_bit;
-                    if (int st = launch_write<B, kInsIafPlace>(a, pairs, nullptr, n, o, s)) return st;
-                    placed = true;
-                }
-            }
-            if (!placed) {
-                auto k1 = k_iaf_place<S, B>;
-                k1<<<grid_for((void const*)k1, kBlock, n, kBlock), kBlock, 0, s>>>(a, pairs, n, pos, newbits, owner,
-                                                                                    claim_bit);
-            }
+            InsOut o{};
+            o.pos = pos;
+            o.newbits = newbits;
+            o.owner = owner;
+            o.claim_bit = claim_bit;
+            if (int st = write<B, kInsIafPlace>(a, pairs, nullptr, n, o, s)) return st;
             auto const grid = [&](void const* k) { return grid_for(k, kBlock, (uint64_t(n) + 3) / 4, kBlock); };
             k_iaf_min<S><<<grid((void const*)k_iaf_min<S>), kBlock, 0, s>>>(pos, newbits, dup, owner, n, claim_bit);
             if (claim_bit)
@@ -195,18 +228,60 @@ struct OaImpl {
         return check_launch(C ? "contains kernel" : "find kernel");
     }
 
+    using DeferFn = void (*)(OaArgs, void const*, void*, uint32_t, uint32_t, WaitCtl);
+
+    // Keys per warp and stage: the batch dealt evenly over the resident warps in
+    // stages of at most kWarpStageKeys, so a batch that cannot fill every warp's
+    // stage still reaches every warp (a stage is a chain of dependent passes:
+    // 65,536 keys in whole stages ran 16 of them one after the other on 32 blocks,
+    // 16.1 us against 10.1).
+    static int launch_wdefer(DeferFn k, bool contains, OaArgs const& a, void const* keys, void* out, uint32_t n,
+                             WaitCtl wc, cudaStream_t s)
+    {
+        uint64_t const warps = uint64_t(grid_for((void const*)k, kBlock, ~0ull, 1)) * (kBlock / 32);
+        uint64_t const share = (n + warps - 1) / warps;
+        uint64_t const rounds = (share + kWarpStageKeys - 1) / kWarpStageKeys;
+        uint64_t const chunk = ((share + rounds - 1) / rounds + 31) / 32 * 32;
+        k<<<grid_for((void const*)k, kBlock, (n + chunk - 1) / chunk, kBlock / 32), kBlock, 0, s>>>(
+            a, keys, out, n, uint32_t(chunk), wc);
+        return check_launch(contains ? "contains kernel" : "find kernel");
+    }
+
     template <int B, int G, bool C>
     static int find_wdefer(OaArgs const& a, uint32_t items, void const* keys, void* out, uint32_t n, WaitCtl wc,
                            cudaStream_t s)
     {
-        void (*k)(OaArgs, void const*, void*, uint32_t, WaitCtl) = nullptr;
+        DeferFn k = nullptr;
         if (items >= 4 && G >= 4) k = k_find_wdefer<S, B, G, (G >= 4 ? 4 : 1), C>;
         else if (items >= 2) k = k_find_wdefer<S, B, G, 2, C>;
         else k = k_find_wdefer<S, B, G, 1, C>;
-        uint64_t warps = (n + kWarpStageKeys - 1) / kWarpStageKeys;
-        uint32_t grid = grid_for((void const*)k, kBlock, warps ? warps : 1, kBlock / 32);
-        k<<<grid, kBlock, 0, s>>>(a, keys, out, n, wc);
+        return launch_wdefer(k, C, a, keys, out, n, wc, s);
+    }
+
+    template <int B, bool C>
+    static int find_sector(OaArgs const& a, void const* keys, uint8_t const* stencil, void* out, uint32_t n,
+                           cudaStream_t s)
+    {
+        auto k = k_find_sector<S, B, C>;
+        uint32_t const block = sector_block(n);
+        k<<<grid_for((void const*)k, block, n, block), block, 0, s>>>(a, keys, stencil, out, n);
         return check_launch(C ? "contains kernel" : "find kernel");
+    }
+
+    // The lookup of a table without a shape of its own (lanes 0); see
+    // kSectorFindBytes.
+    template <int B, bool C>
+    static int find_auto(OaArgs const& a, void const* keys, uint8_t const* stencil, void* out, uint32_t n, WaitCtl wc,
+                         cudaStream_t s)
+    {
+        if constexpr (B > 1) {
+            if ((table_bytes(a) > kSectorFindBytes || S::bytes <= 4) && n > kSectorFindKeys) {
+                bool const narrow = S::bytes <= 4 || table_bytes(a) <= kNarrowFindBytes;
+                return find_shape<B, C>(a, narrow ? 2 : 4, (narrow ? 1 : 2) | kShapeDeferred, keys, stencil, out, n, wc,
+                                        s);
+            }
+        }
+        return find_sector<B, C>(a, keys, stencil, out, n, s);
     }
 
     template <int B, bool C>
@@ -232,10 +307,10 @@ struct OaImpl {
         }
     }
 
-    // The default lookup shapes only (layouts without kAllShapes): per-warp
-    // staging with deferred continuations, 2 or 4 lanes per window, one or two
-    // windows in flight; the ballot tile (stencils, unaligned key streams) or
-    // one lane per key (bucket size 1) otherwise.
+    // The shapes of layouts without kAllShapes: per-warp staging with deferred
+    // continuations, 2 or 4 lanes per window, one or two windows in flight; the
+    // ballot tile (stencils, unaligned key streams) or one lane per key (bucket
+    // size 1) otherwise.
     template <int B, bool C>
     static int find_default(OaArgs const& a, uint32_t lanes, uint32_t items, void const* keys,
                             uint8_t const* stencil, void* out, uint32_t n, WaitCtl wc, cudaStream_t s)
@@ -244,18 +319,14 @@ struct OaImpl {
                             B > 1 && lanes >= 2;
         uint32_t const q = (items & ~(kShapeDeferred | kShapeWarpStaged | kShapeSegmented | kShapeBulk)) >= 2 ? 2 : 1;
         if (staged) {
-            void (*k)(OaArgs, void const*, void*, uint32_t, WaitCtl) = nullptr;
+            DeferFn k = nullptr;
             if (lanes == 2) k = q == 2 ? k_find_wdefer<S, B, 2, 2, C> : k_find_wdefer<S, B, 2, 1, C>;
             else k = q == 2 ? k_find_wdefer<S, B, 4, 2, C> : k_find_wdefer<S, B, 4, 1, C>;
-            uint64_t warps = (n + kWarpStageKeys - 1) / kWarpStageKeys;
-            k<<<grid_for((void const*)k, kBlock, warps ? warps : 1, kBlock / 32), kBlock, 0, s>>>(a, keys, out, n, wc);
-            return check_launch(C ? "contains kernel" : "find kernel");
+            return launch_wdefer(k, C, a, keys, out, n, wc, s);
         }
-        void (*k)(OaArgs, void const*, uint8_t const*, void*, uint32_t) = nullptr;
-        uint64_t per_block = kBlock;
-        if (B == 1 || lanes <= 1) k = k_find_lane<S, B, 1, C>;
-        else if (lanes == 2) k = k_find_tile<S, B, 2, C>, per_block /= 2;
-        else k = k_find_tile<S, B, 4, C>, per_block /= 4;
+        if (B == 1 || lanes <= 1) return find_sector<B, C>(a, keys, stencil, out, n, s);
+        uint64_t const per_block = lanes == 2 ? kBlock / 2 : kBlock / 4;
+        auto k = lanes == 2 ? k_find_tile<S, B, 2, C> : k_find_tile<S, B, 4, C>;
         k<<<grid_for((void const*)k, kBlock, n, per_block), kBlock, 0, s>>>(a, keys, stencil, out, n);
         return check_launch(C ? "contains kernel" : "find kernel");
     }
@@ -315,20 +386,9 @@ struct OaImpl {
         }
         items &= ~kShapeWarpStaged;
         items &= ~kShapeSegmented;
-        void (*k)(OaArgs, void const*, uint8_t const*, void*, uint32_t) = nullptr;
-        uint64_t per_block = kBlock;
-        if (B == 1 || lanes <= 1) {
-            if (items >= 4) k = k_find_lane<S, B, 4, C>, per_block *= 4;
-            else if (items == 2) k = k_find_lane<S, B, 2, C>, per_block *= 2;
-            else k = k_find_lane<S, B, 1, C>;
-        } else if (lanes == 2) {
-            k = k_find_tile<S, B, 2, C>, per_block /= 2;
-        } else if (lanes == 4) {
-            k = k_find_tile<S, B, 4, C>, per_block /= 4;
-        } else {
-            k = k_find_tile<S, B, 8, C>, per_block /= 8;
-        }
-        k<<<grid_for((void const*)k, kBlock, n, per_block), kBlock, 0, s>>>(a, keys, stencil, out, n);
+        if (B == 1 || lanes <= 1) return find_sector<B, C>(a, keys, stencil, out, n, s);
+        auto k = lanes == 2 ? k_find_tile<S, B, 2, C> : lanes == 4 ? k_find_tile<S, B, 4, C> : k_find_tile<S, B, 8, C>;
+        k<<<grid_for((void const*)k, kBlock, n, kBlock / lanes), kBlock, 0, s>>>(a, keys, stencil, out, n);
         return check_launch(C ? "contains kernel" : "find kernel");
     }
 
@@ -337,6 +397,9 @@ struct OaImpl {
     {
         return with_b(b, [&](auto bc) {
             constexpr int B = decltype(bc)::value;
+            if (lanes == 0)
+                return contains ? find_auto<B, true>(a, keys, stencil, out, n, wc, s)
+                                : find_auto<B, false>(a, keys, stencil, out, n, wc, s);
             return contains ? find_shape<B, true>(a, lanes, items, keys, stencil, out, n, wc, s)
                             : find_shape<B, false>(a, lanes, items, keys, stencil, out, n, wc, s);
         });

@@ -174,29 +174,19 @@ __device__ __forceinline__ void warp_add_counter(unsigned long long* counter, ui
     if ((threadIdx.x & 31) == 0 && sum) atomicAdd(counter, (unsigned long long)sum);
 }
 
-// counters[0] += failed, counters[1] += assigned (NULL counters = async form).
-template <class S, int B, bool ASSIGN>
-__global__ void __launch_bounds__(256) k_insert(__grid_constant__ const OaArgs a, void const* pairs, uint8_t const* stencil, uint32_t n,
-                                                unsigned long long* counters)
+// The whole block's sum with one atomic: a counter is one address, and its atomics
+// queue up at L2 (one per warp of a full grid is 6,000 of them).  Every thread of
+// the block calls it once.
+__device__ __forceinline__ void block_add_counter(unsigned long long* counter, uint32_t v)
 {
-    uint32_t failed = 0, assigned = 0;
-    uint32_t const stride = gridDim.x * blockDim.x;
-    // warp-uniform trip count so the counter reduction sees every lane
-    for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += stride) {
-        uint32_t i = base + (threadIdx.x & 31);
-        if (i < n && (!stencil || stencil[i])) {
-            typename S::Raw p = Io<S>::load_pair(pairs, i);
-            int r = insert_one<S, B, ASSIGN>(a, S::key(p), S::value(p));
-            // Insert succeeds only on SUCCESS (open_addressing_ref_impl.h:282-285), so a
-            // duplicate is a failure; InsertOrAssign counts it as an assignment instead.
-            failed += ASSIGN ? r == kFailed : r != kSuccess;
-            assigned += r == kDuplicate;
-        }
-    }
-    if (counters) {
-        warp_add_counter(counters, failed);
-        if (ASSIGN) warp_add_counter(counters + 1, assigned);
-    }
+    __shared__ unsigned int total;
+    if (threadIdx.x == 0) total = 0;
+    __syncthreads();
+    uint32_t const sum = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(&total, sum);
+    __syncthreads();
+    if (threadIdx.x == 0 && total) atomicAdd(counter, (unsigned long long)total);
+    __syncthreads();  // `total` may serve another counter next
 }
 
 // AssignIf (Assign, open_addressing_ref_impl.h:384-410): payload overwrite of
@@ -234,61 +224,6 @@ __global__ void __launch_bounds__(256) k_assign_if(__grid_constant__ const OaArg
 }
 
 // ----------------------------------------------------------------------------
-// InsertAndFind, race mode: exactly the reference's concurrent semantics
-// (open_addressing_ref_impl.h:301-330, 543-565); duplicates in one batch race.
-// ----------------------------------------------------------------------------
-
-template <class S, int B>
-__global__ void __launch_bounds__(256) k_iaf_race(__grid_constant__ const OaArgs a, void const* pairs, void* out_found,
-                                                  uint8_t* out_inserted, uint32_t n)
-{
-    using Raw = typename S::Raw;
-    Raw* slots = reinterpret_cast<Raw*>(a.slots);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        Raw p = Io<S>::load_pair(pairs, i);
-        uint64_t key = S::key(p), val = S::value(p);
-        uint64_t found = empty_payload<S>(a);
-        uint8_t inserted = 0;
-        if (key != a.empty_key) {
-            uint32_t const init = probe_init<S::key_bytes, B>(a.probe, key);
-            uint32_t idx = init, step = 0;
-            bool done = false;
-            while (!done) {
-#pragma unroll
-                for (int j = 0; j < B; ++j) {
-                    if (done) break;
-                    Raw* sp = slots + idx + j;
-                    Raw cur = ld_rw(sp);
-                    uint64_t k = S::key(cur);
-                    if (S::key_eq(k, key)) {
-                        found = S::value(settle<S>(a, sp, cur));
-                        done = true;
-                    } else if (k == a.empty_key) {
-                        Raw expected;
-                        if (!insert_expected<S>(a, cur, expected)) continue;
-                        Raw old = cas_slot(sp, expected, insert_desired<S>(cur, key, val));
-                        if (raw_eq(old, expected)) {
-                            found = S::is_set ? key : val;
-                            inserted = 1;
-                            done = true;
-                        } else if (S::key_eq(S::key(old), key)) {
-                            found = S::value(old);
-                            done = true;
-                        }
-                    }
-                }
-                if (done) break;
-                if (step == 0) step = probe_step<S::key_bytes, B>(a.probe, key);
-                idx = probe_next(idx, step, a.probe.capacity);
-                if (idx == init) break;
-            }
-        }
-        Io<S>::store_payload(out_found, i, found);
-        out_inserted[i] = inserted;
-    }
-}
-
-// ----------------------------------------------------------------------------
 // InsertAndFind, first-wins mode: deterministic, equal to inserting the batch
 // sequentially in input order (the golden of tests/common/golden.h:104-131).
 // When the table has fewer than 2^31 slots, pos[i] of the input that claimed a
@@ -318,58 +253,6 @@ __global__ void __launch_bounds__(256) k_iaf_race(__grid_constant__ const OaArgs
 
 constexpr uint32_t kClaimBit = 0x80000000u;
 constexpr uint32_t kNoOwner = 0xffffffffu;
-
-template <class S, int B>
-__global__ void __launch_bounds__(256) k_iaf_place(__grid_constant__ const OaArgs a, void const* pairs, uint32_t n, uint32_t* pos,
-                                                   uint32_t* newbits, uint32_t* owner, uint32_t claim_bit)
-{
-    using Raw = typename S::Raw;
-    Raw* slots = reinterpret_cast<Raw*>(a.slots);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        Raw p = Io<S>::load_pair(pairs, i);
-        uint64_t key = S::key(p), val = S::value(p);
-        uint32_t where = kNoSlot;
-        if (key != a.empty_key) {
-            uint32_t const init = probe_init<S::key_bytes, B>(a.probe, key);
-            uint32_t idx = init, step = 0;
-            bool done = false;
-            while (!done) {
-#pragma unroll
-                for (int j = 0; j < B; ++j) {
-                    if (done) break;
-                    Raw* sp = slots + idx + j;
-                    Raw cur = ld_rw(sp);
-                    uint64_t k = S::key(cur);
-                    if (S::key_eq(k, key)) {
-                        where = idx + j;
-                        done = true;
-                    } else if (k == a.empty_key) {
-                        Raw expected;
-                        if (!insert_expected<S>(a, cur, expected)) continue;
-                        Raw old = cas_slot(sp, expected, insert_desired<S>(cur, key, val));
-                        if (raw_eq(old, expected)) {
-                            where = idx + j;
-                            atomicOr(newbits + (where >> 5), 1u << (where & 31));
-                            if (!claim_bit) owner[where] = i;
-                            where |= claim_bit;
-                            done = true;
-                        } else if (S::key_eq(S::key(old), key)) {
-                            where = idx + j;
-                            done = true;
-                        }
-                    }
-                }
-                if (done) break;
-                if (step == 0) step = probe_step<S::key_bytes, B>(a.probe, key);
-                idx = probe_next(idx, step, a.probe.capacity);
-                if (idx == init) break;
-            }
-        }
-        pos[i] = where;
-    }
-}
-
-__device__ __forceinline__ bool bit_set(uint32_t const* bits, uint32_t s) { return (bits[s >> 5] >> (s & 31)) & 1u; }
 
 // The passes after placement take four inputs a thread: one 16-byte load of
 // their pos[] entries, then each dependent step (bitmap word, owner entry,
@@ -576,51 +459,6 @@ __device__ __noinline__ bool find_rest(OaArgs const& a, uint64_t key, uint32_t i
     }
     payload = empty_payload<S>(a);
     return false;
-}
-
-// One lane per key, ITEMS keys per lane in flight: all windows are loaded
-// before any is resolved, so a lane keeps ITEMS * B independent loads open.
-template <class S, int B, int ITEMS, bool CONTAINS>
-__global__ void __launch_bounds__(256) k_find_lane(__grid_constant__ const OaArgs a, void const* keys, uint8_t const* stencil, void* out,
-                                                   uint32_t n)
-{
-    using Raw = typename S::Raw;
-    Raw const* slots = reinterpret_cast<Raw const*>(a.slots);
-    uint32_t const stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x; base < n; base += stride * ITEMS) {
-        uint64_t key[ITEMS];
-        uint32_t init[ITEMS];
-        bool live[ITEMS];
-        Raw w[ITEMS][B];
-#pragma unroll
-        for (int t = 0; t < ITEMS; ++t) {
-            uint32_t i = base + t * stride;
-            live[t] = i < n && (!stencil || stencil[i]);
-            key[t] = live[t] ? Io<S>::load_key(keys, i) : 0;
-            init[t] = live[t] ? probe_init<S::key_bytes, B>(a.probe, key[t]) : 0;
-        }
-#pragma unroll
-        for (int t = 0; t < ITEMS; ++t)
-            if (live[t]) load_window<S, B>(slots, init[t], w[t]);
-#pragma unroll
-        for (int t = 0; t < ITEMS; ++t) {
-            uint32_t i = base + t * stride;
-            if (i >= n) continue;
-            uint64_t payload = empty_payload<S>(a);
-            bool hit = false;
-            if (live[t]) {
-                Raw stop;
-                if (scan_window<S, B>(w[t], key[t], a.empty_key, stop)) {
-                    hit = S::key(stop) != a.empty_key;
-                    if (hit) payload = S::value(stop);
-                } else {
-                    hit = find_rest<S, B>(a, key[t], init[t], payload);
-                }
-            }
-            if constexpr (CONTAINS) reinterpret_cast<uint8_t*>(out)[i] = hit;
-            else Io<S>::store_payload(out, i, payload);
-        }
-    }
 }
 
 // G lanes per key: lane r of a tile loads slots r, r+G, ... of the window; the
@@ -1147,7 +985,7 @@ __device__ __forceinline__ int tile_first_stop(typename S::Raw const (&w)[ROUNDS
 
 template <class S, int B, int G, int Q, bool CONTAINS>
 __global__ void __launch_bounds__(256, B2CO_WDEFER_MINB(Q)) k_find_wdefer(__grid_constant__ const OaArgs a, void const* keys, void* out,
-                                                        uint32_t n, WaitCtl wc)
+                                                        uint32_t n, uint32_t chunk, WaitCtl wc)
 {
     static_assert(Q <= G && G <= 8 && (G & (G - 1)) == 0, "tile shape");
     using Raw = typename S::Raw;
@@ -1158,7 +996,7 @@ __global__ void __launch_bounds__(256, B2CO_WDEFER_MINB(Q)) k_find_wdefer(__grid
     static_assert(kWarpStageKeys % PASS == 0, "stage must hold whole passes");
     static_assert(2 * PASS <= kDeferRing, "the ring must hold a pass on top of a partial one");
     constexpr uint32_t RING = kDeferRing - 1;
-    constexpr uint32_t kChunkBytes = kWarpStageKeys * sizeof(Key);
+    uint32_t const chunk_bytes = chunk * uint32_t(sizeof(Key));  // chunk: a multiple of 32 keys, at most kWarpStageKeys
     __shared__ alignas(128) Key sk[8][2][kWarpStageKeys];
     __shared__ alignas(8) uint64_t bar[8][2];
     __shared__ alignas(8) uint64_t never[8];
@@ -1171,7 +1009,7 @@ __global__ void __launch_bounds__(256, B2CO_WDEFER_MINB(Q)) k_find_wdefer(__grid
     uint32_t const r = lane % G, tile_lane0 = lane & ~uint32_t(G - 1), tile = lane / G;
     uint32_t const gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     uint32_t const nwarps = (gridDim.x * blockDim.x) >> 5;
-    uint32_t const chunks = n / kWarpStageKeys;
+    uint32_t const chunks = n / chunk;
     Key const* kin = static_cast<Key const*>(keys);
     uint32_t head = 0, count = 0;  // queue state, the same on every lane
 
@@ -1249,8 +1087,8 @@ __global__ void __launch_bounds__(256, B2CO_WDEFER_MINB(Q)) k_find_wdefer(__grid
         mbar_init(&never[warp], 1);
         fence_mbar_init();
         if (gwarp < chunks) {
-            mbar_arrive_expect_tx(&bar[warp][0], kChunkBytes);
-            bulk_g2s(sk[warp][0], kin + uint64_t(gwarp) * kWarpStageKeys, kChunkBytes, &bar[warp][0]);
+            mbar_arrive_expect_tx(&bar[warp][0], chunk_bytes);
+            bulk_g2s(sk[warp][0], kin + uint64_t(gwarp) * chunk, chunk_bytes, &bar[warp][0]);
         }
     }
     __syncwarp();
@@ -1261,8 +1099,8 @@ __global__ void __launch_bounds__(256, B2CO_WDEFER_MINB(Q)) k_find_wdefer(__grid
         uint32_t const cn = c + nwarps;
         if (lane == 0 && cn < chunks) {
             fence_proxy_async();  // the warp's reads of this buffer (previous chunk) precede the copy
-            mbar_arrive_expect_tx(&bar[warp][b ^ 1], kChunkBytes);
-            bulk_g2s(sk[warp][b ^ 1], kin + uint64_t(cn) * kWarpStageKeys, kChunkBytes, &bar[warp][b ^ 1]);
+            mbar_arrive_expect_tx(&bar[warp][b ^ 1], chunk_bytes);
+            bulk_g2s(sk[warp][b ^ 1], kin + uint64_t(cn) * chunk, chunk_bytes, &bar[warp][b ^ 1]);
         }
         bool const ok = wc.probe_timeout ? mbar_wait_bounded(&never[warp], 0, wc.ns)
                                          : mbar_wait_bounded(&bar[warp][b], (it >> 1) & 1, wc.ns);
@@ -1271,8 +1109,8 @@ __global__ void __launch_bounds__(256, B2CO_WDEFER_MINB(Q)) k_find_wdefer(__grid
             break;
         }
         Key const* ks = sk[warp][b];
-        uint32_t const base = c * kWarpStageKeys;
-        for (uint32_t p = 0; p < kWarpStageKeys; p += PASS) {
+        uint32_t const base = c * chunk;
+        for (uint32_t p = 0; p < chunk; p += PASS) {
             uint64_t key[Q];
             uint32_t idx[Q];
 #pragma unroll
@@ -1310,23 +1148,23 @@ __global__ void __launch_bounds__(256, B2CO_WDEFER_MINB(Q)) k_find_wdefer(__grid
         return;
     }
     while (count > 0) follow();  // each round moves every queued key on by a window or settles it
-    // the ragged tail (< one warp stage) goes to one warp, keys read directly
-    if (chunks * kWarpStageKeys < n && gwarp == chunks % nwarps) {
-        for (uint32_t i0 = chunks * kWarpStageKeys; i0 < n; i0 += TILES) {
-            uint32_t const i = i0 + tile;
-            bool const live = i < n;
-            uint64_t const key = live ? Io<S>::load_key(keys, i) : 0;
-            uint32_t const init0 = live ? probe_init<S::key_bytes, B>(a.probe, key) : 0;
-            Raw w[ROUNDS];
-            load_range<S, B, G, ROUNDS>(slots, init0, 0, B, r, !live, w);
-            TileResult res{0, false, !live};
-            resolve_range<S, B, G, ROUNDS>(a, w, 0, B, key, r, tile_lane0, !live, res);
-            if (__any_sync(0xffffffffu, !res.done))
-                res = tile_continue<S, B, G, ROUNDS>(a, slots, key, init0, r, tile_lane0, res);
-            if (r == 0 && live) {
-                if constexpr (CONTAINS) reinterpret_cast<uint8_t*>(out)[i] = res.hit;
-                else Io<S>::store_payload(out, i, res.hit ? res.payload : empty_payload<S>(a));
-            }
+    // the keys after the last whole chunk, read directly: one pass of TILES keys a
+    // warp, from the warp after the one that took the last chunk
+    uint32_t const tail_warp = gwarp + (gwarp < chunks % nwarps ? nwarps : 0) - chunks % nwarps;
+    for (uint32_t i0 = chunks * chunk + tail_warp * TILES; i0 < n; i0 += nwarps * TILES) {
+        uint32_t const i = i0 + tile;
+        bool const live = i < n;
+        uint64_t const key = live ? Io<S>::load_key(keys, i) : 0;
+        uint32_t const init0 = live ? probe_init<S::key_bytes, B>(a.probe, key) : 0;
+        Raw w[ROUNDS];
+        load_range<S, B, G, ROUNDS>(slots, init0, 0, B, r, !live, w);
+        TileResult res{0, false, !live};
+        resolve_range<S, B, G, ROUNDS>(a, w, 0, B, key, r, tile_lane0, !live, res);
+        if (__any_sync(0xffffffffu, !res.done))
+            res = tile_continue<S, B, G, ROUNDS>(a, slots, key, init0, r, tile_lane0, res);
+        if (r == 0 && live) {
+            if constexpr (CONTAINS) reinterpret_cast<uint8_t*>(out)[i] = res.hit;
+            else Io<S>::store_payload(out, i, res.hit ? res.payload : empty_payload<S>(a));
         }
     }
 }

@@ -1,0 +1,368 @@
+// oa_sector.cuh -- the default lookup and write kernels of the open-addressing
+// containers: one key per lane, its window read as whole 32-byte sectors.
+//
+// What bounds these operations while the table is in L2 is what a bucket window
+// costs an SM: instructions and L1 requests.  A window of B slots is read here
+// as the 32-byte sectors it covers, a sector a load (ld.global.v4.u64): five
+// 16-byte slots are three loads, five 8-byte slots two, where one lane per slot
+// took five lanes' worth of compares and shuffles.  A lane works alone, so a pass
+// serves 32 keys of a warp with no shuffles, and results leave coalesced.  Keys
+// whose window decides nothing are queued in shared memory and followed a full
+// pass at a time, one window each, through the same code, so a pass waits on one
+// window load only, whatever the load factor.
+//
+// Measured on one B200, 16 M lookups at 50% hits: 97 Gkeys/s on a 20 MB table of
+// 8-byte slots (two lanes a window: 92) and 67 on an 80 MB table of 16-byte slots
+// (46); 1.3 M inserts into a 20 MB table 38 Gpairs/s (slot by slot: 30).  Which
+// tables and batches take these kernels is decided in oa_inst.cuh.
+//
+// Every loop is bounded by the probe cycle, so no kernel can spin.
+#pragma once
+
+#include "oa_kernels.cuh"
+
+namespace b2co {
+
+struct alignas(32) Sector {
+    unsigned long long w[4];
+};
+
+__device__ __forceinline__ Sector ld_sector_ro(void const* p)
+{
+    Sector v;
+    asm(B2CO_LD_RO ".v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(v.w[0]), "=l"(v.w[1]), "=l"(v.w[2]), "=l"(v.w[3]) : "l"(p));
+    return v;
+}
+// Coherent (L2, never a stale L1 line), for kernels that race with writers.
+__device__ __forceinline__ Sector ld_sector_rw(void const* p)
+{
+    Sector v;
+    asm volatile("ld.relaxed.gpu.global.L2::64B.v4.u64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(v.w[0]), "=l"(v.w[1]), "=l"(v.w[2]), "=l"(v.w[3])
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
+
+constexpr uint32_t gcd_u32(uint32_t a, uint32_t b) { return b == 0 ? a : gcd_u32(b, a % b); }
+
+// A bucket window of B slots as the aligned 32-byte sectors it covers.  The
+// sectors may hold slots beside the window; they are masked (slot storage is a
+// multiple of 32 bytes, so no load leaves it).
+template <class S, int B>
+struct SectorWindow {
+    using Raw = typename S::Raw;
+    static constexpr int N = 32 / S::bytes;                                 // slots per sector
+    static constexpr uint32_t kStep = gcd_u32(uint32_t(B) * S::bytes, 32);  // window starts are multiples of this
+    static constexpr int NS = int((32 - kStep + uint32_t(B) * S::bytes + 31) / 32);  // sectors that may be covered
+    static_assert(NS * N <= 32, "slot mask");
+    Sector s[NS];
+    uint32_t off;  // the window's first slot within its first sector
+
+    template <bool COHERENT>
+    __device__ __forceinline__ void load(Raw const* win)
+    {
+        uintptr_t const addr = reinterpret_cast<uintptr_t>(win);
+        off = uint32_t(addr & 31) / S::bytes;
+        char const* p = reinterpret_cast<char const*>(addr & ~uintptr_t(31));
+#pragma unroll
+        for (int i = 0; i < NS; ++i) {
+            // the last sector is covered only when the window starts late enough in the first
+            bool const need = i == 0 || off + B > uint32_t(i) * N;
+            if (need) s[i] = COHERENT ? ld_sector_rw(p + 32 * i) : ld_sector_ro(p + 32 * i);
+        }
+    }
+    __device__ __forceinline__ Raw slot(int j) const
+    {
+        Sector const& w = s[j / N];
+        int const i = j % N;
+        if constexpr (S::bytes == 16) return U128{w.w[2 * i], w.w[2 * i + 1]};
+        else if constexpr (S::bytes == 8) return w.w[i];
+        else if constexpr (S::bytes == 4) return Raw(w.w[i / 2] >> (32 * (i % 2)));
+        else return Raw(w.w[i / 4] >> (16 * (i % 4)));
+    }
+    // First slot of the window, in scan order, that is empty or holds an equal
+    // key: its place among the loaded slots (window slot + off), or -1.
+    __device__ __forceinline__ int first_stop(uint64_t key, uint64_t empty_key) const
+    {
+        uint32_t m = 0;
+#pragma unroll
+        for (int j = 0; j < NS * N; ++j) {
+            uint64_t const k = S::key(slot(j));
+            if (k == empty_key || S::key_eq(k, key)) m |= 1u << j;
+        }
+        m &= ((1u << B) - 1u) << off;
+        return __ffs(m) - 1;
+    }
+    // Slot j of the loaded ones (an unrolled select: a computed index would move
+    // the window to local memory).
+    __device__ __forceinline__ Raw pick(int j) const
+    {
+        Raw r = slot(0);
+#pragma unroll
+        for (int i = 1; i < NS * N; ++i)
+            if (j == i) r = slot(i);
+        return r;
+    }
+};
+
+constexpr uint32_t kSectorRing = 64;  // queued keys per warp: a pass may add 31 + 32
+
+// ----------------------------------------------------------------------------
+// Find / Contains, with or without a stencil
+// ----------------------------------------------------------------------------
+
+#ifndef B2CO_SECTOR_FIND_MINB
+#define B2CO_SECTOR_FIND_MINB(NS) ((NS) >= 3 ? 4 : 5)
+#endif
+
+template <class S, int B, bool CONTAINS>
+__global__ void __launch_bounds__(256, B2CO_SECTOR_FIND_MINB((SectorWindow<S, B>::NS)))
+    k_find_sector(__grid_constant__ const OaArgs a, void const* keys, uint8_t const* stencil, void* out, uint32_t n)
+{
+    using Raw = typename S::Raw;
+    constexpr uint32_t RING = kSectorRing - 1;
+    __shared__ uint64_t qkey[8][kSectorRing];
+    __shared__ uint32_t qinit[8][kSectorRing], qidx[8][kSectorRing], qpos[8][kSectorRing];
+
+    uint32_t const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t const stride = gridDim.x * blockDim.x;  // keys of one pass of the whole grid
+    uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
+    uint32_t head = 0, count = 0;  // queue state, the same on every lane
+    Raw const* const slots = reinterpret_cast<Raw const*>(a.slots);
+
+    auto store = [&](uint32_t pos, bool hit, uint64_t payload) {
+        if constexpr (CONTAINS) reinterpret_cast<uint8_t*>(out)[pos] = hit;
+        else Io<S>::store_payload(out, pos, payload);
+    };
+    // the next pass's key is loaded one pass ahead
+    uint64_t next_key = base + lane < n ? Io<S>::load_key(keys, base + lane) : 0;
+    for (;;) {
+        uint64_t key;
+        uint32_t init, idx, pos;
+        bool live;
+        if (count >= 32 || base >= n) {
+            if (count == 0) break;
+            __syncwarp();  // the queue writes precede these reads
+            uint32_t const take = count < 32 ? count : 32;
+            live = lane < take;
+            uint32_t const e = (head + (live ? lane : 0u)) & RING;
+            key = qkey[warp][e];
+            init = qinit[warp][e];
+            idx = qidx[warp][e];
+            pos = qpos[warp][e];
+            __syncwarp();  // every read of the taken entries precedes their reuse
+            head = (head + take) & RING;
+            count -= take;
+            idx = probe_next(idx, probe_step<S::key_bytes, B>(a.probe, key), a.probe.capacity);
+            if (live && idx == init) {  // full cycle: not present
+                store(pos, false, empty_payload<S>(a));
+                live = false;
+            }
+        } else {
+            pos = base + lane;
+            key = next_key;
+            live = pos < n;
+            if (stencil && live && !stencil[pos]) {
+                store(pos, false, empty_payload<S>(a));
+                live = false;
+            }
+            init = idx = probe_init<S::key_bytes, B>(a.probe, key);
+            base += stride;
+            next_key = base < n && base + lane < n ? Io<S>::load_key(keys, base + lane) : 0;
+        }
+        bool open = false;
+        if (live) {
+            SectorWindow<S, B> w;
+            w.template load<false>(slots + idx);
+            int const j = w.first_stop(key, a.empty_key);
+            if (j >= 0) {
+                Raw const slot = w.pick(j);
+                bool const hit = S::key(slot) != a.empty_key;
+                store(pos, hit, hit ? S::value(slot) : empty_payload<S>(a));
+            } else {
+                open = true;
+            }
+        }
+        uint32_t const m = __ballot_sync(0xffffffffu, open);
+        if (open) {
+            uint32_t const e = (head + count + __popc(m & ((1u << lane) - 1u))) & RING;
+            qkey[warp][e] = key;
+            qinit[warp][e] = init;
+            qidx[warp][e] = idx;
+            qpos[warp][e] = pos;
+        }
+        count += __popc(m);
+    }
+}
+
+// ----------------------------------------------------------------------------
+// Insert / InsertIf / InsertOrAssign, InsertAndFind (race), first-wins placement
+// ----------------------------------------------------------------------------
+
+enum { kInsPlain = 0, kInsAssign = 1, kInsIafRace = 2, kInsIafPlace = 3 };
+
+// Outputs of one insert-family launch (only the mode's fields are used).
+struct InsOut {
+    unsigned long long* counters;  // plain/assign: [failed, assigned] or NULL (async)
+    void* found;                   // race: payload found or inserted
+    uint8_t* inserted;             // race: 1 = this input inserted the key
+    uint32_t* pos;                 // place: slot of every input (kNoSlot = failed)
+    uint32_t* newbits;             // place: slots claimed by this batch
+    uint32_t* owner;               // place: claiming input of each claimed slot (claim_bit 0 only)
+    uint32_t claim_bit;            // place: flag OR-ed into pos[] of the claiming input (0 = none)
+};
+
+enum { kOpen = 3 };  // no verdict yet: the key goes on to its next window
+
+// Claims slot j of a window that was seen empty, or scans on from it as the
+// reference does (InsertVerdict, open_addressing_ref_impl.h:489-532): a lost
+// CAS goes on after that slot unless the winner holds an equal key.  Returns
+// the verdict (kOpen: the window is exhausted) with the deciding slot in j and,
+// for a duplicate met by a CAS, its contents in `old`.
+template <class S, int B>
+__device__ __forceinline__ int sector_claim(OaArgs const& a, typename S::Raw* win, uint64_t key, uint64_t val, int& j,
+                                            typename S::Raw& old)
+{
+    using Raw = typename S::Raw;
+    Raw expected = S::make(a.empty_key, a.empty_value);
+    old = cas_slot(win + j, expected, insert_desired<S>(expected, key, val));
+    if (raw_eq(old, expected)) return kSuccess;
+    if (S::key_eq(S::key(old), key)) return kDuplicate;
+    // rare: the slot was taken by another key, or is empty with another payload
+    if (S::bytes < 16 || S::key(old) != a.empty_key) ++j;
+    for (; j < B; ++j) {
+        Raw cur = ld_rw(win + j);
+        uint64_t const k = S::key(cur);
+        if (S::key_eq(k, key)) {
+            old = cur;
+            return kDuplicate;
+        }
+        if (k != a.empty_key || !insert_expected<S>(a, cur, expected)) continue;
+        old = cas_slot(win + j, expected, insert_desired<S>(cur, key, val));
+        if (raw_eq(old, expected)) return kSuccess;
+        if (S::key_eq(S::key(old), key)) return kDuplicate;
+    }
+    return kOpen;
+}
+
+#ifndef B2CO_SECTOR_WRITE_MINB
+#define B2CO_SECTOR_WRITE_MINB(NS) ((NS) >= 3 ? 4 : 5)
+#endif
+
+template <class S, int B, int MODE>
+__global__ void __launch_bounds__(256, B2CO_SECTOR_WRITE_MINB((SectorWindow<S, B>::NS)))
+    k_insert_sector(__grid_constant__ const OaArgs a, void const* pairs, uint8_t const* stencil, uint32_t n, InsOut o)
+{
+    using Raw = typename S::Raw;
+    constexpr uint32_t RING = kSectorRing - 1;
+    __shared__ Raw qpair[8][kSectorRing];
+    __shared__ uint32_t qinit[8][kSectorRing], qidx[8][kSectorRing], qpos[8][kSectorRing];
+
+    uint32_t const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t const stride = gridDim.x * blockDim.x;
+    uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
+    uint32_t head = 0, count = 0;
+    uint32_t failed = 0, assigned = 0;
+    Raw* const slots = reinterpret_cast<Raw*>(a.slots);
+
+    auto record = [&](uint32_t i, int verdict, uint32_t where, uint64_t found) {
+        if constexpr (MODE == kInsPlain || MODE == kInsAssign) {
+            // Insert succeeds only on SUCCESS (open_addressing_ref_impl.h:282-285);
+            // InsertOrAssign counts a duplicate as an assignment instead.
+            failed += MODE == kInsAssign ? verdict == kFailed : verdict != kSuccess;
+            assigned += verdict == kDuplicate;
+        } else if constexpr (MODE == kInsIafRace) {
+            Io<S>::store_payload(o.found, i, verdict == kFailed ? empty_payload<S>(a) : found);
+            o.inserted[i] = verdict == kSuccess;
+        } else {
+            uint32_t const p = verdict == kFailed ? kNoSlot : where;
+            if (verdict == kSuccess) {
+                atomicOr(o.newbits + (p >> 5), 1u << (p & 31));
+                if (!o.claim_bit) o.owner[p] = i;  // tables without room for the claim bit
+            }
+            o.pos[i] = verdict == kSuccess ? (p | o.claim_bit) : p;
+        }
+    };
+    bool next_in = base + lane < n && (!stencil || stencil[base + lane]);
+    Raw next_pair = next_in ? Io<S>::load_pair(pairs, base + lane) : Raw{};
+    for (;;) {
+        Raw pr;
+        uint32_t init, idx, pos;
+        bool live;
+        if (count >= 32 || base >= n) {
+            if (count == 0) break;
+            __syncwarp();
+            uint32_t const take = count < 32 ? count : 32;
+            live = lane < take;
+            uint32_t const e = (head + (live ? lane : 0u)) & RING;
+            pr = qpair[warp][e];
+            init = qinit[warp][e];
+            idx = qidx[warp][e];
+            pos = qpos[warp][e];
+            __syncwarp();
+            head = (head + take) & RING;
+            count -= take;
+            idx = probe_next(idx, probe_step<S::key_bytes, B>(a.probe, S::key(pr)), a.probe.capacity);
+            if (live && idx == init) {  // a whole cycle: the table is full for this key
+                record(pos, kFailed, 0, 0);
+                live = false;
+            }
+        } else {
+            pos = base + lane;
+            pr = next_pair;
+            live = next_in;
+            if (live && S::key(pr) == a.empty_key) {  // the empty key itself: FAILED
+                record(pos, kFailed, 0, 0);
+                live = false;
+            }
+            init = idx = probe_init<S::key_bytes, B>(a.probe, S::key(pr));
+            base += stride;
+            next_in = base < n && base + lane < n && (!stencil || stencil[base + lane]);
+            next_pair = next_in ? Io<S>::load_pair(pairs, base + lane) : Raw{};
+        }
+        int verdict = kOpen;
+        if (live) {
+            uint64_t const key = S::key(pr), val = S::value(pr);
+            Raw* const win = slots + idx;
+            SectorWindow<S, B> w;
+            w.template load<true>(win);
+            int j = w.first_stop(key, a.empty_key);
+            if (j >= 0) {
+                Raw old = w.pick(j);
+                j -= int(w.off);
+                if (S::key(old) == a.empty_key) {
+                    verdict = sector_claim<S, B>(a, win, key, val, j, old);
+                } else {
+                    verdict = kDuplicate;
+                }
+                uint64_t found = 0;
+                if (verdict == kDuplicate) {
+                    if constexpr (MODE == kInsAssign) assign_payload<S>(win + j, key, val);
+                    if constexpr (MODE == kInsIafRace) found = S::value(settle<S>(a, win + j, old));
+                } else if (verdict == kSuccess) {
+                    found = S::is_set ? key : val;
+                }
+                if (verdict != kOpen) record(pos, verdict, idx + uint32_t(j), found);
+            }
+        }
+        bool const open = live && verdict == kOpen;
+        uint32_t const m = __ballot_sync(0xffffffffu, open);
+        if (open) {
+            uint32_t const e = (head + count + __popc(m & ((1u << lane) - 1u))) & RING;
+            qpair[warp][e] = pr;
+            qinit[warp][e] = init;
+            qidx[warp][e] = idx;
+            qpos[warp][e] = pos;
+        }
+        count += __popc(m);
+    }
+    if constexpr (MODE == kInsPlain || MODE == kInsAssign) {
+        if (o.counters) {
+            block_add_counter(o.counters, failed);
+            if (MODE == kInsAssign) block_add_counter(o.counters + 1, assigned);
+        }
+    }
+}
+
+}  // namespace b2co
