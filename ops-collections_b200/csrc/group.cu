@@ -35,7 +35,7 @@ struct b2co_oa_group {
     GroupTable* d_tables = nullptr;
     unsigned long long* d_counters = nullptr;  // [failed, status]
     unsigned long long* h_counters = nullptr;
-    uint32_t find_shape = 4u | (2u << 8);  // lanes | keys per lane group << 8 | block << 16 (0 = 256)
+    uint32_t find_shape = 1u | (1u << 8);  // lanes | keys per lane group << 8 | block << 16 (0 = 256)
     // one cached graph of the group Find launch
     cudaStream_t capture_stream = nullptr;
     cudaGraphExec_t graph = nullptr;
@@ -71,6 +71,8 @@ GroupArgs group_args(b2co_oa_group const* g, uint64_t const* d_offsets)
     a.tables = g->d_tables;
     a.offsets = d_offsets;
     a.count = g->count;
+    a.probing = g->desc.probing;
+    a.hash = g->desc.hash;
     a.empty_key = g->desc.empty_key_bits;
     a.empty_value = g->desc.value_bytes ? g->desc.empty_value_bits : 0;
     return a;
@@ -227,7 +229,7 @@ int b2co_oa_group_create(b2co_oa_desc const* d, uint64_t const* requested, uint3
         off += cap;
     }
     g->total_slots = off;
-    B2CO_CUDA(cudaMalloc(&g->slab, off * g->slot_bytes));
+    B2CO_CUDA(cudaMalloc(&g->slab, (off * g->slot_bytes + 31) / 32 * 32));  // whole sectors (oa_sector.cuh)
     B2CO_CUDA(cudaMalloc(&g->d_tables, sizeof(GroupTable) * count));
     B2CO_CUDA(cudaMemcpy(g->d_tables, g->host_tables.data(), sizeof(GroupTable) * count, cudaMemcpyHostToDevice));
     B2CO_CUDA(cudaMalloc(&g->d_counters, 2 * sizeof(unsigned long long)));

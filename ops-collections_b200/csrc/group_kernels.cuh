@@ -3,14 +3,22 @@
 // per-partition group-by / join builds).
 //
 // One launch covers every table: the items of all tables are concatenated
-// (table t owns items [offsets[t], offsets[t+1])) and each warp takes one
-// contiguous span of the concatenation, so work is balanced by items, not by
-// tables.  A lane finds its table once by binary search and then only walks
-// forward; the table's probe parameters stay in registers while it does not
-// change.  Per key the algorithms are exactly the single-table ones.
+// (table t owns items [offsets[t], offsets[t+1])) and dealt to the warps in
+// chunks of at most 256 items, chunk c to warp c % warps, so work is balanced by
+// items, not by tables, and the chunks in flight at one time are neighbours:
+// the few tables they touch stay in L2, and the slab crosses HBM about once.
+// (One contiguous span per warp instead keeps the whole slab in play at once, so
+// that every window is a random HBM read.  4,096 tables of 280 M int32 pairs, a
+// 4.5 GB slab, 561 M lookups, with two lanes a window and two windows in flight:
+// Find 23.6 ms with spans, 11.8 with chunks.  With one lane a key reading whole
+// sectors, see below, 7.7 ms, and Insert 11.0 ms against 16.8 slot by slot.)
+// The warp searches the table of a chunk's first item together and each lane
+// walks forward from there; the table's probe parameters stay in registers
+// while it does not change.  Per key the algorithms are exactly the
+// single-table ones.
 #pragma once
 
-#include "oa_kernels.cuh"
+#include "oa_sector.cuh"
 
 namespace b2co {
 
@@ -24,17 +32,23 @@ struct GroupArgs {
     GroupTable const* tables;
     uint64_t const* offsets;  // count + 1 item offsets (device)
     uint32_t count;
+    uint32_t probing, hash;  // the same for every table
     uint64_t empty_key;
     uint64_t empty_value;
 };
 
+// The table of item i (the last t with offsets[t] <= i), searched by the whole
+// warp: 32 probes a round, so 1,024 tables take two rounds and 32,768 three.
 __device__ __forceinline__ uint32_t group_table_of(uint64_t const* offsets, uint32_t count, uint64_t i)
 {
-    uint32_t lo = 0, hi = count;  // offsets[lo] <= i < offsets[hi]
-    while (hi - lo > 1) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(offsets + mid) <= i) lo = mid;
-        else hi = mid;
+    uint32_t const lane = threadIdx.x & 31;
+    uint32_t lo = 0, left = count;  // the answer is in [lo, lo + left); offsets[lo] <= i
+    while (left > 1) {
+        uint32_t const step = (left + 31) / 32, at = lane * step;
+        bool const below = at < left && __ldg(offsets + lo + at) <= i;
+        uint32_t const last = 31 - __clz(__ballot_sync(0xffffffffu, below) | 1u);
+        lo += last * step;
+        left = left - last * step < step ? left - last * step : step;
     }
     return lo;
 }
@@ -46,89 +60,173 @@ __device__ __forceinline__ OaArgs group_table_args(GroupArgs const& g, uint32_t 
     GroupTable const& d = g.tables[t];
     a.slots = static_cast<typename S::Raw*>(g.slots) + d.slot_offset;
     a.probe = d.probe;
+    a.probe.probing = g.probing;
+    a.probe.hash = g.hash;
     a.empty_key = g.empty_key;
     a.empty_value = g.empty_value;
     a.erased_key = g.empty_key;
     return a;
 }
 
-// Span of the concatenation owned by this warp: multiples of `step` items.
-__device__ __forceinline__ void warp_span(uint64_t n, uint32_t step, uint64_t& begin, uint64_t& end)
+// Items per chunk: a multiple of 32 (every kernel's pass divides it), small
+// enough that a small batch still reaches every warp.
+constexpr uint32_t kGroupChunk = 256;
+inline uint32_t group_chunk(uint64_t n, uint64_t warps)
 {
-    uint64_t const warps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
-    uint64_t const warp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    uint64_t span = (n + warps - 1) / warps;
-    span = (span + step - 1) / step * step;
-    begin = warp * span;
-    end = begin + span < n ? begin + span : n;
+    uint64_t const share = ((n + warps - 1) / warps + 31) / 32 * 32;
+    return share < kGroupChunk ? uint32_t(share ? share : 32) : kGroupChunk;
+}
+__device__ __forceinline__ uint64_t group_warps() { return (uint64_t(gridDim.x) * blockDim.x) >> 5; }
+__device__ __forceinline__ uint64_t group_warp()
+{
+    return (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
 }
 
-// One lane per key: the window is scanned in the lane's own registers, with no
-// ballots or shuffles, and a key that needs further windows walks on alone.
+// A lane's place in the concatenation: the table of its item, with what its
+// probing needs, walked forward as the items ascend.
+template <class S, int B>
+struct GroupCursor {
+    uint32_t t;
+    uint64_t next_off;
+    OaArgs a;
+    __device__ __forceinline__ void start(GroupArgs const& g, uint64_t begin)  // the whole warp
+    {
+        t = group_table_of(g.offsets, g.count, begin);
+        next_off = __ldg(g.offsets + t + 1);
+        a = group_table_args<S>(g, t);
+    }
+    __device__ __forceinline__ void advance(GroupArgs const& g, uint64_t i)
+    {
+        if (i < next_off) return;
+        do {
+            ++t;
+            next_off = __ldg(g.offsets + t + 1);
+        } while (i >= next_off);
+        a = group_table_args<S>(g, t);
+    }
+};
+
+// One lane per key, its window read as whole sectors (oa_sector.cuh); a key whose
+// window settles nothing is queued in the warp's shared-memory ring with its
+// table and followed a full pass at a time, one window each.  Bound by the L2
+// requests of the windows, as the single-table kernel: 73 Gkeys/s over the 4,096
+// tables above.  Asking L2 for the slab ahead of the chunks with bulk prefetches
+// was slower (10.0 ms).  Blocks of up to 256 threads.
 template <class S, int B, bool CONTAINS>
-__device__ __forceinline__ void group_find_lane(GroupArgs const& g, void const* keys, void* out, uint64_t begin,
-                                                uint64_t end)
+__global__ void __launch_bounds__(256, 4) k_group_find_lane(__grid_constant__ const GroupArgs g, void const* keys,
+                                                            void* out, uint64_t n, uint32_t chunk)
 {
     using Raw = typename S::Raw;
-    uint32_t const lane = threadIdx.x & 31;
-    uint32_t t = group_table_of(g.offsets, g.count, begin + lane < end ? begin + lane : begin);
-    OaArgs a = group_table_args<S>(g, t);
-    uint64_t next_off = __ldg(g.offsets + t + 1);
-    for (uint64_t i = begin + lane; i < end; i += 32) {
-        if (i >= next_off) {
-            do {
-                ++t;
-                next_off = __ldg(g.offsets + t + 1);
-            } while (i >= next_off);
-            a = group_table_args<S>(g, t);
-        }
-        uint64_t const key = uint64_t(__ldg(reinterpret_cast<typename Io<S>::Key const*>(keys) + i));
-        uint32_t const init = probe_init<S::key_bytes, B>(a.probe, key);
-        Raw w[B];
-        load_window<S, B>(reinterpret_cast<Raw const*>(a.slots), init, w);
-        Raw stop;
-        uint64_t payload = empty_payload<S>(a);
-        bool hit;
-        if (scan_window<S, B>(w, key, a.empty_key, stop)) {
-            hit = S::key(stop) != a.empty_key;
-            if (hit) payload = S::value(stop);
+    using Key = typename Io<S>::Key;
+    constexpr uint32_t RING = kSectorRing - 1;
+    __shared__ uint64_t qkey[8][kSectorRing], qpos[8][kSectorRing];
+    __shared__ uint32_t qtab[8][kSectorRing], qinit[8][kSectorRing], qidx[8][kSectorRing];
+
+    uint32_t const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t const stride = group_warps() * chunk;
+    uint64_t begin = group_warp() * chunk, at = begin, end = begin + chunk < n ? begin + chunk : n;
+    Key const* const kin = static_cast<Key const*>(keys);
+    uint64_t const empty = S::is_set ? g.empty_key : g.empty_value;
+    uint32_t head = 0, count = 0;
+
+    auto store = [&](uint64_t pos, bool hit, uint64_t payload) {
+        if constexpr (CONTAINS) reinterpret_cast<uint8_t*>(out)[pos] = hit;
+        else reinterpret_cast<typename Io<S>::Payload*>(out)[pos] = typename Io<S>::Payload(hit ? payload : empty);
+    };
+    GroupCursor<S, B> cur;
+    uint64_t next_key = 0;
+    if (begin < n) {
+        cur.start(g, begin);
+        next_key = at + lane < end ? uint64_t(__ldg(kin + at + lane)) : 0;
+    }
+    for (;;) {
+        uint64_t key, pos;
+        uint32_t tab, init, idx;
+        Raw const* slots;
+        bool live;
+        if (count >= 32 || begin >= n) {
+            if (count == 0) break;
+            __syncwarp();
+            uint32_t const take = count < 32 ? count : 32;
+            live = lane < take;
+            uint32_t const e = (head + (live ? lane : 0u)) & RING;
+            key = qkey[warp][e];
+            pos = qpos[warp][e];
+            tab = qtab[warp][e];
+            init = qinit[warp][e];
+            idx = qidx[warp][e];
+            __syncwarp();
+            head = (head + take) & RING;
+            count -= take;
+            OaArgs const a = group_table_args<S>(g, tab);
+            slots = static_cast<Raw const*>(a.slots);
+            idx = probe_next(idx, probe_step<S::key_bytes, B>(a.probe, key), a.probe.capacity);
+            if (live && idx == init) {  // a whole cycle: not present
+                store(pos, false, empty);
+                live = false;
+            }
         } else {
-            hit = find_rest<S, B>(a, key, init, payload);
+            pos = at + lane;
+            live = pos < end;
+            key = next_key;
+            if (live) cur.advance(g, pos);
+            tab = cur.t;
+            slots = static_cast<Raw const*>(cur.a.slots);
+            init = idx = probe_init<S::key_bytes, B>(cur.a.probe, key);
+            at += 32;
+            if (at >= end) {  // the next chunk
+                begin += stride;
+                at = begin;
+                end = begin + chunk < n ? begin + chunk : n;
+                if (begin < n) cur.start(g, begin);
+            }
+            next_key = begin < n && at + lane < end ? uint64_t(__ldg(kin + at + lane)) : 0;
         }
-        if constexpr (CONTAINS) reinterpret_cast<uint8_t*>(out)[i] = hit;
-        else reinterpret_cast<typename Io<S>::Payload*>(out)[i] = typename Io<S>::Payload(hit ? payload : empty_payload<S>(a));
+        bool open = false;
+        if (live) {
+            SectorWindow<S, B> w;
+            w.template load<false>(slots + idx);
+            int const j = w.first_stop(key, g.empty_key);
+            if (j >= 0) {
+                Raw const slot = w.pick(j);
+                store(pos, S::key(slot) != g.empty_key, S::value(slot));
+            } else {
+                open = true;
+            }
+        }
+        uint32_t const m = __ballot_sync(0xffffffffu, open);
+        if (open) {
+            uint32_t const e = (head + count + __popc(m & ((1u << lane) - 1u))) & RING;
+            qkey[warp][e] = key;
+            qpos[warp][e] = pos;
+            qtab[warp][e] = tab;
+            qinit[warp][e] = init;
+            qidx[warp][e] = idx;
+        }
+        count += __popc(m);
     }
 }
 
 template <class S, int B, int G, bool CONTAINS>
-__global__ void __launch_bounds__(256) k_group_find(GroupArgs g, void const* keys, void* out, uint64_t n)
+__global__ void __launch_bounds__(256) k_group_find(__grid_constant__ const GroupArgs g, void const* keys,
+                                                    void* out, uint64_t n, uint32_t chunk)
 {
-    if constexpr (G == 1) {
-        uint64_t begin, end;
-        warp_span(n, 32, begin, end);
-        if (begin < end) group_find_lane<S, B, CONTAINS>(g, keys, out, begin, end);
-        return;
-    }
+    uint64_t const stride = group_warps() * chunk;
     using Raw = typename S::Raw;
     constexpr int ROUNDS = (B + G - 1) / G;
     constexpr uint32_t TILES = 32 / G;
     uint32_t const lane = threadIdx.x & 31, r = lane % G, tile_lane0 = lane & ~uint32_t(G - 1), tile = lane / G;
-    uint64_t begin, end;
-    warp_span(n, TILES, begin, end);
-    if (begin >= end) return;  // warp-uniform
-    uint32_t t = group_table_of(g.offsets, g.count, begin + tile < end ? begin + tile : begin);
-    OaArgs a = group_table_args<S>(g, t);
-    uint64_t next_off = __ldg(g.offsets + t + 1);
-    for (uint64_t i0 = begin; i0 < end; i0 += TILES) {
+    GroupCursor<S, B> cur;
+    uint64_t end = 0;
+    for (uint64_t i0 = group_warp() * chunk, begin = i0; begin < n;) {
+        if (i0 == begin) {
+            end = begin + chunk < n ? begin + chunk : n;
+            cur.start(g, begin);
+        }
         uint64_t const i = i0 + tile;
         bool const live = i < end;
-        if (live && i >= next_off) {
-            do {
-                ++t;
-                next_off = __ldg(g.offsets + t + 1);
-            } while (i >= next_off);
-            a = group_table_args<S>(g, t);
-        }
+        if (live) cur.advance(g, i);
+        OaArgs const& a = cur.a;
         uint64_t const key = live ? uint64_t(__ldg(reinterpret_cast<typename Io<S>::Key const*>(keys) + i)) : 0;
         uint32_t const init = live ? probe_init<S::key_bytes, B>(a.probe, key) : 0;
         Raw const* slots = reinterpret_cast<Raw const*>(a.slots);
@@ -146,6 +244,8 @@ __global__ void __launch_bounds__(256) k_group_find(GroupArgs g, void const* key
             else reinterpret_cast<typename Io<S>::Payload*>(out)[i] =
                 typename Io<S>::Payload(res.hit ? res.payload : empty_payload<S>(a));
         }
+        i0 += TILES;
+        if (i0 >= end) i0 = begin += stride;
     }
 }
 
@@ -156,7 +256,8 @@ __global__ void __launch_bounds__(256) k_group_find(GroupArgs g, void const* key
 // q-slot of a tile walks forward through the tables on its own, so a pass may
 // span a table boundary.  Blocks of up to 256 threads.
 template <class S, int B, int G, int Q, bool CONTAINS>
-__global__ void __launch_bounds__(256) k_group_find_q(GroupArgs g, void const* keys, void* out, uint64_t n)
+__global__ void __launch_bounds__(256) k_group_find_q(__grid_constant__ const GroupArgs g, void const* keys,
+                                                    void* out, uint64_t n, uint32_t chunk)
 {
     static_assert(Q <= G && G >= 2 && G <= 8, "tile shape");
     using Raw = typename S::Raw;
@@ -170,9 +271,6 @@ __global__ void __launch_bounds__(256) k_group_find_q(GroupArgs g, void const* k
 
     uint32_t const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t const r = lane % G, tile_lane0 = lane & ~uint32_t(G - 1), tile = lane / G;
-    uint64_t begin, end;
-    warp_span(n, PASS, begin, end);
-    if (begin >= end) return;  // warp-uniform
     uint32_t head = 0, count = 0;
     using Key = typename Io<S>::Key;
     Key const* kin = static_cast<Key const*>(keys);
@@ -239,15 +337,17 @@ __global__ void __launch_bounds__(256) k_group_find_q(GroupArgs g, void const* k
         }
     };
 
+    uint64_t const stride = group_warps() * chunk;
     uint32_t tq[Q];
-    uint64_t nextq[Q];
+    uint64_t nextq[Q], end = 0;
+    for (uint64_t i0 = group_warp() * chunk, begin = i0; begin < n;) {
+        if (i0 == begin) {
+            end = begin + chunk < n ? begin + chunk : n;
+            tq[0] = group_table_of(g.offsets, g.count, begin);
+            nextq[0] = __ldg(g.offsets + tq[0] + 1);
 #pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        uint64_t const i = begin + q * TILES + tile;
-        tq[q] = group_table_of(g.offsets, g.count, i < end ? i : end - 1);
-        nextq[q] = __ldg(g.offsets + tq[q] + 1);
-    }
-    for (uint64_t i0 = begin; i0 < end; i0 += PASS) {
+            for (int q = 1; q < Q; ++q) tq[q] = tq[0], nextq[q] = nextq[0];
+        }
         uint64_t key[Q];
         uint32_t idx[Q];
         bool live[Q];
@@ -282,37 +382,109 @@ __global__ void __launch_bounds__(256) k_group_find_q(GroupArgs g, void const* k
             enqueue(live[q] && st == kNoStop && r == 0, key[q], tq[q], idx[q], idx[q], i);
         }
         while (count >= PASS) follow();
+        i0 += PASS;
+        if (i0 >= end) i0 = begin += stride;
     }
     while (count > 0) follow();
 }
 
+// Insert into every table: k_insert_sector's pass with the item's own table.
 template <class S, int B>
-__global__ void __launch_bounds__(256) k_group_insert(GroupArgs g, void const* pairs, uint64_t n,
-                                                      unsigned long long* failed_counter)
+__global__ void __launch_bounds__(256, 4) k_group_insert(__grid_constant__ const GroupArgs g, void const* pairs, uint64_t n,
+                                                         uint32_t chunk, unsigned long long* failed_counter)
 {
-    uint64_t begin, end;
-    warp_span(n, 32, begin, end);
-    uint32_t failed = 0;
-    if (begin < end) {
-        uint32_t const lane = threadIdx.x & 31;
-        uint32_t t = group_table_of(g.offsets, g.count, begin + lane < end ? begin + lane : begin);
-        OaArgs a = group_table_args<S>(g, t);
-        uint64_t next_off = __ldg(g.offsets + t + 1);
-        for (uint64_t i0 = begin; i0 < end; i0 += 32) {
-            uint64_t const i = i0 + lane;
-            if (i >= end) continue;
-            if (i >= next_off) {
-                do {
-                    ++t;
-                    next_off = __ldg(g.offsets + t + 1);
-                } while (i >= next_off);
-                a = group_table_args<S>(g, t);
-            }
-            typename S::Raw p = ld_ro(reinterpret_cast<typename S::Raw const*>(pairs) + i);
-            failed += insert_one<S, B, false>(a, S::key(p), S::value(p)) != kSuccess;
-        }
+    using Raw = typename S::Raw;
+    constexpr uint32_t RING = kSectorRing - 1;
+    __shared__ Raw qpair[8][kSectorRing];
+    __shared__ uint32_t qtab[8][kSectorRing], qinit[8][kSectorRing], qidx[8][kSectorRing];
+
+    uint32_t const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t const stride = group_warps() * chunk;
+    uint64_t begin = group_warp() * chunk, at = begin, end = begin + chunk < n ? begin + chunk : n;
+    Raw const* const pin = static_cast<Raw const*>(pairs);
+    uint32_t head = 0, count = 0, failed = 0;
+    GroupCursor<S, B> cur;
+    Raw next_pair{};
+    if (begin < n) {
+        cur.start(g, begin);
+        if (at + lane < end) next_pair = ld_ro(pin + at + lane);
     }
-    if (failed_counter) warp_add_counter(failed_counter, failed);
+    for (;;) {
+        Raw pr;
+        uint32_t tab, init, idx;
+        Raw* slots;
+        bool live;
+        if (count >= 32 || begin >= n) {
+            if (count == 0) break;
+            __syncwarp();
+            uint32_t const take = count < 32 ? count : 32;
+            live = lane < take;
+            uint32_t const e = (head + (live ? lane : 0u)) & RING;
+            pr = qpair[warp][e];
+            tab = qtab[warp][e];
+            init = qinit[warp][e];
+            idx = qidx[warp][e];
+            __syncwarp();
+            head = (head + take) & RING;
+            count -= take;
+            OaArgs const a = group_table_args<S>(g, tab);
+            slots = static_cast<Raw*>(a.slots);
+            idx = probe_next(idx, probe_step<S::key_bytes, B>(a.probe, S::key(pr)), a.probe.capacity);
+            if (live && idx == init) {  // a whole cycle: the table is full for this key
+                ++failed;
+                live = false;
+            }
+        } else {
+            live = at + lane < end;
+            pr = next_pair;
+            if (live) cur.advance(g, at + lane);
+            tab = cur.t;
+            slots = static_cast<Raw*>(cur.a.slots);
+            init = idx = probe_init<S::key_bytes, B>(cur.a.probe, S::key(pr));
+            if (live && S::key(pr) == g.empty_key) {  // the empty key itself: FAILED
+                ++failed;
+                live = false;
+            }
+            at += 32;
+            if (at >= end) {
+                begin += stride;
+                at = begin;
+                end = begin + chunk < n ? begin + chunk : n;
+                if (begin < n) cur.start(g, begin);
+            }
+            if (begin < n && at + lane < end) next_pair = ld_ro(pin + at + lane);
+        }
+        int verdict = kOpen;
+        if (live) {
+            uint64_t const key = S::key(pr);
+            SectorWindow<S, B> w;
+            w.template load<true>(slots + idx);
+            int j = w.first_stop(key, g.empty_key);
+            if (j >= 0) {
+                Raw old = w.pick(j);
+                verdict = kDuplicate;
+                if (S::key(old) == g.empty_key) {
+                    OaArgs a{};
+                    a.empty_key = g.empty_key;
+                    a.empty_value = g.empty_value;
+                    j -= int(w.off);
+                    verdict = sector_claim<S, B>(a, slots + idx, key, S::value(pr), j, old);
+                }
+                failed += verdict == kDuplicate;
+            }
+        }
+        bool const open = live && verdict == kOpen;
+        uint32_t const m = __ballot_sync(0xffffffffu, open);
+        if (open) {
+            uint32_t const e = (head + count + __popc(m & ((1u << lane) - 1u))) & RING;
+            qpair[warp][e] = pr;
+            qtab[warp][e] = tab;
+            qinit[warp][e] = init;
+            qidx[warp][e] = idx;
+        }
+        count += __popc(m);
+    }
+    if (failed_counter) block_add_counter(failed_counter, failed);
 }
 
 }  // namespace b2co

@@ -443,7 +443,7 @@ struct GroupImpl {
     {
         uint32_t const lanes = shape & 0xffu, items = (shape >> 8) & 0xffu;
         uint32_t const block = (shape >> 16) ? (shape >> 16) : kBlock;
-        void (*k)(GroupArgs, void const*, void*, uint64_t) = nullptr;
+        void (*k)(GroupArgs, void const*, void*, uint64_t, uint32_t) = nullptr;
         if (lanes >= 2 && items >= 2) {
             if constexpr (B == 5) {
                 if (lanes == 2) k = k_group_find_q<S, B, 2, 2, C>;
@@ -452,7 +452,7 @@ struct GroupImpl {
             }
             if (!k) k = k_group_find_q<S, B, 4, 2, C>;
         } else if (lanes <= 1) {
-            k = k_group_find<S, B, 1, C>;
+            k = k_group_find_lane<S, B, C>;
         } else if (lanes == 2) {
             k = k_group_find<S, B, 2, C>;
         } else if (lanes == 4) {
@@ -460,8 +460,9 @@ struct GroupImpl {
         } else {
             k = k_group_find<S, B, 8, C>;
         }
-        // persistent: every resident block, spans balanced by items
-        k<<<grid_for((void const*)k, block, n, 1), block, 0, s>>>(g, keys, out, n);
+        // persistent: every resident block, at least 32 items a warp
+        uint32_t const grid = grid_for((void const*)k, block, n, block);
+        k<<<grid, block, 0, s>>>(g, keys, out, n, group_chunk(n, uint64_t(grid) * block / 32));
         return OaImpl<S>::check_launch(C ? "group contains kernel" : "group find kernel");
     }
 
@@ -480,7 +481,8 @@ struct GroupImpl {
         return OaImpl<S>::with_b(b, [&](auto bc) {
             constexpr int B = decltype(bc)::value;
             auto k = k_group_insert<S, B>;
-            k<<<grid_for((void const*)k, kBlock, n, 1), kBlock, 0, s>>>(g, pairs, n, failed);
+            uint32_t const grid = grid_for((void const*)k, kBlock, n, kBlock);
+            k<<<grid, kBlock, 0, s>>>(g, pairs, n, group_chunk(n, uint64_t(grid) * kBlock / 32), failed);
             return OaImpl<S>::check_launch("group insert kernel");
         });
     }

@@ -133,41 +133,6 @@ __device__ __forceinline__ typename S::Raw settle(OaArgs const& a, typename S::R
 
 enum { kFailed = 0, kSuccess = 1, kDuplicate = 2 };
 
-template <class S, int B, bool ASSIGN>
-__device__ __forceinline__ int insert_one(OaArgs const& a, uint64_t key, uint64_t val)
-{
-    using Raw = typename S::Raw;
-    if (key == a.empty_key) return kFailed;
-    Raw* slots = reinterpret_cast<Raw*>(a.slots);
-    uint32_t const init = probe_init<S::key_bytes, B>(a.probe, key);
-    uint32_t idx = init, step = 0;
-    for (;;) {
-#pragma unroll
-        for (int j = 0; j < B; ++j) {
-            Raw* sp = slots + idx + j;
-            Raw cur = ld_rw(sp);
-            uint64_t k = S::key(cur);
-            if (S::key_eq(k, key)) {
-                if constexpr (ASSIGN) assign_payload<S>(sp, key, val);
-                return kDuplicate;
-            }
-            if (k == a.empty_key) {
-                Raw expected;
-                if (!insert_expected<S>(a, cur, expected)) continue;
-                Raw old = cas_slot(sp, expected, insert_desired<S>(cur, key, val));
-                if (raw_eq(old, expected)) return kSuccess;
-                if (S::key_eq(S::key(old), key)) {
-                    if constexpr (ASSIGN) assign_payload<S>(sp, key, val);
-                    return kDuplicate;
-                }
-            }
-        }
-        if (step == 0) step = probe_step<S::key_bytes, B>(a.probe, key);
-        idx = probe_next(idx, step, a.probe.capacity);
-        if (idx == init) return kFailed;
-    }
-}
-
 __device__ __forceinline__ void warp_add_counter(unsigned long long* counter, uint32_t v)
 {
     uint32_t sum = __reduce_add_sync(0xffffffffu, v);
