@@ -20,6 +20,13 @@ struct WaitCtl {
 };
 
 #ifdef __CUDACC__
+// The status word may be host memory.
+__device__ __forceinline__ void report_timeout(WaitCtl const& wc)
+{
+    *reinterpret_cast<volatile unsigned int*>(wc.status) = kStatusTimeout;
+    __threadfence_system();
+}
+
 // Atomic compare-and-swap of a whole slot: 32-, 64- or 128-bit (the 128-bit form
 // needs sm_90+; it publishes key and payload together, so no reader ever sees a
 // key without its payload).

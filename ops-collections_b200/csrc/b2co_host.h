@@ -57,6 +57,7 @@ uint64_t prime_at_least(uint64_t n);
 uint64_t prime_table_last();
 
 struct OaArgs;
+struct Counters;
 
 // Lookup shape flag carried in the keys-per-lane field: scan each first window
 // by 64-byte segments (B2CO_FIND_SEGMENTED in the C ABI).
@@ -74,7 +75,7 @@ constexpr uint32_t kShapeDeferred = 0x800;
 struct OaOps {
     int (*clear)(OaArgs const& a, cudaStream_t s);
     int (*insert)(OaArgs const& a, uint32_t b, void const* pairs, uint8_t const* stencil, uint32_t n, bool assign,
-                  unsigned long long* counters, cudaStream_t s);
+                  Counters const& counters, cudaStream_t s);
     int (*assign_if)(OaArgs const& a, uint32_t b, void const* pairs, uint8_t const* stencil, uint32_t n,
                      cudaStream_t s);
     int (*iaf_race)(OaArgs const& a, uint32_t b, void const* pairs, void* found, uint8_t* inserted, uint32_t n,

@@ -390,7 +390,7 @@ int b2co_oa_group_insert_per_table(b2co_oa_group* g, void const* pairs, uint64_t
         uint64_t const lo = h_offsets[t], m = h_offsets[t + 1] - lo;
         if (m == 0) continue;
         int st = g->ops->insert(table_args(g, t), g->desc.bucket_size, static_cast<char const*>(pairs) + lo * g->slot_bytes,
-                                nullptr, uint32_t(m), false, nullptr, cs(s));
+                                nullptr, uint32_t(m), false, Counters{}, cs(s));
         if (st) return st;
     }
     return B2CO_OK;

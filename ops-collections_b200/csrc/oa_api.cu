@@ -5,7 +5,9 @@
 // and an async call return, batches beyond the kernel index range are a
 // length error, sync calls synchronize the stream and read the counters back.
 #include <cstring>
+#include <mutex>
 #include <new>
+#include <vector>
 
 #include "b2co_host.h"
 #include "oa_kernels.cuh"
@@ -57,8 +59,11 @@ struct b2co_oa_table {
     OaOps const* ops = nullptr;
     uint64_t capacity = 0;
     int device = 0;
-    unsigned long long* d_counters = nullptr;  // [failed, assigned]
-    unsigned long long* h_counters = nullptr;  // pinned mirror
+    unsigned long long* d_counters = nullptr;  // [keys not erased / keys counted]
+    unsigned long long* h_counters = nullptr;  // pinned: its mirror, then the status word that kernels write
+    std::mutex counters_mu;
+    std::vector<Counters> counters;       // of synchronous insert calls; one per call at a time
+    std::vector<Counters> idle_counters;
     // first-wins InsertAndFind scratch, grown on demand
     uint32_t* d_pos = nullptr;
     uint64_t pos_cap = 0;
@@ -93,7 +98,7 @@ int check_batch(uint64_t n)
 
 cudaStream_t cs(b2co_stream s) { return reinterpret_cast<cudaStream_t>(s); }
 
-unsigned int* status_word(b2co_oa_table* t) { return reinterpret_cast<unsigned int*>(t->d_counters + 2); }
+unsigned int* status_word(b2co_oa_table* t) { return reinterpret_cast<unsigned int*>(t->h_counters + 1); }
 
 int launch_find(b2co_oa_table* t, bool contains, void const* keys, uint8_t const* stencil, void* out, uint64_t n,
                 cudaStream_t s)
@@ -102,19 +107,48 @@ int launch_find(b2co_oa_table* t, bool contains, void const* keys, uint8_t const
                         uint32_t(n), wait_ctl(status_word(t)), s);
 }
 
-// Reads (and clears) the table's device status word; a set word means a
-// bounded device wait expired in some earlier kernel on this table.
+// Waits for the stream, then reads (and clears) the table's status word; a set
+// word means a bounded device wait expired in some earlier kernel on this table.
+// The word is host memory: a lookup's result check costs no copy.
 int check_status(b2co_oa_table* t, cudaStream_t s)
 {
-    B2CO_CUDA(cudaMemcpyAsync(t->h_counters + 2, t->d_counters + 2, sizeof(unsigned long long),
-                              cudaMemcpyDeviceToHost, s));
     B2CO_CUDA(cudaStreamSynchronize(s));
-    if (t->h_counters[2] != 0) {
-        B2CO_CUDA(cudaMemsetAsync(t->d_counters + 2, 0, sizeof(unsigned long long), s));
-        B2CO_CUDA(cudaStreamSynchronize(s));
+    auto* word = reinterpret_cast<unsigned int volatile*>(status_word(t));
+    if (*word != 0) {
+        *word = 0;
         return fail(B2CO_ETIMEOUT, "a bounded device wait expired (bulk key copy did not complete in time)");
     }
     return B2CO_OK;
+}
+
+// Counters for one synchronous insert call (concurrent calls on a table each
+// take their own); release() returns them.
+int take_counters(b2co_oa_table* t, Counters& c)
+{
+    std::lock_guard<std::mutex> g(t->counters_mu);
+    if (!t->idle_counters.empty()) {
+        c = t->idle_counters.back();
+        t->idle_counters.pop_back();
+        return B2CO_OK;
+    }
+    c = Counters{};
+    cudaError_t e = cudaMalloc(&c.sum, (kCounterWords + 1) * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMemset(c.sum, 0, (kCounterWords + 1) * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // zero before any stream of the caller's uses it
+    if (e == cudaSuccess) e = cudaMallocHost(&c.host, kCounterWords * sizeof(unsigned long long));
+    if (e != cudaSuccess) {
+        if (c.sum) cudaFree(c.sum);
+        return cuda_fail(e, "insert counters");
+    }
+    t->counters.push_back(c);
+    t->idle_counters.reserve(t->counters.size());  // giving one back never allocates
+    return B2CO_OK;
+}
+
+void give_counters(b2co_oa_table* t, Counters const& c)
+{
+    std::lock_guard<std::mutex> g(t->counters_mu);
+    t->idle_counters.push_back(c);
 }
 
 int sync_counters(b2co_oa_table* t, cudaStream_t s, int words)
@@ -171,13 +205,31 @@ int b2co_oa_launch_insert(b2co_oa_table* t, void const* pairs, uint64_t n, bool 
     if (int st = check_table(t)) return st;
     if (n == 0 || !pairs) return B2CO_OK;
     if (int st = check_batch(n)) return st;
-    return t->ops->insert(t->args, t->desc.bucket_size, pairs, nullptr, uint32_t(n), assign, d_counters, s);
+    return t->ops->insert(t->args, t->desc.bucket_size, pairs, nullptr, uint32_t(n), assign,
+                          Counters{d_counters, nullptr}, s);
+}
+
+// Insert / InsertOrAssign of the selected pairs, waited for:
+// counts = [failed, assigned, selected].
+int b2co_oa_insert_counted(b2co_oa_table* t, void const* pairs, uint8_t const* stencil, uint64_t n, bool assign,
+                           cudaStream_t s, uint64_t* counts)
+{
+    Counters c;
+    if (int st = take_counters(t, c)) return st;
+    int st = t->ops->insert(t->args, t->desc.bucket_size, pairs, stencil, uint32_t(n), assign, c, s);
+    if (!st) {
+        cudaError_t const e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) st = cuda_fail(e, "cudaStreamSynchronize");
+    }
+    for (int i = 0; i < kCounterWords; ++i) counts[i] = st ? 0 : static_cast<unsigned long long volatile*>(c.host)[i];
+    give_counters(t, c);
+    return st;
 }
 
 // Device bytes a table holds (slots and counters).
 uint64_t b2co_oa_table_bytes(b2co_oa_table const* t)
 {
-    return t ? t->capacity * slot_bytes(t->desc.key_bytes, t->desc.value_bytes) + 3 * sizeof(unsigned long long) : 0;
+    return t ? t->capacity * slot_bytes(t->desc.key_bytes, t->desc.value_bytes) + sizeof(unsigned long long) : 0;
 }
 
 // Key / payload / pair sizes of a table.
@@ -238,10 +290,9 @@ int b2co_oa_create_ex(b2co_oa_desc const* d, uint64_t requested, bool clear, b2c
 
     // whole 32-byte sectors: kernels read the sectors that a window covers
     cudaError_t e = cudaMalloc(&t->args.slots, (cap * slot_bytes(d->key_bytes, d->value_bytes) + 31) / 32 * 32);
-    // counters: [failed, assigned, status word]
-    if (e == cudaSuccess) e = cudaMalloc(&t->d_counters, 3 * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMemset(t->d_counters, 0, 3 * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMallocHost(&t->h_counters, 3 * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMalloc(&t->d_counters, sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMallocHost(&t->h_counters, 2 * sizeof(unsigned long long));
+    if (e == cudaSuccess) std::memset(t->h_counters, 0, 2 * sizeof(unsigned long long));
     if (e != cudaSuccess) {
         b2co_oa_destroy(t);
         return cuda_fail(e, "table allocation");
@@ -353,6 +404,10 @@ int b2co_oa_destroy(b2co_oa_table* t)
     if (t->args.slots) cudaFree(t->args.slots);
     if (t->d_counters) cudaFree(t->d_counters);
     if (t->h_counters) cudaFreeHost(t->h_counters);
+    for (Counters const& c : t->counters) {
+        cudaFree(c.sum);
+        cudaFreeHost(c.host);
+    }
     if (t->d_pos) cudaFree(t->d_pos);
     if (t->d_newbits) cudaFree(t->d_newbits);
     if (t->d_owner) cudaFree(t->d_owner);
@@ -426,14 +481,12 @@ static int insert_impl(b2co_oa_table* t, void const* pairs, uint8_t const* stenc
         return B2CO_OK;
     }
     if (int st = check_batch(n)) return st;
-    cudaStream_t c = cs(s);
-    if (sync) B2CO_CUDA(cudaMemsetAsync(t->d_counters, 0, 2 * sizeof(unsigned long long), c));
-    int st = t->ops->insert(t->args, t->desc.bucket_size, pairs, stencil, uint32_t(n), assign,
-                            sync ? t->d_counters : nullptr, c);
-    if (st || !sync) return st;
-    if ((st = sync_counters(t, c, 2))) return st;
-    if (failed) *failed = t->h_counters[0];
-    if (assigned) *assigned = t->h_counters[1];
+    if (!sync)
+        return t->ops->insert(t->args, t->desc.bucket_size, pairs, stencil, uint32_t(n), assign, Counters{}, cs(s));
+    uint64_t counts[kCounterWords];
+    if (int st = b2co_oa_insert_counted(t, pairs, stencil, n, assign, cs(s), counts)) return st;
+    if (failed) *failed = counts[kCountFailed];
+    if (assigned) *assigned = counts[kCountAssigned];
     return B2CO_OK;
 }
 

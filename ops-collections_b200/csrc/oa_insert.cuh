@@ -1,6 +1,6 @@
-// oa_insert.cuh -- cooperative-window kernels for the write side of the
-// open-addressing containers: Insert / InsertIf, InsertOrAssign, InsertAndFind
-// (race) and the placement pass of first-wins InsertAndFind.
+// oa_insert.cuh -- the write kernel of large tables: Insert / InsertIf,
+// InsertOrAssign, InsertAndFind (race) and the placement pass of first-wins
+// InsertAndFind.
 //
 // Per-key algorithm (InsertVerdict, open_addressing_ref_impl.h:489-532): walk
 // the key's probe sequence bucket window by bucket window; in a window the
@@ -11,225 +11,150 @@
 // winner holds an equal key (DUPLICATE).  A whole cycle without a decision, or
 // the empty key itself, is FAILED.
 //
-// B200 shape (the lookup kernels' machinery applied to writes):
-//  * G lanes share a bucket window: lane r loads slots r, r+G, ... with one
-//    coherent 16-byte-or-narrower load each, so a window is one or two
-//    coalesced requests, not a chain of dependent slot loads;
-//  * each tile keeps Q keys in flight; the tile agrees on the first deciding
-//    slot by a min over shuffles, and the lane holding that slot issues the
-//    CAS, whose returned value settles a lost race without another load;
-//  * a key whose first window decides nothing goes to the warp's queue in
-//    shared memory and is followed later, a pass of queued keys at a time, so
-//    a pass waits on one window load and one CAS, never on a long probe;
-//  * the window is a snapshot: slots only ever go from empty to occupied
-//    during these kernels, so a slot seen occupied by another key stays so,
-//    and a slot seen empty is re-checked by the CAS itself.
-// Every loop is bounded by the probe cycle (and a lost CAS retries a slot a
-// bounded number of times), so no kernel can spin.
+// As in the sector kernels (oa_sector.cuh) a lane owns a key, hashes it, issues
+// its CAS and queues it.  Between, the warp reads its 32 windows in G sub-passes
+// of 32/G windows: the G lanes of a tile read one sector each, so a window is
+// one load instruction and one or two requests, all sub-passes in flight
+// together.  HBM answers a missed request, not a byte, at a time, which is why
+// large tables want a window in as few requests as it takes.  A tile agrees by
+// one ballot (the lowest lane holding a deciding slot), and the owner gets the
+// slot's place by one shuffle.
+//
+// The window is a snapshot, and that is safe: during these kernels slots only
+// go from empty to occupied, so a slot seen occupied by another key stays so,
+// and a slot seen empty is re-checked by the CAS itself.
+//
+// Bound by HBM's random accesses, a read of the window and the write-back of a
+// slot per key.  134 M pairs into a half-full 4.3 GB table: 17.4 Gpairs/s, against
+// 15.2 with one key per four lanes (a slot a lane, two loads a window, 8 keys in
+// flight a warp and not 32).
+// Every loop is bounded by the probe cycle, so no kernel can spin.
 #pragma once
 
 #include "oa_sector.cuh"
 
 namespace b2co {
 
-// Coherent window loads (L2, never a stale L1 line) with the 64-byte fill hint.
-__device__ __forceinline__ uint32_t ld_win(uint32_t const* p)
-{
-    uint32_t v;
-    asm volatile("ld.relaxed.gpu.global.L2::64B.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ unsigned long long ld_win(unsigned long long const* p)
-{
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.L2::64B.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ U128 ld_win(U128 const* p)
-{
-    unsigned long long lo, hi;
-    asm volatile("ld.relaxed.gpu.global.L2::64B.v2.u64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
-    return U128{lo, hi};
-}
-__device__ __forceinline__ unsigned short ld_win(unsigned short const* p)
-{
-    unsigned short v;
-    asm volatile("ld.relaxed.gpu.global.L2::64B.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
-    return v;
-}
+template <class S, int B>
+constexpr int kTileLanes = SectorWindow<S, B>::NS <= 1 ? 1 : SectorWindow<S, B>::NS <= 2 ? 2 : 4;
 
-enum { kWinOpen = 0, kWinSettled = 1, kWinIdle = 2, kWinExhausted = 3 };
-
-// Resolution of the bucket windows of the Q keys each tile has in flight (the
-// whole warp calls it; tiles whose state is not kWinOpen only take part in the
-// shuffles).  On return a key's state is kWinSettled (verdict, slot and, for
-// the race mode, the found payload set on every lane of the tile) or
-// kWinExhausted (no slot of the window decided: probe on).  The first deciding
-// slot of every key is found, then the CASes of all Q keys are issued back to
-// back before any result is awaited, so a pass waits on one CAS round trip
-// instead of Q.  A lost CAS updates the snapshot with the winner; a torn read
-// retries the slot; a slot that keeps changing (not seen in practice) gives
-// the rest of the window up after a bounded number of rounds.
-template <class S, int B, int G, int Q, int ROUNDS, int MODE>
-__device__ __forceinline__ void tile_insert_windows(OaArgs const& a, typename S::Raw* const (&win_base)[Q],
-                                                    typename S::Raw (&w)[Q][ROUNDS], uint64_t const (&key)[Q],
-                                                    uint64_t const (&val)[Q], uint32_t r, uint32_t lane0,
-                                                    int (&state)[Q], int (&verdict)[Q], int (&slot)[Q],
-                                                    uint64_t (&found)[Q])
-{
-    using Raw = typename S::Raw;
-    uint32_t skip[Q];
-#pragma unroll
-    for (int q = 0; q < Q; ++q) skip[q] = 0;
-    for (int guard = 0; guard < 4 * B + 8; ++guard) {
-        bool open = false;
-#pragma unroll
-        for (int q = 0; q < Q; ++q) open = open || state[q] == kWinOpen;
-        if (!__any_sync(0xffffffffu, open)) return;
-        int s[Q], own[Q], outcome[Q];
-        Raw mine[Q], old[Q];
-        uint64_t got[Q];
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            own[q] = kNoStop;
-            mine[q] = Raw{};
-            if (state[q] == kWinOpen) {
-#pragma unroll
-                for (int t = ROUNDS - 1; t >= 0; --t) {
-                    int const j = int(r) + t * G;
-                    if (j < B && !((skip[q] >> j) & 1u)) {
-                        uint64_t const k = S::key(w[q][t]);
-                        if (k == a.empty_key || S::key_eq(k, key[q])) {
-                            own[q] = j;
-                            mine[q] = w[q][t];
-                        }
-                    }
-                }
-            }
-            s[q] = own[q];
-#pragma unroll
-            for (int o = 1; o < G; o <<= 1) s[q] = min(s[q], __shfl_xor_sync(0xffffffffu, s[q], o));
-        }
-        // issue: every key's deciding lane starts its CAS (or settles a duplicate)
-        Raw expected[Q];
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            outcome[q] = 0;
-            got[q] = 0;
-            if (state[q] == kWinOpen && s[q] != kNoStop && own[q] == s[q]) {
-                Raw* sp = win_base[q] + s[q];
-                if (S::key(mine[q]) != a.empty_key) {
-                    outcome[q] = 2;
-                    if constexpr (MODE == kInsAssign) assign_payload<S>(sp, key[q], val[q]);
-                    if constexpr (MODE == kInsIafRace) got[q] = S::value(settle<S>(a, sp, mine[q]));
-                } else if (!insert_expected<S>(a, mine[q], expected[q])) {
-                    outcome[q] = 5;
-                } else {
-                    outcome[q] = -1;  // CAS in flight
-                    old[q] = cas_slot(sp, expected[q], insert_desired<S>(mine[q], key[q], val[q]));
-                }
-            }
-        }
-        // settle the CASes
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            if (outcome[q] == -1) {
-                Raw* sp = win_base[q] + s[q];
-                if (raw_eq(old[q], expected[q])) {
-                    outcome[q] = 1;
-                    got[q] = S::is_set ? key[q] : val[q];
-                } else if (S::key_eq(S::key(old[q]), key[q])) {
-                    outcome[q] = 2;
-                    if constexpr (MODE == kInsAssign) assign_payload<S>(sp, key[q], val[q]);
-                    got[q] = S::value(old[q]);
-                } else {
-                    outcome[q] = S::key(old[q]) == a.empty_key ? 4 : 3;
-                }
-#pragma unroll
-                for (int t = 0; t < ROUNDS; ++t)
-                    if (int(r) + t * G == s[q]) w[q][t] = old[q];
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            int const src = int(lane0) + (s[q] == kNoStop ? 0 : s[q] % G);
-            int const oc = __shfl_sync(0xffffffffu, outcome[q], src);
-            uint64_t g = 0;
-            if constexpr (MODE == kInsIafRace) g = __shfl_sync(0xffffffffu, (unsigned long long)got[q], src);
-            if (state[q] == kWinOpen) {
-                if (s[q] == kNoStop) {
-                    state[q] = kWinExhausted;
-                } else if (oc == 1 || oc == 2) {
-                    state[q] = kWinSettled;
-                    verdict[q] = oc == 1 ? kSuccess : kDuplicate;
-                    slot[q] = s[q];
-                    found[q] = g;
-                } else if (oc == 5) {
-                    skip[q] |= 1u << s[q];
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < Q; ++q)
-        if (state[q] == kWinOpen) state[q] = kWinExhausted;
-}
-
-// Resident blocks per SM the write kernel is compiled for: one key per lane
-// group fits 64 registers; more keys in flight keep their windows, snapshots
-// and CAS operands live at once and get the registers of two blocks per SM
-// instead of spilling.
-#ifndef B2CO_WRITE_MINB1
-#define B2CO_WRITE_MINB1 4
+#ifndef B2CO_TILE_WRITE_MINB
+#define B2CO_TILE_WRITE_MINB(G) ((G) >= 4 ? 3 : 4)
 #endif
-template <int Q>
-constexpr int kWriteMinBlocks = Q == 1 ? B2CO_WRITE_MINB1 : 2;
 
-template <class S, int B, int G, int Q, int MODE>
-__global__ void __launch_bounds__(256, kWriteMinBlocks<Q>) k_insert_win(__grid_constant__ const OaArgs a, void const* pairs,
-                                                       uint8_t const* stencil, uint32_t n, InsOut o)
+template <class S, int B, int MODE>
+__global__ void __launch_bounds__(256, B2CO_TILE_WRITE_MINB((kTileLanes<S, B>)))
+    k_insert_tile(__grid_constant__ const OaArgs a, void const* pairs, uint8_t const* stencil, uint32_t n,
+                  __grid_constant__ const InsOut o)
 {
-    static_assert(Q <= G && G <= 8 && (G & (G - 1)) == 0, "tile shape");
     using Raw = typename S::Raw;
-    constexpr int ROUNDS = (B + G - 1) / G;
-    constexpr uint32_t TILES = 32 / G;
-    constexpr uint32_t PASS = TILES * Q;
-    static_assert(2 * PASS <= kDeferRing, "the ring must hold a pass on top of a partial one");
-    constexpr uint32_t RING = kDeferRing - 1;
-    __shared__ Raw qpair[8][kDeferRing];
-    __shared__ uint32_t qinit[8][kDeferRing], qidx[8][kDeferRing], qpos[8][kDeferRing];
+    constexpr int G = kTileLanes<S, B>;
+    static_assert(SectorWindow<S, B>::NS <= G && G * (32 / S::bytes) <= 32, "tile shape");
+    constexpr uint32_t TILES = 32 / G, TM = (1u << G) - 1u, N = 32 / S::bytes;
+    constexpr uint32_t RING = kSectorRing - 1;
+    __shared__ Raw qpair[8][kSectorRing];
+    __shared__ uint32_t qinit[8][kSectorRing], qidx[8][kSectorRing], qpos[8][kSectorRing];
 
-    Raw* slots = reinterpret_cast<Raw*>(a.slots);
     uint32_t const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t const r = lane % G, tile_lane0 = lane & ~uint32_t(G - 1), tile = lane / G;
-    uint32_t const gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint32_t const nwarps = (gridDim.x * blockDim.x) >> 5;
+    uint32_t const r = lane % G, tile = lane / G;
+    uint32_t const own_q = lane / TILES, own_shift = (lane % TILES) * G;  // who reads this lane's window
+    uint32_t const stride = gridDim.x * blockDim.x;
+    uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
     uint32_t head = 0, count = 0;
-    uint32_t failed = 0, assigned = 0;
+    Raw* const slots = reinterpret_cast<Raw*>(a.slots);
+    InsRecord<S, MODE> record;
 
-    // The tile's first lane records a decided key.
-    auto record = [&](uint32_t i, int verdict, uint32_t where, uint64_t key, uint64_t found) {
-        if constexpr (MODE == kInsPlain || MODE == kInsAssign) {
-            // Insert succeeds only on SUCCESS (open_addressing_ref_impl.h:282-285);
-            // InsertOrAssign counts a duplicate as an assignment instead.
-            failed += MODE == kInsAssign ? verdict == kFailed : verdict != kSuccess;
-            assigned += verdict == kDuplicate;
-        } else if constexpr (MODE == kInsIafRace) {
-            Io<S>::store_payload(o.found, i, verdict == kFailed ? empty_payload<S>(a) : found);
-            o.inserted[i] = verdict == kSuccess;
-        } else {
-            uint32_t const p = verdict == kFailed ? kNoSlot : where;
-            if (verdict == kSuccess) {
-                atomicOr(o.newbits + (p >> 5), 1u << (p & 31));
-                if (!o.claim_bit) o.owner[p] = i;  // tables without room for the claim bit
+    bool next_in = base + lane < n && (!stencil || stencil[base + lane]);
+    Raw next_pair = next_in ? Io<S>::load_pair(pairs, base + lane) : Raw{};
+    for (;;) {
+        Raw pr;
+        uint32_t init, idx, pos;
+        bool live;
+        if (count >= 32 || base >= n) {
+            if (count == 0) break;
+            __syncwarp();
+            uint32_t const take = count < 32 ? count : 32;
+            live = lane < take;
+            uint32_t const e = (head + (live ? lane : 0u)) & RING;
+            pr = qpair[warp][e];
+            init = qinit[warp][e];
+            idx = qidx[warp][e];
+            pos = qpos[warp][e];
+            __syncwarp();
+            head = (head + take) & RING;
+            count -= take;
+            idx = probe_next(idx, probe_step<S::key_bytes, B>(a.probe, S::key(pr)), a.probe.capacity);
+            if (live && idx == init) {
+                record(a, o, pos, kFailed, 0, 0);
+                live = false;
             }
-            o.pos[i] = verdict == kSuccess ? (p | o.claim_bit) : p;
+        } else {
+            pos = base + lane;
+            pr = next_pair;
+            live = next_in;
+            if (live && S::key(pr) == a.empty_key) {
+                record(a, o, pos, kFailed, 0, 0);
+                live = false;
+            }
+            init = idx = probe_init<S::key_bytes, B>(a.probe, S::key(pr));
+            base += stride;
+            next_in = base < n && base + lane < n && (!stencil || stencil[base + lane]);
+            next_pair = next_in ? Io<S>::load_pair(pairs, base + lane) : Raw{};
         }
-        (void)key;
-    };
-    auto enqueue = [&](bool unsettled, Raw const& pr, uint32_t init, uint32_t idx, uint32_t pos) {
-        uint32_t const m = __ballot_sync(0xffffffffu, unsettled);
-        if (unsettled) {
+        uint64_t const key = S::key(pr);
+        uint32_t const live_mask = __ballot_sync(0xffffffffu, live);
+        Sector w[G];
+        uint64_t k[G];
+        uint32_t valid[G];  // the slots of this lane's sector that lie in the window
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            uint32_t const src = q * TILES + tile;
+            k[q] = S::key_bytes <= 4 ? uint64_t(__shfl_sync(0xffffffffu, uint32_t(key), src))
+                                     : __shfl_sync(0xffffffffu, (unsigned long long)key, src);
+            uint32_t const ix = __shfl_sync(0xffffffffu, idx, src);
+            uintptr_t const addr = reinterpret_cast<uintptr_t>(slots + ix);
+            valid[q] = ((((1u << B) - 1u) << (uint32_t(addr & 31) / S::bytes)) >> (r * N)) & ((1u << N) - 1u);
+            if (!((live_mask >> src) & 1u)) valid[q] = 0;
+            if (valid[q]) w[q] = ld_sector<true, false>(reinterpret_cast<void const*>((addr & ~uintptr_t(31)) + r * 32));
+        }
+        // each owner learns where its window's first deciding slot is and whether it is empty
+        uint32_t mine = 0;  // slot among the window's sectors | 32: empty | 64: found
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            uint32_t info = 0;
+            if (valid[q]) {
+                uint32_t stops = 0, empties = 0;
+#pragma unroll
+                for (int i = 0; i < int(N); ++i) {
+                    uint64_t const sk = S::key(sector_slot<S>(w[q], i));
+                    if (sk == a.empty_key) empties |= 1u << i;
+                    else if (S::key_eq(sk, k[q])) stops |= 1u << i;
+                }
+                stops = (stops | empties) & valid[q];
+                if (stops) {
+                    uint32_t const i = uint32_t(__ffs(stops) - 1);
+                    info = i | (((empties >> i) & 1u) ? 96u : 64u);
+                }
+            }
+            uint32_t const m = (__ballot_sync(0xffffffffu, info != 0) >> own_shift) & TM;
+            uint32_t const first = m ? uint32_t(__ffs(m) - 1) : 0u;
+            uint32_t const got = __shfl_sync(0xffffffffu, info, own_shift + first);
+            if (uint32_t(q) == own_q && m) mine = got + first * N;
+        }
+        int verdict = kOpen;
+        if (live && mine) {
+            Raw* const win = slots + idx;
+            int j = int(mine & 31u) - int(uint32_t(reinterpret_cast<uintptr_t>(win) & 31) / S::bytes);
+            // the slot itself stayed with the tile: a present one is read again where its payload is wanted
+            Raw cur = S::make(a.empty_key, a.empty_value);
+            if (!(mine & 32u)) cur = MODE == kInsIafRace ? ld_rw(win + j) : S::make(~a.empty_key, 0);
+            uint64_t found = 0;
+            verdict = sector_decide<S, B, MODE>(a, win, j, cur, key, S::value(pr), found);
+            if (verdict != kOpen) record(a, o, pos, verdict, idx + uint32_t(j), found);
+        }
+        bool const open = live && verdict == kOpen;
+        uint32_t const m = __ballot_sync(0xffffffffu, open);
+        if (open) {
             uint32_t const e = (head + count + __popc(m & ((1u << lane) - 1u))) & RING;
             qpair[warp][e] = pr;
             qinit[warp][e] = init;
@@ -237,149 +162,8 @@ __global__ void __launch_bounds__(256, kWriteMinBlocks<Q>) k_insert_win(__grid_c
             qpos[warp][e] = pos;
         }
         count += __popc(m);
-    };
-    // Takes up to one pass of queued keys and resolves the next window of each.
-    auto follow = [&]() {
-        __syncwarp();
-        uint32_t const take = count < PASS ? count : PASS;
-        Raw pr[Q];
-        uint32_t init[Q], idx[Q], pos[Q];
-        bool live[Q];
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            uint32_t const j = q * TILES + tile;
-            live[q] = j < take;
-            uint32_t const e = (head + (live[q] ? j : 0u)) & RING;
-            pr[q] = qpair[warp][e];
-            init[q] = qinit[warp][e];
-            idx[q] = qidx[warp][e];
-            pos[q] = qpos[warp][e];
-        }
-        __syncwarp();
-        head = (head + take) & RING;
-        count -= take;
-        uint32_t my_step = 0;
-#pragma unroll
-        for (int q = 0; q < Q; ++q)
-            if (int(r) == q && live[q]) my_step = probe_step<S::key_bytes, B>(a.probe, S::key(pr[q]));
-        Raw w[Q][ROUNDS];
-        int state[Q];
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            uint32_t const step = __shfl_sync(0xffffffffu, my_step, tile_lane0 + q);
-            state[q] = live[q] ? kWinOpen : kWinIdle;
-            if (live[q]) {
-                idx[q] = probe_next(idx[q], step, a.probe.capacity);
-                if (idx[q] == init[q]) {  // a whole cycle: the table is full for this key
-                    if (r == 0) record(pos[q], kFailed, 0, S::key(pr[q]), 0);
-                    state[q] = kWinIdle;
-                }
-            }
-            if (state[q] == kWinOpen) {
-#pragma unroll
-                for (int t = 0; t < ROUNDS; ++t)
-                    if (int(r) + t * G < B) w[q][t] = ld_win(slots + idx[q] + r + t * G);
-            }
-        }
-        {
-            Raw* base[Q];
-            uint64_t key[Q], val[Q], found[Q];
-            int verdict[Q], slot[Q];
-#pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                base[q] = slots + idx[q];
-                key[q] = S::key(pr[q]);
-                val[q] = S::value(pr[q]);
-                verdict[q] = kFailed;
-                slot[q] = 0;
-                found[q] = 0;
-            }
-            tile_insert_windows<S, B, G, Q, ROUNDS, MODE>(a, base, w, key, val, r, tile_lane0, state, verdict, slot,
-                                                          found);
-#pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                if (state[q] == kWinSettled && r == 0) record(pos[q], verdict[q], idx[q] + slot[q], key[q], found[q]);
-                enqueue(state[q] == kWinExhausted && r == 0, pr[q], init[q], idx[q], pos[q]);
-            }
-        }
-    };
-
-    // the next pass's pairs are loaded one pass ahead (B2CO_WRITE_PREFETCH 0:
-    // at the start of their own pass)
-#ifndef B2CO_WRITE_PREFETCH
-#define B2CO_WRITE_PREFETCH 1
-#endif
-    Raw nxt[Q];
-    bool nin[Q];
-    auto load_pass = [&](uint32_t base) {
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            uint32_t const i = base + q * TILES + tile;
-            nin[q] = i < n && (!stencil || stencil[i]);
-            nxt[q] = nin[q] ? Io<S>::load_pair(pairs, i) : Raw{};
-        }
-    };
-    if (B2CO_WRITE_PREFETCH) load_pass(gwarp * PASS);
-    for (uint32_t base = gwarp * PASS; base < n; base += nwarps * PASS) {
-        if (!B2CO_WRITE_PREFETCH) load_pass(base);
-        Raw pr[Q];
-        uint32_t idx[Q];
-        int state[Q];
-        uint32_t my_init = 0;
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            pr[q] = nxt[q];
-            uint64_t const key = S::key(pr[q]);
-            state[q] = !nin[q] ? kWinIdle : (key == a.empty_key ? kWinSettled : kWinOpen);
-            if (int(r) == q && state[q] == kWinOpen) my_init = probe_init<S::key_bytes, B>(a.probe, key);
-        }
-        if (B2CO_WRITE_PREFETCH) load_pass(base + nwarps * PASS);
-        Raw w[Q][ROUNDS];
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            idx[q] = __shfl_sync(0xffffffffu, my_init, tile_lane0 + q);
-            if (state[q] == kWinOpen) {
-#pragma unroll
-                for (int t = 0; t < ROUNDS; ++t)
-                    if (int(r) + t * G < B) w[q][t] = ld_win(slots + idx[q] + r + t * G);
-            }
-        }
-        {
-            Raw* wb[Q];
-            uint64_t key[Q], val[Q], found[Q];
-            int verdict[Q], slot[Q];
-#pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                uint32_t const i = base + q * TILES + tile;
-                key[q] = S::key(pr[q]);
-                val[q] = S::value(pr[q]);
-                wb[q] = slots + idx[q];
-                verdict[q] = kFailed;
-                slot[q] = 0;
-                found[q] = 0;
-                if (state[q] == kWinSettled) {  // the empty key itself: FAILED
-                    if (r == 0) record(i, kFailed, 0, key[q], 0);
-                    state[q] = kWinIdle;
-                }
-            }
-            tile_insert_windows<S, B, G, Q, ROUNDS, MODE>(a, wb, w, key, val, r, tile_lane0, state, verdict, slot,
-                                                          found);
-#pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                uint32_t const i = base + q * TILES + tile;
-                if (state[q] == kWinSettled && r == 0) record(i, verdict[q], idx[q] + slot[q], key[q], found[q]);
-                enqueue(state[q] == kWinExhausted && r == 0, pr[q], idx[q], idx[q], i);
-            }
-        }
-        while (count >= PASS) follow();
     }
-    while (count > 0) follow();
-    if constexpr (MODE == kInsPlain || MODE == kInsAssign) {
-        if (o.counters) {
-            block_add_counter(o.counters, failed);
-            if (MODE == kInsAssign) block_add_counter(o.counters + 1, assigned);
-        }
-    }
+    record.finish(o);
 }
 
 }  // namespace b2co

@@ -86,49 +86,26 @@ struct OaImpl {
                (lanes == 0 && table_bytes(a) <= (mode == kInsAssign ? kSectorAssignBytes : kSectorInsertBytes));
     }
 
+    // A write of one mode.
     template <int B, int MODE>
-    static int launch_sector_write(OaArgs const& a, void const* pairs, uint8_t const* stencil, uint32_t n,
-                                   InsOut const& o, cudaStream_t s)
+    static int write(OaArgs const& a, void const* pairs, uint8_t const* stencil, uint32_t n, InsOut const& o,
+                     cudaStream_t s)
     {
+        if constexpr (B > 1) {
+            if (!sector_writes(a, B, MODE)) {
+                auto k = k_insert_tile<S, B, MODE>;
+                k<<<grid_for((void const*)k, kBlock, n, kBlock), kBlock, 0, s>>>(a, pairs, stencil, n, o);
+                return check_launch("insert kernel");
+            }
+        }
         auto k = k_insert_sector<S, B, MODE>;
         uint32_t const block = sector_block(n);
         k<<<grid_for((void const*)k, block, n, block), block, 0, s>>>(a, pairs, stencil, n, o);
         return check_launch("insert kernel");
     }
 
-    // A write of one mode: the sector kernel, or the table's cooperative shape.
-    template <int B, int MODE>
-    static int write(OaArgs const& a, void const* pairs, uint8_t const* stencil, uint32_t n, InsOut const& o,
-                     cudaStream_t s)
-    {
-        if constexpr (B > 1) {
-            if (!sector_writes(a, B, MODE)) return launch_write<B, MODE>(a, pairs, stencil, n, o, s);
-        }
-        return launch_sector_write<B, MODE>(a, pairs, stencil, n, o, s);
-    }
-
-    // Cooperative-window write kernel (oa_insert.cuh) of the table's shape.
-    template <int B, int MODE>
-    static int launch_write(OaArgs const& a, void const* pairs, uint8_t const* stencil, uint32_t n, InsOut const& o,
-                            cudaStream_t s)
-    {
-        uint32_t lanes = a.write_shape >> 8, items = a.write_shape & 0xffu;
-        if (lanes == 0) lanes = 4, items = 1;  // default: 4 lanes per window, one key per lane group
-        void (*k)(OaArgs, void const*, uint8_t const*, uint32_t, InsOut) = nullptr;
-        if constexpr (kAllShapes && B == 5) {  // other shapes: the common bucket size only (build time)
-            if (lanes == 2) k = items >= 2 ? k_insert_win<S, B, 2, 2, MODE> : k_insert_win<S, B, 2, 1, MODE>;
-            else if (lanes == 8) k = items >= 4 ? k_insert_win<S, B, 8, 4, MODE> : k_insert_win<S, B, 8, 2, MODE>;
-            else if (items == 2) k = k_insert_win<S, B, 4, 2, MODE>;
-            else if (items >= 4) k = k_insert_win<S, B, 4, 4, MODE>;
-        }
-        if (!k) lanes = 4, items = 1, k = k_insert_win<S, B, 4, 1, MODE>;
-        uint64_t const per_block = (kBlock / 32) * (32 / lanes) * items;
-        k<<<grid_for((void const*)k, kBlock, n, per_block), kBlock, 0, s>>>(a, pairs, stencil, n, o);
-        return check_launch("insert kernel");
-    }
-
     static int insert(OaArgs const& a, uint32_t b, void const* pairs, uint8_t const* stencil, uint32_t n,
-                      bool assign, unsigned long long* counters, cudaStream_t s)
+                      bool assign, Counters const& counters, cudaStream_t s)
     {
         return with_b(b, [&](auto bc) {
             constexpr int B = decltype(bc)::value;
@@ -230,21 +207,30 @@ struct OaImpl {
 
     using DeferFn = void (*)(OaArgs, void const*, void*, uint32_t, uint32_t, WaitCtl);
 
-    // Keys per warp and stage: the batch dealt evenly over the resident warps in
-    // stages of at most kWarpStageKeys, so a batch that cannot fill every warp's
-    // stage still reaches every warp (a stage is a chain of dependent passes:
-    // 65,536 keys in whole stages ran 16 of them one after the other on 32 blocks,
-    // 16.1 us against 10.1).
+    // Resident warps of a deferred lookup.
+    static uint64_t defer_warps(DeferFn k) { return uint64_t(grid_for((void const*)k, kBlock, ~0ull, 1)) * (kBlock / 32); }
+
     static int launch_wdefer(DeferFn k, bool contains, OaArgs const& a, void const* keys, void* out, uint32_t n,
-                             WaitCtl wc, cudaStream_t s)
+                             uint64_t chunk, WaitCtl wc, cudaStream_t s)
     {
-        uint64_t const warps = uint64_t(grid_for((void const*)k, kBlock, ~0ull, 1)) * (kBlock / 32);
-        uint64_t const share = (n + warps - 1) / warps;
-        uint64_t const rounds = (share + kWarpStageKeys - 1) / kWarpStageKeys;
-        uint64_t const chunk = ((share + rounds - 1) / rounds + 31) / 32 * 32;
         k<<<grid_for((void const*)k, kBlock, (n + chunk - 1) / chunk, kBlock / 32), kBlock, 0, s>>>(
             a, keys, out, n, uint32_t(chunk), wc);
         return check_launch(contains ? "contains kernel" : "find kernel");
+    }
+
+    // The default deferred lookup.  A batch that does not fill every resident
+    // warp's stage is dealt evenly over them (a stage is a chain of dependent
+    // passes: 65,536 keys in whole stages ran 16 of them one after the other on 32
+    // blocks, 16.1 us against 10.1).
+    template <int B, int G, int Q, bool C>
+    static int find_defer_auto(OaArgs const& a, void const* keys, void* out, uint32_t n, WaitCtl wc, cudaStream_t s)
+    {
+        DeferFn const even = k_find_wdefer<S, B, G, Q, C, true>;
+        uint64_t const share = (n + defer_warps(even) - 1) / defer_warps(even);
+        if (share >= kWarpStageKeys)
+            return launch_wdefer(k_find_wdefer<S, B, G, Q, C>, C, a, keys, out, n, kWarpStageKeys, wc, s);
+        uint64_t const rounds = (share + kWarpStageKeys - 1) / kWarpStageKeys;
+        return launch_wdefer(even, C, a, keys, out, n, ((share + rounds - 1) / rounds + 31) / 32 * 32, wc, s);
     }
 
     template <int B, int G, bool C>
@@ -255,7 +241,7 @@ struct OaImpl {
         if (items >= 4 && G >= 4) k = k_find_wdefer<S, B, G, (G >= 4 ? 4 : 1), C>;
         else if (items >= 2) k = k_find_wdefer<S, B, G, 2, C>;
         else k = k_find_wdefer<S, B, G, 1, C>;
-        return launch_wdefer(k, C, a, keys, out, n, wc, s);
+        return launch_wdefer(k, C, a, keys, out, n, kWarpStageKeys, wc, s);
     }
 
     template <int B, bool C>
@@ -277,8 +263,10 @@ struct OaImpl {
         if constexpr (B > 1) {
             if ((table_bytes(a) > kSectorFindBytes || S::bytes <= 4) && n > kSectorFindKeys) {
                 bool const narrow = S::bytes <= 4 || table_bytes(a) <= kNarrowFindBytes;
-                return find_shape<B, C>(a, narrow ? 2 : 4, (narrow ? 1 : 2) | kShapeDeferred, keys, stencil, out, n, wc,
-                                        s);
+                if (stencil || (reinterpret_cast<uintptr_t>(keys) & 15))  // keys cannot be staged
+                    return find_shape<B, C>(a, narrow ? 2 : 4, 1, keys, stencil, out, n, wc, s);
+                return narrow ? find_defer_auto<B, 2, 1, C>(a, keys, out, n, wc, s)
+                              : find_defer_auto<B, 4, 2, C>(a, keys, out, n, wc, s);
             }
         }
         return find_sector<B, C>(a, keys, stencil, out, n, s);
@@ -322,7 +310,7 @@ struct OaImpl {
             DeferFn k = nullptr;
             if (lanes == 2) k = q == 2 ? k_find_wdefer<S, B, 2, 2, C> : k_find_wdefer<S, B, 2, 1, C>;
             else k = q == 2 ? k_find_wdefer<S, B, 4, 2, C> : k_find_wdefer<S, B, 4, 1, C>;
-            return launch_wdefer(k, C, a, keys, out, n, wc, s);
+            return launch_wdefer(k, C, a, keys, out, n, kWarpStageKeys, wc, s);
         }
         if (B == 1 || lanes <= 1) return find_sector<B, C>(a, keys, stencil, out, n, s);
         uint64_t const per_block = lanes == 2 ? kBlock / 2 : kBlock / 4;

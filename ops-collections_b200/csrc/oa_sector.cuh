@@ -27,21 +27,36 @@ struct alignas(32) Sector {
     unsigned long long w[4];
 };
 
-__device__ __forceinline__ Sector ld_sector_ro(void const* p)
+// A sector, coherently (L2, never a stale L1 line) for kernels that race with
+// writers, else through the read-only path.  A missed sector brings 64 bytes
+// from HBM, or 128 with WIDE, where the neighbours will be wanted as well.
+#ifndef B2CO_WIDE_FILL
+#define B2CO_WIDE_FILL "128B"
+#endif
+template <bool COHERENT, bool WIDE>
+__device__ __forceinline__ Sector ld_sector(void const* p)
 {
     Sector v;
-    asm(B2CO_LD_RO ".v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(v.w[0]), "=l"(v.w[1]), "=l"(v.w[2]), "=l"(v.w[3]) : "l"(p));
+#define B2CO_LD_SECTOR(volatility, op, fill, clobber)                                     \
+    asm volatility("ld." op ".L2::" fill ".v4.u64 {%0, %1, %2, %3}, [%4];"                \
+                   : "=l"(v.w[0]), "=l"(v.w[1]), "=l"(v.w[2]), "=l"(v.w[3])               \
+                   : "l"(p)                                                               \
+                   clobber)
+    if constexpr (COHERENT && WIDE) B2CO_LD_SECTOR(volatile, "relaxed.gpu.global", B2CO_WIDE_FILL, : "memory");
+    else if constexpr (COHERENT) B2CO_LD_SECTOR(volatile, "relaxed.gpu.global", "64B", : "memory");
+    else if constexpr (WIDE) B2CO_LD_SECTOR(, "global.nc", B2CO_WIDE_FILL, );
+    else B2CO_LD_SECTOR(, "global.nc", "64B", );
+#undef B2CO_LD_SECTOR
     return v;
 }
-// Coherent (L2, never a stale L1 line), for kernels that race with writers.
-__device__ __forceinline__ Sector ld_sector_rw(void const* p)
+
+template <class S>
+__device__ __forceinline__ typename S::Raw sector_slot(Sector const& w, int i)
 {
-    Sector v;
-    asm volatile("ld.relaxed.gpu.global.L2::64B.v4.u64 {%0, %1, %2, %3}, [%4];"
-                 : "=l"(v.w[0]), "=l"(v.w[1]), "=l"(v.w[2]), "=l"(v.w[3])
-                 : "l"(p)
-                 : "memory");
-    return v;
+    if constexpr (S::bytes == 16) return U128{w.w[2 * i], w.w[2 * i + 1]};
+    else if constexpr (S::bytes == 8) return w.w[i];
+    else if constexpr (S::bytes == 4) return typename S::Raw(w.w[i / 2] >> (32 * (i % 2)));
+    else return typename S::Raw(w.w[i / 4] >> (16 * (i % 4)));
 }
 
 constexpr uint32_t gcd_u32(uint32_t a, uint32_t b) { return b == 0 ? a : gcd_u32(b, a % b); }
@@ -59,7 +74,7 @@ struct SectorWindow {
     Sector s[NS];
     uint32_t off;  // the window's first slot within its first sector
 
-    template <bool COHERENT>
+    template <bool COHERENT, bool WIDE = false>
     __device__ __forceinline__ void load(Raw const* win)
     {
         uintptr_t const addr = reinterpret_cast<uintptr_t>(win);
@@ -69,18 +84,10 @@ struct SectorWindow {
         for (int i = 0; i < NS; ++i) {
             // the last sector is covered only when the window starts late enough in the first
             bool const need = i == 0 || off + B > uint32_t(i) * N;
-            if (need) s[i] = COHERENT ? ld_sector_rw(p + 32 * i) : ld_sector_ro(p + 32 * i);
+            if (need) s[i] = ld_sector<COHERENT, WIDE>(p + 32 * i);
         }
     }
-    __device__ __forceinline__ Raw slot(int j) const
-    {
-        Sector const& w = s[j / N];
-        int const i = j % N;
-        if constexpr (S::bytes == 16) return U128{w.w[2 * i], w.w[2 * i + 1]};
-        else if constexpr (S::bytes == 8) return w.w[i];
-        else if constexpr (S::bytes == 4) return Raw(w.w[i / 2] >> (32 * (i % 2)));
-        else return Raw(w.w[i / 4] >> (16 * (i % 4)));
-    }
+    __device__ __forceinline__ Raw slot(int j) const { return sector_slot<S>(s[j / N], j % N); }
     // First slot of the window, in scan order, that is empty or holds an equal
     // key: its place among the loaded slots (window slot + off), or -1.
     __device__ __forceinline__ int first_stop(uint64_t key, uint64_t empty_key) const
@@ -131,10 +138,6 @@ __global__ void __launch_bounds__(256, B2CO_SECTOR_FIND_MINB((SectorWindow<S, B>
     uint32_t head = 0, count = 0;  // queue state, the same on every lane
     Raw const* const slots = reinterpret_cast<Raw const*>(a.slots);
 
-    auto store = [&](uint32_t pos, bool hit, uint64_t payload) {
-        if constexpr (CONTAINS) reinterpret_cast<uint8_t*>(out)[pos] = hit;
-        else Io<S>::store_payload(out, pos, payload);
-    };
     // the next pass's key is loaded one pass ahead
     uint64_t next_key = base + lane < n ? Io<S>::load_key(keys, base + lane) : 0;
     for (;;) {
@@ -156,7 +159,7 @@ __global__ void __launch_bounds__(256, B2CO_SECTOR_FIND_MINB((SectorWindow<S, B>
             count -= take;
             idx = probe_next(idx, probe_step<S::key_bytes, B>(a.probe, key), a.probe.capacity);
             if (live && idx == init) {  // full cycle: not present
-                store(pos, false, empty_payload<S>(a));
+                store_result<S, CONTAINS>(a, out, pos, false, 0);
                 live = false;
             }
         } else {
@@ -164,7 +167,7 @@ __global__ void __launch_bounds__(256, B2CO_SECTOR_FIND_MINB((SectorWindow<S, B>
             key = next_key;
             live = pos < n;
             if (stencil && live && !stencil[pos]) {
-                store(pos, false, empty_payload<S>(a));
+                store_result<S, CONTAINS>(a, out, pos, false, 0);
                 live = false;
             }
             init = idx = probe_init<S::key_bytes, B>(a.probe, key);
@@ -178,8 +181,7 @@ __global__ void __launch_bounds__(256, B2CO_SECTOR_FIND_MINB((SectorWindow<S, B>
             int const j = w.first_stop(key, a.empty_key);
             if (j >= 0) {
                 Raw const slot = w.pick(j);
-                bool const hit = S::key(slot) != a.empty_key;
-                store(pos, hit, hit ? S::value(slot) : empty_payload<S>(a));
+                store_result<S, CONTAINS>(a, out, pos, S::key(slot) != a.empty_key, S::value(slot));
             } else {
                 open = true;
             }
@@ -204,13 +206,53 @@ enum { kInsPlain = 0, kInsAssign = 1, kInsIafRace = 2, kInsIafPlace = 3 };
 
 // Outputs of one insert-family launch (only the mode's fields are used).
 struct InsOut {
-    unsigned long long* counters;  // plain/assign: [failed, assigned] or NULL (async)
-    void* found;                   // race: payload found or inserted
-    uint8_t* inserted;             // race: 1 = this input inserted the key
-    uint32_t* pos;                 // place: slot of every input (kNoSlot = failed)
-    uint32_t* newbits;             // place: slots claimed by this batch
-    uint32_t* owner;               // place: claiming input of each claimed slot (claim_bit 0 only)
-    uint32_t claim_bit;            // place: flag OR-ed into pos[] of the claiming input (0 = none)
+    Counters counters;   // plain/assign
+    void* found;         // race: payload found or inserted
+    uint8_t* inserted;   // race: 1 = this input inserted the key
+    uint32_t* pos;       // place: slot of every input (kNoSlot = failed)
+    uint32_t* newbits;   // place: slots claimed by this batch
+    uint32_t* owner;     // place: claiming input of each claimed slot (claim_bit 0 only)
+    uint32_t claim_bit;  // place: flag OR-ed into pos[] of the claiming input (0 = none)
+};
+
+// What a decided key leaves behind, by mode; one per thread.
+template <class S, int MODE>
+struct InsRecord {
+    uint32_t failed = 0, assigned = 0, selected = 0;
+    __device__ __forceinline__ void operator()(OaArgs const& a, InsOut const& o, uint32_t i, int verdict, uint32_t where,
+                                               uint64_t found)
+    {
+        if constexpr (MODE == kInsPlain || MODE == kInsAssign) {
+            // Insert succeeds only on SUCCESS (open_addressing_ref_impl.h:282-285);
+            // InsertOrAssign counts a duplicate as an assignment instead.
+            failed += MODE == kInsAssign ? verdict == kFailed : verdict != kSuccess;
+            assigned += verdict == kDuplicate;
+            ++selected;
+        } else if constexpr (MODE == kInsIafRace) {
+            Io<S>::store_payload(o.found, i, verdict == kFailed ? empty_payload<S>(a) : found);
+            o.inserted[i] = verdict == kSuccess;
+        } else {
+            uint32_t const p = verdict == kFailed ? kNoSlot : where;
+            if (verdict == kSuccess) {
+                atomicOr(o.newbits + (p >> 5), 1u << (p & 31));
+                if (!o.claim_bit) o.owner[p] = i;  // tables without room for the claim bit
+            }
+            o.pos[i] = verdict == kSuccess ? (p | o.claim_bit) : p;
+        }
+    }
+    __device__ __forceinline__ void finish(InsOut const& o) const  // every thread of the block
+    {
+        if constexpr (MODE == kInsPlain || MODE == kInsAssign) {
+            if (o.counters.sum) {
+                block_add_counter(o.counters.sum + kCountFailed, failed);
+                if (MODE == kInsAssign) {
+                    block_add_counter(o.counters.sum + kCountAssigned, assigned);
+                }
+                if (o.counters.host) block_add_counter(o.counters.sum + kCountSelected, selected);
+                finish_counters(o.counters);
+            }
+        }
+    }
 };
 
 enum { kOpen = 3 };  // no verdict yet: the key goes on to its next window
@@ -246,13 +288,32 @@ __device__ __forceinline__ int sector_claim(OaArgs const& a, typename S::Raw* wi
     return kOpen;
 }
 
+// What an owner does with its window's first deciding slot `cur` (window slot j):
+// claims it when it is empty, otherwise its key is present.  Returns the verdict,
+// kOpen when the window turned out exhausted after all.
+template <class S, int B, int MODE>
+__device__ __forceinline__ int sector_decide(OaArgs const& a, typename S::Raw* win, int& j, typename S::Raw cur,
+                                             uint64_t key, uint64_t val, uint64_t& found)
+{
+    bool const empty = S::key(cur) == a.empty_key;
+    int const verdict = empty ? sector_claim<S, B>(a, win, key, val, j, cur) : int(kDuplicate);
+    if (verdict == kDuplicate) {
+        if constexpr (MODE == kInsAssign) assign_payload<S>(win + j, key, val);
+        if constexpr (MODE == kInsIafRace) found = S::value(settle<S>(a, win + j, cur));
+    } else if (verdict == kSuccess) {
+        found = S::is_set ? key : val;
+    }
+    return verdict;
+}
+
 #ifndef B2CO_SECTOR_WRITE_MINB
 #define B2CO_SECTOR_WRITE_MINB(NS) ((NS) >= 3 ? 4 : 5)
 #endif
 
 template <class S, int B, int MODE>
 __global__ void __launch_bounds__(256, B2CO_SECTOR_WRITE_MINB((SectorWindow<S, B>::NS)))
-    k_insert_sector(__grid_constant__ const OaArgs a, void const* pairs, uint8_t const* stencil, uint32_t n, InsOut o)
+    k_insert_sector(__grid_constant__ const OaArgs a, void const* pairs, uint8_t const* stencil, uint32_t n,
+                    __grid_constant__ const InsOut o)
 {
     using Raw = typename S::Raw;
     constexpr uint32_t RING = kSectorRing - 1;
@@ -263,27 +324,10 @@ __global__ void __launch_bounds__(256, B2CO_SECTOR_WRITE_MINB((SectorWindow<S, B
     uint32_t const stride = gridDim.x * blockDim.x;
     uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
     uint32_t head = 0, count = 0;
-    uint32_t failed = 0, assigned = 0;
     Raw* const slots = reinterpret_cast<Raw*>(a.slots);
+    InsRecord<S, MODE> record;
 
-    auto record = [&](uint32_t i, int verdict, uint32_t where, uint64_t found) {
-        if constexpr (MODE == kInsPlain || MODE == kInsAssign) {
-            // Insert succeeds only on SUCCESS (open_addressing_ref_impl.h:282-285);
-            // InsertOrAssign counts a duplicate as an assignment instead.
-            failed += MODE == kInsAssign ? verdict == kFailed : verdict != kSuccess;
-            assigned += verdict == kDuplicate;
-        } else if constexpr (MODE == kInsIafRace) {
-            Io<S>::store_payload(o.found, i, verdict == kFailed ? empty_payload<S>(a) : found);
-            o.inserted[i] = verdict == kSuccess;
-        } else {
-            uint32_t const p = verdict == kFailed ? kNoSlot : where;
-            if (verdict == kSuccess) {
-                atomicOr(o.newbits + (p >> 5), 1u << (p & 31));
-                if (!o.claim_bit) o.owner[p] = i;  // tables without room for the claim bit
-            }
-            o.pos[i] = verdict == kSuccess ? (p | o.claim_bit) : p;
-        }
-    };
+    // the next pass's pair is loaded one pass ahead
     bool next_in = base + lane < n && (!stencil || stencil[base + lane]);
     Raw next_pair = next_in ? Io<S>::load_pair(pairs, base + lane) : Raw{};
     for (;;) {
@@ -292,7 +336,7 @@ __global__ void __launch_bounds__(256, B2CO_SECTOR_WRITE_MINB((SectorWindow<S, B
         bool live;
         if (count >= 32 || base >= n) {
             if (count == 0) break;
-            __syncwarp();
+            __syncwarp();  // the queue writes precede these reads
             uint32_t const take = count < 32 ? count : 32;
             live = lane < take;
             uint32_t const e = (head + (live ? lane : 0u)) & RING;
@@ -300,12 +344,12 @@ __global__ void __launch_bounds__(256, B2CO_SECTOR_WRITE_MINB((SectorWindow<S, B
             init = qinit[warp][e];
             idx = qidx[warp][e];
             pos = qpos[warp][e];
-            __syncwarp();
+            __syncwarp();  // every read of the taken entries precedes their reuse
             head = (head + take) & RING;
             count -= take;
             idx = probe_next(idx, probe_step<S::key_bytes, B>(a.probe, S::key(pr)), a.probe.capacity);
             if (live && idx == init) {  // a whole cycle: the table is full for this key
-                record(pos, kFailed, 0, 0);
+                record(a, o, pos, kFailed, 0, 0);
                 live = false;
             }
         } else {
@@ -313,7 +357,7 @@ __global__ void __launch_bounds__(256, B2CO_SECTOR_WRITE_MINB((SectorWindow<S, B
             pr = next_pair;
             live = next_in;
             if (live && S::key(pr) == a.empty_key) {  // the empty key itself: FAILED
-                record(pos, kFailed, 0, 0);
+                record(a, o, pos, kFailed, 0, 0);
                 live = false;
             }
             init = idx = probe_init<S::key_bytes, B>(a.probe, S::key(pr));
@@ -323,27 +367,16 @@ __global__ void __launch_bounds__(256, B2CO_SECTOR_WRITE_MINB((SectorWindow<S, B
         }
         int verdict = kOpen;
         if (live) {
-            uint64_t const key = S::key(pr), val = S::value(pr);
-            Raw* const win = slots + idx;
+            uint64_t const key = S::key(pr);
             SectorWindow<S, B> w;
-            w.template load<true>(win);
+            w.template load<true>(slots + idx);
             int j = w.first_stop(key, a.empty_key);
             if (j >= 0) {
-                Raw old = w.pick(j);
+                Raw const cur = w.pick(j);
                 j -= int(w.off);
-                if (S::key(old) == a.empty_key) {
-                    verdict = sector_claim<S, B>(a, win, key, val, j, old);
-                } else {
-                    verdict = kDuplicate;
-                }
                 uint64_t found = 0;
-                if (verdict == kDuplicate) {
-                    if constexpr (MODE == kInsAssign) assign_payload<S>(win + j, key, val);
-                    if constexpr (MODE == kInsIafRace) found = S::value(settle<S>(a, win + j, old));
-                } else if (verdict == kSuccess) {
-                    found = S::is_set ? key : val;
-                }
-                if (verdict != kOpen) record(pos, verdict, idx + uint32_t(j), found);
+                verdict = sector_decide<S, B, MODE>(a, slots + idx, j, cur, key, S::value(pr), found);
+                if (verdict != kOpen) record(a, o, pos, verdict, idx + uint32_t(j), found);
             }
         }
         bool const open = live && verdict == kOpen;
@@ -357,12 +390,7 @@ __global__ void __launch_bounds__(256, B2CO_SECTOR_WRITE_MINB((SectorWindow<S, B
         }
         count += __popc(m);
     }
-    if constexpr (MODE == kInsPlain || MODE == kInsAssign) {
-        if (o.counters) {
-            block_add_counter(o.counters, failed);
-            if (MODE == kInsAssign) block_add_counter(o.counters + 1, assigned);
-        }
-    }
+    record.finish(o);
 }
 
 }  // namespace b2co
