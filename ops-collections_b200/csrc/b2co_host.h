@@ -76,6 +76,9 @@ struct OaOps {
     int (*clear)(OaArgs const& a, cudaStream_t s);
     int (*insert)(OaArgs const& a, uint32_t b, void const* pairs, uint8_t const* stencil, uint32_t n, bool assign,
                   Counters const& counters, cudaStream_t s);
+    // absent[i] = 0 for every pair whose key is in the table, whose payload is overwritten when `assign`
+    int (*mark)(OaArgs const& a, uint32_t b, void const* pairs, uint32_t n, bool assign, uint8_t* absent,
+                cudaStream_t s);
     int (*assign_if)(OaArgs const& a, uint32_t b, void const* pairs, uint8_t const* stencil, uint32_t n,
                      cudaStream_t s);
     int (*iaf_race)(OaArgs const& a, uint32_t b, void const* pairs, void* found, uint8_t* inserted, uint32_t n,

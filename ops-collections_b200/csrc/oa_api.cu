@@ -226,6 +226,29 @@ int b2co_oa_insert_counted(b2co_oa_table* t, void const* pairs, uint8_t const* s
     return st;
 }
 
+// Clears absent[i] of every pair whose key the table holds, and with `assign`
+// overwrites its payload (DynamicMap's older submaps).
+int b2co_oa_mark(b2co_oa_table* t, void const* pairs, uint64_t n, bool assign, uint8_t* absent, cudaStream_t s)
+{
+    if (int st = check_table(t)) return st;
+    if (int st = check_batch(n)) return st;
+    return t->ops->mark(t->args, t->desc.bucket_size, pairs, uint32_t(n), assign, absent, s);
+}
+
+// A lookup that leaves the outputs of keys it does not find (or finds with the
+// empty payload) as they are, and with `skip` need not ask for keys whose output
+// says they were found (DynamicMap's older submaps).
+int b2co_oa_lookup_over(b2co_oa_table* t, bool contains, void const* keys, void* out, uint64_t n, bool skip,
+                        cudaStream_t s)
+{
+    if (int st = check_table(t)) return st;
+    if (int st = check_batch(n)) return st;
+    OaArgs a = t->args;
+    a.keep_misses = skip ? 2 : 1;
+    return t->ops->find(a, t->desc.bucket_size, 0, 0, contains, keys, nullptr, out, uint32_t(n),
+                        wait_ctl(status_word(t)), s);
+}
+
 // Device bytes a table holds (slots and counters).
 uint64_t b2co_oa_table_bytes(b2co_oa_table const* t)
 {

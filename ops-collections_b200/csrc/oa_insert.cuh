@@ -1,6 +1,6 @@
 // oa_insert.cuh -- the write kernel of large tables: Insert / InsertIf,
-// InsertOrAssign, InsertAndFind (race) and the placement pass of first-wins
-// InsertAndFind.
+// InsertOrAssign, InsertAndFind (race), the placement pass of first-wins
+// InsertAndFind, and the marking passes of DynamicMap.
 //
 // Per-key algorithm (InsertVerdict, open_addressing_ref_impl.h:489-532): walk
 // the key's probe sequence bucket window by bucket window; in a window the

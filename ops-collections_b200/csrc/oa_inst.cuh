@@ -83,7 +83,9 @@ struct OaImpl {
     {
         uint32_t const lanes = a.write_shape >> 8;
         return B == 1 || lanes == 1 ||
-               (lanes == 0 && table_bytes(a) <= (mode == kInsAssign ? kSectorAssignBytes : kSectorInsertBytes));
+               (lanes == 0 && table_bytes(a) <= (mode == kInsAssign ? kSectorAssignBytes
+                                              : mode >= kInsMark  ? kSectorFindBytes
+                                                                  : kSectorInsertBytes));
     }
 
     // A write of one mode.
@@ -113,6 +115,18 @@ struct OaImpl {
             o.counters = counters;
             return assign ? write<B, kInsAssign>(a, pairs, stencil, n, o, s)
                           : write<B, kInsPlain>(a, pairs, stencil, n, o, s);
+        });
+    }
+
+    static int mark(OaArgs const& a, uint32_t b, void const* pairs, uint32_t n, bool assign, uint8_t* absent,
+                    cudaStream_t s)
+    {
+        return with_b(b, [&](auto bc) {
+            constexpr int B = decltype(bc)::value;
+            InsOut o{};
+            o.inserted = absent;
+            return assign ? write<B, kInsMarkAssign>(a, pairs, nullptr, n, o, s)
+                          : write<B, kInsMark>(a, pairs, nullptr, n, o, s);
         });
     }
 
@@ -225,9 +239,9 @@ struct OaImpl {
     template <int B, int G, int Q, bool C>
     static int find_defer_auto(OaArgs const& a, void const* keys, void* out, uint32_t n, WaitCtl wc, cudaStream_t s)
     {
-        DeferFn const even = k_find_wdefer<S, B, G, Q, C, true>;
+        DeferFn const even = a.keep_misses ? k_find_wdefer<S, B, G, Q, C, true, true> : k_find_wdefer<S, B, G, Q, C, true>;
         uint64_t const share = (n + defer_warps(even) - 1) / defer_warps(even);
-        if (share >= kWarpStageKeys)
+        if (share >= kWarpStageKeys && !a.keep_misses)
             return launch_wdefer(k_find_wdefer<S, B, G, Q, C>, C, a, keys, out, n, kWarpStageKeys, wc, s);
         uint64_t const rounds = (share + kWarpStageKeys - 1) / kWarpStageKeys;
         return launch_wdefer(even, C, a, keys, out, n, ((share + rounds - 1) / rounds + 31) / 32 * 32, wc, s);
@@ -248,7 +262,7 @@ struct OaImpl {
     static int find_sector(OaArgs const& a, void const* keys, uint8_t const* stencil, void* out, uint32_t n,
                            cudaStream_t s)
     {
-        auto k = k_find_sector<S, B, C>;
+        auto k = a.keep_misses ? k_find_sector<S, B, C, true> : k_find_sector<S, B, C, false>;
         uint32_t const block = sector_block(n);
         k<<<grid_for((void const*)k, block, n, block), block, 0, s>>>(a, keys, stencil, out, n);
         return check_launch(C ? "contains kernel" : "find kernel");
@@ -415,7 +429,7 @@ struct OaImpl {
         });
     }
 
-    static constexpr OaOps ops{&clear, &insert, &assign_if, &iaf_race, &iaf_first, &find, &erase, &count};
+    static constexpr OaOps ops{&clear, &insert, &mark, &assign_if, &iaf_race, &iaf_first, &find, &erase, &count};
 };
 
 template <class S>

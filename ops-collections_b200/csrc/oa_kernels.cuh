@@ -36,6 +36,8 @@ struct OaArgs {
     uint64_t empty_value;
     uint64_t erased_key;
     uint32_t write_shape;  // insert-family kernel shape: 0 = default, else (lanes << 8) | keys per tile
+    uint32_t keep_misses;  // default lookups: 1: outputs of keys that are not found stay as they are;
+                           // 2: and a key whose output says it was found already may be left out
 };
 
 template <int N>
@@ -399,12 +401,17 @@ __global__ void __launch_bounds__(256) k_iaf_final(__grid_constant__ const OaArg
 // Find / Contains (FindAndContains, open_addressing_ref_impl.h:567-605)
 // ----------------------------------------------------------------------------
 
-// One lookup's result: the payload found or the empty payload, or the flag.
+// One lookup's result: the payload found or the empty payload, or the flag.  With
+// `keep` (OaArgs::keep_misses) a key that is not found, or is found with the
+// empty payload, leaves its output as it is.
 template <class S, bool CONTAINS>
-__device__ __forceinline__ void store_result(OaArgs const& a, void* out, uint32_t i, bool hit, uint64_t payload)
+__device__ __forceinline__ void store_result(OaArgs const& a, bool keep, void* out, uint32_t i, bool hit,
+                                             uint64_t payload)
 {
+    uint64_t const v = hit ? payload : empty_payload<S>(a);
+    if (keep && !(hit && (CONTAINS || v != empty_payload<S>(a)))) return;
     if constexpr (CONTAINS) reinterpret_cast<uint8_t*>(out)[i] = hit;
-    else Io<S>::store_payload(out, i, hit ? payload : empty_payload<S>(a));
+    else Io<S>::store_payload(out, i, v);
 }
 
 // Whether a loaded window holds a slot that ends the scan (empty or equal); the
@@ -516,7 +523,7 @@ __global__ void __launch_bounds__(256) k_find_tile(__grid_constant__ const OaArg
         }
         uint32_t const src = tile_shift + (stop_j >= 0 ? uint32_t(stop_j % G) : 0u);
         uint64_t const pv = __shfl_sync(0xffffffffu, (unsigned long long)payload, src);
-        if (r == 0 && i < n) store_result<S, CONTAINS>(a, out, i, hit, pv);
+        if (r == 0 && i < n) store_result<S, CONTAINS>(a, a.keep_misses != 0, out, i, hit, pv);
     }
 }
 
@@ -979,7 +986,7 @@ __device__ __forceinline__ int tile_first_stop(typename S::Raw const (&w)[ROUNDS
 // Keys per warp and stage: kWarpStageKeys, or `even_chunk` (a multiple of 32, at
 // most kWarpStageKeys) when EVEN, for batches that do not fill every warp's
 // stage.  (A stage length known at compile time is worth 0.4% on large batches.)
-template <class S, int B, int G, int Q, bool CONTAINS, bool EVEN = false>
+template <class S, int B, int G, int Q, bool CONTAINS, bool EVEN = false, bool KEEP = false>
 __global__ void __launch_bounds__(256, B2CO_WDEFER_MINB(Q)) k_find_wdefer(__grid_constant__ const OaArgs a, void const* keys, void* out,
                                                         uint32_t n, uint32_t even_chunk, WaitCtl wc)
 {
@@ -1011,10 +1018,10 @@ __global__ void __launch_bounds__(256, B2CO_WDEFER_MINB(Q)) k_find_wdefer(__grid
     uint32_t head = 0, count = 0;  // queue state, the same on every lane
 
     auto settle = [&](uint32_t pos, Raw const& slot) {  // result from the slot that ended the scan
-        store_result<S, CONTAINS>(a, out, pos, S::key(slot) != a.empty_key, S::value(slot));
+        store_result<S, CONTAINS>(a, KEEP, out, pos, S::key(slot) != a.empty_key, S::value(slot));
     };
     auto settle_miss = [&](uint32_t pos) {
-        store_result<S, CONTAINS>(a, out, pos, false, 0);
+        store_result<S, CONTAINS>(a, KEEP, out, pos, false, 0);
     };
     // Lane 0 of each tile whose window ended no scan queues its key.
     auto enqueue = [&](bool unsettled, uint64_t key, uint32_t init, uint32_t idx, uint32_t pos) {
@@ -1156,7 +1163,7 @@ __global__ void __launch_bounds__(256, B2CO_WDEFER_MINB(Q)) k_find_wdefer(__grid
         resolve_range<S, B, G, ROUNDS>(a, w, 0, B, key, r, tile_lane0, !live, res);
         if (__any_sync(0xffffffffu, !res.done))
             res = tile_continue<S, B, G, ROUNDS>(a, slots, key, init0, r, tile_lane0, res);
-        if (r == 0 && live) store_result<S, CONTAINS>(a, out, i, res.hit, res.payload);
+        if (r == 0 && live) store_result<S, CONTAINS>(a, KEEP, out, i, res.hit, res.payload);
     }
 }
 

@@ -123,7 +123,7 @@ constexpr uint32_t kSectorRing = 64;  // queued keys per warp: a pass may add 31
 #define B2CO_SECTOR_FIND_MINB(NS) ((NS) >= 3 ? 4 : 5)
 #endif
 
-template <class S, int B, bool CONTAINS>
+template <class S, int B, bool CONTAINS, bool KEEP>
 __global__ void __launch_bounds__(256, B2CO_SECTOR_FIND_MINB((SectorWindow<S, B>::NS)))
     k_find_sector(__grid_constant__ const OaArgs a, void const* keys, uint8_t const* stencil, void* out, uint32_t n)
 {
@@ -138,7 +138,14 @@ __global__ void __launch_bounds__(256, B2CO_SECTOR_FIND_MINB((SectorWindow<S, B>
     uint32_t head = 0, count = 0;  // queue state, the same on every lane
     Raw const* const slots = reinterpret_cast<Raw const*>(a.slots);
 
+    // whether an earlier lookup has answered key i already (OaArgs::keep_misses 2)
+    auto answered = [&](uint32_t i) {
+        if (!KEEP || a.keep_misses < 2) return false;
+        if constexpr (CONTAINS) return reinterpret_cast<uint8_t const*>(out)[i] != 0;
+        else return uint64_t(reinterpret_cast<typename Io<S>::Payload const*>(out)[i]) != empty_payload<S>(a);
+    };
     // the next pass's key is loaded one pass ahead
+    bool next_done = base + lane < n && answered(base + lane);
     uint64_t next_key = base + lane < n ? Io<S>::load_key(keys, base + lane) : 0;
     for (;;) {
         uint64_t key;
@@ -159,19 +166,20 @@ __global__ void __launch_bounds__(256, B2CO_SECTOR_FIND_MINB((SectorWindow<S, B>
             count -= take;
             idx = probe_next(idx, probe_step<S::key_bytes, B>(a.probe, key), a.probe.capacity);
             if (live && idx == init) {  // full cycle: not present
-                store_result<S, CONTAINS>(a, out, pos, false, 0);
+                store_result<S, CONTAINS>(a, KEEP, out, pos, false, 0);
                 live = false;
             }
         } else {
             pos = base + lane;
             key = next_key;
-            live = pos < n;
+            live = pos < n && !next_done;
             if (stencil && live && !stencil[pos]) {
-                store_result<S, CONTAINS>(a, out, pos, false, 0);
+                store_result<S, CONTAINS>(a, KEEP, out, pos, false, 0);
                 live = false;
             }
             init = idx = probe_init<S::key_bytes, B>(a.probe, key);
             base += stride;
+            next_done = base < n && base + lane < n && answered(base + lane);
             next_key = base < n && base + lane < n ? Io<S>::load_key(keys, base + lane) : 0;
         }
         bool open = false;
@@ -181,7 +189,7 @@ __global__ void __launch_bounds__(256, B2CO_SECTOR_FIND_MINB((SectorWindow<S, B>
             int const j = w.first_stop(key, a.empty_key);
             if (j >= 0) {
                 Raw const slot = w.pick(j);
-                store_result<S, CONTAINS>(a, out, pos, S::key(slot) != a.empty_key, S::value(slot));
+                store_result<S, CONTAINS>(a, KEEP, out, pos, S::key(slot) != a.empty_key, S::value(slot));
             } else {
                 open = true;
             }
@@ -202,13 +210,13 @@ __global__ void __launch_bounds__(256, B2CO_SECTOR_FIND_MINB((SectorWindow<S, B>
 // Insert / InsertIf / InsertOrAssign, InsertAndFind (race), first-wins placement
 // ----------------------------------------------------------------------------
 
-enum { kInsPlain = 0, kInsAssign = 1, kInsIafRace = 2, kInsIafPlace = 3 };
+enum { kInsPlain = 0, kInsAssign = 1, kInsIafRace = 2, kInsIafPlace = 3, kInsMark = 4, kInsMarkAssign = 5 };
 
 // Outputs of one insert-family launch (only the mode's fields are used).
 struct InsOut {
     Counters counters;   // plain/assign
     void* found;         // race: payload found or inserted
-    uint8_t* inserted;   // race: 1 = this input inserted the key
+    uint8_t* inserted;   // race: 1 = this input inserted the key; mark: cleared where the key is present
     uint32_t* pos;       // place: slot of every input (kNoSlot = failed)
     uint32_t* newbits;   // place: slots claimed by this batch
     uint32_t* owner;     // place: claiming input of each claimed slot (claim_bit 0 only)
@@ -231,13 +239,15 @@ struct InsRecord {
         } else if constexpr (MODE == kInsIafRace) {
             Io<S>::store_payload(o.found, i, verdict == kFailed ? empty_payload<S>(a) : found);
             o.inserted[i] = verdict == kSuccess;
-        } else {
+        } else if constexpr (MODE == kInsIafPlace) {
             uint32_t const p = verdict == kFailed ? kNoSlot : where;
             if (verdict == kSuccess) {
                 atomicOr(o.newbits + (p >> 5), 1u << (p & 31));
                 if (!o.claim_bit) o.owner[p] = i;  // tables without room for the claim bit
             }
             o.pos[i] = verdict == kSuccess ? (p | o.claim_bit) : p;
+        } else {
+            if (verdict == kDuplicate) o.inserted[i] = 0;
         }
     }
     __device__ __forceinline__ void finish(InsOut const& o) const  // every thread of the block
@@ -296,14 +306,20 @@ __device__ __forceinline__ int sector_decide(OaArgs const& a, typename S::Raw* w
                                              uint64_t key, uint64_t val, uint64_t& found)
 {
     bool const empty = S::key(cur) == a.empty_key;
-    int const verdict = empty ? sector_claim<S, B>(a, win, key, val, j, cur) : int(kDuplicate);
-    if (verdict == kDuplicate) {
-        if constexpr (MODE == kInsAssign) assign_payload<S>(win + j, key, val);
-        if constexpr (MODE == kInsIafRace) found = S::value(settle<S>(a, win + j, cur));
-    } else if (verdict == kSuccess) {
-        found = S::is_set ? key : val;
+    if constexpr (MODE == kInsMark || MODE == kInsMarkAssign) {
+        if (empty) return kFailed;  // absent: nothing is written
+        if constexpr (MODE == kInsMarkAssign) assign_payload<S>(win + j, key, val);
+        return kDuplicate;
+    } else {
+        int const verdict = empty ? sector_claim<S, B>(a, win, key, val, j, cur) : int(kDuplicate);
+        if (verdict == kDuplicate) {
+            if constexpr (MODE == kInsAssign) assign_payload<S>(win + j, key, val);
+            if constexpr (MODE == kInsIafRace) found = S::value(settle<S>(a, win + j, cur));
+        } else if (verdict == kSuccess) {
+            found = S::is_set ? key : val;
+        }
+        return verdict;
     }
-    return verdict;
 }
 
 #ifndef B2CO_SECTOR_WRITE_MINB
