@@ -4,6 +4,7 @@
 // items is a no-op, a NULL input makes a sync insert report every item failed
 // and an async call return, batches beyond the kernel index range are a
 // length error, sync calls synchronize the stream and read the counters back.
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -729,14 +730,23 @@ int b2co_oa_set_write_shape(b2co_oa_table* t, uint32_t lanes, uint32_t keys_per_
 // Only the first copy-in and the last copy-out run with the other direction
 // idle, so a batch of 16 Mi keys or more starts with chunks of 1 and 2 Mi keys
 // and ends with 2 and 1 Mi (uniform 1 or 2 Mi chunks measured slower: each
-// chunk costs about 40 us of pipeline overhead).  Pinned host buffers give full
-// overlap.
-constexpr uint64_t kHostChunk = 1ull << 22;  // keys per full chunk
+// chunk costs about 40 us of pipeline overhead), and a smaller one is dealt
+// evenly over kHostChunks chunks, down to kHostChunkMin keys each (int64 pairs,
+// 1 / 2 / 4 / 8 chunks: 4.2 Mi keys 1,379 / 1,085 / 1,025 / 1,100 us, 10 M keys
+// 2,450 / 2,377 / 2,240 / 2,225, 1 Mi keys 365 / 320 / 312 / 320).
+// Pinned host buffers give full overlap.
+constexpr uint64_t kHostChunk = 1ull << 22;     // keys per full chunk
+constexpr uint64_t kHostChunks = 4;             // chunks of a batch below 4 full ones
+constexpr uint64_t kHostChunkMin = 1ull << 17;  // a batch of one chunk needs no pipeline
 
 static uint64_t host_chunk_at(uint64_t off, uint64_t n)
 {
     uint64_t const q = kHostChunk / 4, h = kHostChunk / 2, left = n - off;
-    if (n < 4 * kHostChunk) return left < kHostChunk ? left : kHostChunk;
+    if (n < 4 * kHostChunk) {
+        uint64_t const even = (n + kHostChunks - 1) / kHostChunks;
+        uint64_t const chunk = std::min(std::max((even + 63) / 64 * 64, kHostChunkMin), kHostChunk);
+        return left < chunk ? left : chunk;
+    }
     if (off == 0) return q;
     if (off == q) return h;
     if (left <= q) return left;
@@ -758,13 +768,16 @@ int b2co_oa_find_host(b2co_oa_table* t, void const* host_keys, void* host_out, u
         for (auto& e : t->ev) B2CO_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     cudaStream_t c = cs(s);
-    B2CO_CUDA(cudaEventRecord(t->ev[kHostSlots], c));
-    for (auto& p : t->pipe) B2CO_CUDA(cudaStreamWaitEvent(p, t->ev[kHostSlots], 0));
     char* base = static_cast<char*>(t->stage);
+    bool const piped = host_chunk_at(0, n) < n;  // one chunk stays on the caller's stream
+    if (piped) {
+        B2CO_CUDA(cudaEventRecord(t->ev[kHostSlots], c));
+        for (auto& p : t->pipe) B2CO_CUDA(cudaStreamWaitEvent(p, t->ev[kHostSlots], 0));
+    }
     for (uint64_t off = 0, c_i = 0, m = 0; off < n; off += m, ++c_i) {
         m = host_chunk_at(off, n);
         int slot = int(c_i % kHostSlots);
-        cudaStream_t p = t->pipe[slot];
+        cudaStream_t p = piped ? t->pipe[slot] : c;
         char* dk = base + uint64_t(slot) * chunk * (kb + ob);
         char* dout = dk + chunk * kb;
         B2CO_CUDA(cudaMemcpyAsync(dk, static_cast<char const*>(host_keys) + off * kb, m * kb,
@@ -772,7 +785,7 @@ int b2co_oa_find_host(b2co_oa_table* t, void const* host_keys, void* host_out, u
         if (int st = launch_find(t, false, dk, nullptr, dout, m, p)) return st;
         B2CO_CUDA(cudaMemcpyAsync(static_cast<char*>(host_out) + off * ob, dout, m * ob, cudaMemcpyDeviceToHost, p));
     }
-    for (int i = 0; i < kHostSlots; ++i) {
+    for (int i = 0; piped && i < kHostSlots; ++i) {
         B2CO_CUDA(cudaEventRecord(t->ev[i], t->pipe[i]));
         B2CO_CUDA(cudaStreamWaitEvent(c, t->ev[i], 0));
     }
