@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256, 4) k_group_find_lane(__grid_constant__ co
         bool open = false;
         if (live) {
             SectorWindow<S, B> w;
-            w.template load<false>(slots + idx);
+            w.template load<false, true>(slots + idx);
             int const j = w.first_stop(key, g.empty_key);
             if (j >= 0) {
                 Raw const slot = w.pick(j);
@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(256, 4) k_group_insert(__grid_constant__ const
         if (live) {
             uint64_t const key = S::key(pr);
             SectorWindow<S, B> w;
-            w.template load<true>(slots + idx);
+            w.template load<true, true>(slots + idx);
             int j = w.first_stop(key, g.empty_key);
             if (j >= 0) {
                 Raw old = w.pick(j);
