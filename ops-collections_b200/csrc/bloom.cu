@@ -17,6 +17,7 @@
 // Other policies run one key per thread: W/2 64-bit REDs (one 32-bit RED for
 // W = 1) and vector loads of the block.  Merge/Intersect stream 16 bytes per
 // lane (4 when the word count is not a multiple of 4).
+#include <cmath>
 #include <new>
 
 #include "b2co_host.h"
@@ -135,22 +136,23 @@ __global__ void __launch_bounds__(256) k_bloom_add_bulk(uint32_t* words, uint32_
 // shapes.  The filter is cut into slices of kSliceBlocks blocks (128 KiB); a
 // key's record is its block within the slice (high 32 bits) and the lower
 // hash half (low 32 bits).  Each of R route CTAs owns one contiguous chunk of
-// the batch.
-//   count   : CTA c counts its chunk's records per slice -> counts[c][s];
-//   colscan : per slice, the exclusive prefix over the CTAs (in place) and the
-//             slice's total;
-//   scan    : slice offsets into the record workspace (records of a slice are
-//             contiguous, CTA by CTA);
+// the batch, and of every slice a segment of the record workspace, sized for
+// the chunk's even share of the slice and six standard deviations of it.
 //   route   : CTA c hashes its chunk a tile at a time, sorts the tile's
-//             records by slice in shared memory and writes each slice's run at
-//             its own running cursor -- no global atomics, and writes leave in
-//             runs rather than one record at a time;
+//             records by slice in shared memory and appends each slice's run to
+//             its own segment -- no global atomics, and writes leave in runs
+//             rather than one record at a time.  A record that its segment has
+//             no room for (skewed keys) is ORed into the filter at once; its
+//             block is read first, so a key that comes again and again costs a
+//             read, not an atomic on one address;
 //   apply   : one CTA per slice ORs the slice's records into a shared-memory
 //             copy of the slice and reduces the whole copy into the filter with
 //             TMA bulk ORs (element-wise atomic in L2, so concurrent Adds on
 //             other streams stay correct).
-// DRAM traffic per key is the key twice and a record written and read back
-// (8 + 8 + 8 + 8 bytes), against two scattered 32-byte block transfers per key
+// Fixed segments take a fifth more workspace than exact ones, and save the pass
+// that counts (and hashes) every key to size them: 0.46 of 2.2 ms for 2^27 keys.
+// DRAM traffic per key is the key once and a record written and read back
+// (8 + 8 + 8 bytes), against two scattered 32-byte block transfers per key
 // otherwise.
 constexpr uint32_t kSliceBlocks = 4096;
 constexpr uint32_t kMaxSlices = 2048;  // filters up to 256 MiB take this path
@@ -160,114 +162,47 @@ constexpr int kRouteTile = kRouteThreads * kRouteKeys;
 constexpr int kApplyThreads = 1024;
 
 // Chunk of route CTA c: whole tiles, the last chunk possibly short.
-__device__ __forceinline__ void route_chunk(uint64_t n, uint32_t c, uint32_t nctas, uint64_t& begin, uint64_t& end)
+__host__ __device__ __forceinline__ uint64_t route_chunk_keys(uint64_t n, uint32_t nctas)
 {
     uint64_t const tiles = (n + kRouteTile - 1) / kRouteTile;
-    uint64_t const per = (tiles + nctas - 1) / nctas;
-    begin = uint64_t(c) * per * kRouteTile;
-    end = begin + per * kRouteTile;
+    return (tiles + nctas - 1) / nctas * kRouteTile;
+}
+__device__ __forceinline__ void route_chunk(uint64_t n, uint32_t c, uint32_t nctas, uint64_t& begin, uint64_t& end)
+{
+    uint64_t const per = route_chunk_keys(n, nctas);
+    begin = uint64_t(c) * per;
+    end = begin + per;
     if (begin > n) begin = n;
     if (end > n) end = n;
 }
 
-template <int KB>
-__global__ void __launch_bounds__(1024, 2) k_bloom_count(uint32_t nblocks, uint64_t seed, void const* keys,
-                                                     uint8_t const* stencil, uint64_t n, uint32_t nslices,
-                                                     uint32_t nctas, uint32_t* counts)
+// Records of one segment: a CTA's even share of a slice, and what chance adds.
+uint32_t route_segment(uint64_t n, uint32_t nctas, uint32_t nslices)
 {
-    __shared__ uint32_t hist[kMaxSlices];
-    for (uint32_t i = threadIdx.x; i < nslices; i += blockDim.x) hist[i] = 0;
-    __syncthreads();
-    uint64_t begin, end;
-    route_chunk(n, blockIdx.x, nctas, begin, end);
-    constexpr int kKeys = 8;  // keys loaded before any is hashed
-    for (uint64_t i0 = begin + threadIdx.x; i0 < end; i0 += uint64_t(kKeys) * blockDim.x) {
-        uint64_t key[kKeys];
-        bool live[kKeys];
-#pragma unroll
-        for (int j = 0; j < kKeys; ++j) {
-            uint64_t const i = i0 + uint64_t(j) * blockDim.x;
-            live[j] = i < end && (!stencil || stencil[i]);
-            key[j] = live[j] ? load_key<KB>(keys, i) : 0;
-        }
-#pragma unroll
-        for (int j = 0; j < kKeys; ++j) {
-            uint32_t block, lower;
-            locate<KB>(key[j], seed, nblocks, block, lower);
-            if (live[j]) atomicAdd(&hist[block / kSliceBlocks], 1u);
-        }
-    }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < nslices; i += blockDim.x) counts[uint64_t(blockIdx.x) * nslices + i] = hist[i];
+    double const mean = double(route_chunk_keys(n, nctas)) / nslices;
+    return uint32_t(mean + 6.0 * std::sqrt(mean) + 16.0);
 }
 
-// Per slice (one thread each): exclusive prefix of its counts over the route
-// CTAs, in place, and the slice's total.
-__global__ void __launch_bounds__(256) k_bloom_colscan(uint32_t* counts, uint32_t nslices, uint32_t nctas,
-                                                       uint32_t* totals)
+// ORs one key's pattern into its block unless every bit is set already.
+__device__ __forceinline__ void or_block(uint32_t* words, uint32_t block, uint32_t lower)
 {
-    uint32_t const sl = blockIdx.x * blockDim.x + threadIdx.x;
-    if (sl >= nslices) return;
-    uint32_t run = 0;
-    for (uint32_t c = 0; c < nctas; ++c) {
-        uint32_t* p = counts + uint64_t(c) * nslices + sl;
-        uint32_t const v = *p;
-        *p = run;
-        run += v;
-    }
-    totals[sl] = run;
-}
-
-// Exclusive scan of the slice totals (one CTA): offsets[0..nslices].
-__global__ void __launch_bounds__(1024) k_bloom_scan(uint32_t const* totals, uint32_t nslices, uint32_t* offsets)
-{
-    __shared__ uint32_t warp_tot[32];
-    constexpr int kPer = kMaxSlices / 1024;
-    uint32_t const t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    uint32_t v[kPer], sum = 0;
+    auto* p = reinterpret_cast<unsigned long long*>(words + uint64_t(block) * 8);
 #pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-        uint32_t const i = t * kPer + j;
-        v[j] = i < nslices ? totals[i] : 0u;
-        sum += v[j];
+    for (int q = 0; q < 4; ++q) {
+        unsigned long long const bits =
+            (unsigned long long)word_bit(2 * q, lower) | ((unsigned long long)word_bit(2 * q + 1, lower) << 32);
+        if ((ld_rw(p + q) & bits) != bits) atomicOr(p + q, bits);
     }
-    uint32_t incl = sum;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        uint32_t const o = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= uint32_t(d)) incl += o;
-    }
-    if (lane == 31) warp_tot[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t const w = warp_tot[lane];
-        uint32_t wi = w;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            uint32_t const o = __shfl_up_sync(0xffffffffu, wi, d);
-            if (lane >= uint32_t(d)) wi += o;
-        }
-        warp_tot[lane] = wi - w;  // exclusive prefix of the warp totals
-    }
-    __syncthreads();
-    uint32_t run = warp_tot[warp] + incl - sum;
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-        uint32_t const i = t * kPer + j;
-        if (i <= nslices) offsets[i] = run;
-        run += v[j];
-    }
-    if (t == 1023 && nslices == kMaxSlices) offsets[nslices] = run;
 }
 
 // Shared memory of one route CTA: the next tile's keys (8 bytes a key), the
 // tile's records and their destinations, then per slice the tile's count, its
-// offset in the tile, its run's global start, the CTA's running cursor and the
-// slice's end in the workspace.
+// offset in the tile, where its run starts in the segment and the segment's
+// fill.
 __host__ __device__ constexpr uint32_t route_bins(uint32_t nslices) { return (nslices + 31) & ~31u; }
 __host__ __device__ constexpr size_t route_smem(uint32_t nslices)
 {
-    return size_t(kRouteTile) * (8 + 8 + 4) + size_t(route_bins(nslices)) * 4 * 5 + (kRouteThreads / 32 + 1) * 4;
+    return size_t(kRouteTile) * (8 + 8 + 4) + size_t(route_bins(nslices)) * 4 * 4 + (kRouteThreads / 32 + 1) * 4;
 }
 
 template <int KB>
@@ -277,10 +212,10 @@ __device__ __forceinline__ void cp_async_key(void* dst, void const* src)
 }
 
 template <int KB>
-__global__ void __launch_bounds__(kRouteThreads) k_bloom_route(uint32_t nblocks, uint64_t seed, void const* keys,
-                                                               uint8_t const* stencil, uint64_t n, uint32_t nslices,
-                                                               uint32_t nctas, uint32_t const* prefix,
-                                                               uint32_t const* offsets, unsigned long long* recs)
+__global__ void __launch_bounds__(kRouteThreads) k_bloom_route(uint32_t* words, uint32_t nblocks, uint64_t seed,
+                                                               void const* keys, uint8_t const* stencil, uint64_t n,
+                                                               uint32_t nslices, uint32_t nctas, uint32_t segment,
+                                                               uint32_t* counts, unsigned long long* recs)
 {
     extern __shared__ __align__(16) unsigned char route_smem_[];
     auto* kbuf = reinterpret_cast<unsigned long long*>(route_smem_);  // one 8-byte cell a key
@@ -291,16 +226,12 @@ __global__ void __launch_bounds__(kRouteThreads) k_bloom_route(uint32_t nblocks,
     uint32_t* loff = hist + nbins;
     uint32_t* gbase = loff + nbins;
     uint32_t* gcur = gbase + nbins;
-    uint32_t* gend = gcur + nbins;
-    uint32_t* warp_tot = gend + nbins;  // kRouteThreads / 32 warp sums, then the tile's total
+    uint32_t* warp_tot = gcur + nbins;  // kRouteThreads / 32 warp sums, then the tile's total
     uint32_t const t = threadIdx.x, lane = t & 31, warp = t >> 5;
     constexpr uint32_t kNone = 0xffffffffu;
     constexpr int kWarps = kRouteThreads / 32;
     constexpr int kPer = kMaxSlices / kRouteThreads;
-    for (uint32_t i = t; i < nslices; i += kRouteThreads) {
-        gcur[i] = offsets[i] + prefix[uint64_t(blockIdx.x) * nslices + i];
-        gend[i] = offsets[i + 1];
-    }
+    for (uint32_t i = t; i < nslices; i += kRouteThreads) gcur[i] = 0;
     uint64_t begin, end;
     route_chunk(n, blockIdx.x, nctas, begin, end);
     // a thread copies its own keys of the next tile into its own cells while the
@@ -343,7 +274,7 @@ __global__ void __launch_bounds__(kRouteThreads) k_bloom_route(uint32_t nblocks,
             where[j] = live[j] ? (where[j] << 16) | atomicAdd(&hist[where[j]], 1u) : kNone;
         __syncthreads();
         // the tile's offsets per slice (exclusive scan, kPer slices per thread);
-        // each slice's run starts at the CTA's cursor for it
+        // each slice's run starts at the fill of its segment
         uint32_t v[kPer], sum = 0;
 #pragma unroll
         for (int q = 0; q < kPer; ++q) {
@@ -377,21 +308,21 @@ __global__ void __launch_bounds__(kRouteThreads) k_bloom_route(uint32_t nblocks,
             uint32_t const i = t * kPer + q;
             if (i < nslices) {
                 loff[i] = run;
-                gbase[i] = gcur[i];
-                gcur[i] += v[q];
+                uint32_t const at = gcur[i];
+                gbase[i] = at;
+                gcur[i] = at + v[q] < segment ? at + v[q] : segment;
             }
             run += v[q];
         }
         __syncthreads();
-        // records sorted by slice in shared memory, each with its destination; a
-        // record never passes its slice's end (only keys changed between the
-        // count and this pass could ask it to)
+        // records sorted by slice in shared memory, each with its destination
 #pragma unroll
         for (int j = 0; j < kRouteKeys; ++j) {
             if (where[j] == kNone) continue;
             uint32_t const sl = where[j] >> 16, r = where[j] & 0xffffu, g = gbase[sl] + r;
             stage[loff[sl] + r] = rec[j];
-            stage_at[loff[sl] + r] = g < gend[sl] ? g : kNone;
+            stage_at[loff[sl] + r] = g < segment ? (sl * nctas + blockIdx.x) * segment + g : kNone;
+            if (g >= segment) or_block(words, sl * kSliceBlocks + uint32_t(rec[j] >> 32), uint32_t(rec[j]));
         }
         __syncthreads();
         // each slice's records leave as one run
@@ -402,34 +333,50 @@ __global__ void __launch_bounds__(kRouteThreads) k_bloom_route(uint32_t nblocks,
         }
         // the next tile rewrites the shared arrays only after its first barrier
     }
+    __syncthreads();
+    for (uint32_t i = t; i < nslices; i += kRouteThreads) counts[uint64_t(i) * nctas + blockIdx.x] = gcur[i];
 }
 
-// One CTA per slice: OR the slice's records into a shared copy of its words,
-// then bulk-OR the copy into the filter in 16 KiB pieces.
+// One CTA per slice: OR the slice's records into a shared copy of its words (a
+// warp takes a segment), then bulk-OR the copy into the filter in 16 KiB pieces.
+// The shared-memory atomics bound it.
 constexpr uint32_t kApplyChunk = 16384;
 
 __global__ void __launch_bounds__(kApplyThreads) k_bloom_apply(uint32_t* words, uint32_t nblocks,
-                                                               unsigned long long const* recs,
-                                                               uint32_t const* offsets)
+                                                               unsigned long long const* recs, uint32_t const* counts,
+                                                               uint32_t nctas, uint32_t segment)
 {
     extern __shared__ __align__(128) uint32_t slice[];  // kSliceBlocks * 8 words
     uint32_t const sl = blockIdx.x, first = sl * kSliceBlocks;
     uint32_t const nb = nblocks - first < kSliceBlocks ? nblocks - first : kSliceBlocks;
     uint32_t const nwords = nb * 8;
+    uint32_t const lane = threadIdx.x & 31;
     for (uint32_t i = threadIdx.x * 4; i < nwords; i += kApplyThreads * 4)
         *reinterpret_cast<uint4*>(slice + i) = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
-    uint32_t const beg = offsets[sl], end = offsets[sl + 1];
-    for (uint32_t r = beg + threadIdx.x; r < end; r += kApplyThreads) {
-        unsigned long long const rec = __ldcs(recs + r);
+    // word w of block b sits at b * 8 + (w ^ swz(b)): the words that a warp writes
+    // in one step spread over all banks instead of four of them.  (Lanes that start
+    // with different words of unswizzled blocks spread as well, but ran 1.11 ms
+    // against 0.49 for 2^27 records.)
+    auto apply = [&](unsigned long long rec) {
         uint32_t const b = uint32_t(rec >> 32), lower = uint32_t(rec);
-        if (b >= nb) continue;
-        // word w of block b sits at b * 8 + (w ^ swz(b)): the words that a warp
-        // writes in one step spread over the banks instead of four of them
-        uint32_t* blk = slice + b * 8;
+        if (b >= nb) return;
+        uint32_t* const blk = slice + b * 8;
         uint32_t const swz = (b >> 2) & 7u;
 #pragma unroll
         for (int w = 0; w < 8; ++w) atomicOr(blk + (uint32_t(w) ^ swz), word_bit(w, lower));
+    };
+    for (uint32_t c = threadIdx.x >> 5; c < nctas; c += kApplyThreads / 32) {
+        uint32_t const count = counts[uint64_t(sl) * nctas + c];
+        unsigned long long const* const seg = recs + uint64_t(sl * nctas + c) * segment;
+                constexpr int kAhead = 4;  // records loaded before any is applied
+        for (uint32_t r = lane; r < count; r += 32 * kAhead) {
+            unsigned long long rec[kAhead];
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) rec[j] = r + 32 * j < count ? __ldcs(seg + r + 32 * j) : ~0ull;
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) apply(rec[j]);  // the filler's block is out of range
+        }
     }
     __syncthreads();
     // back to the filter's word order, a block per thread
@@ -607,7 +554,7 @@ struct b2co_bloom {
     int add_mode = B2CO_BLOOM_ADD_AUTO;  // default-policy Add: see b2co_bloom_add_mode
     unsigned long long* recs = nullptr;  // partitioned Add: record workspace
     uint64_t recs_cap = 0;
-    uint32_t* part = nullptr;  // partitioned Add: per-CTA slice counts, slice totals and offsets
+    uint32_t* part = nullptr;  // partitioned Add: records of every segment
     size_t part_words = 0;
     ScratchOrder part_order;  // the workspace serves one partitioned Add at a time
     uint64_t num_blocks = 0;
@@ -685,7 +632,8 @@ int launch_contains_policy(b2co_bloom* f, void const* keys, uint8_t const* stenc
 // at 16 keys per block) and routing's fixed cost of about 45 us dominates.
 constexpr uint64_t kPartitionKeysPerBlock = 8;
 constexpr uint64_t kPartitionFilterBytes = uint64_t(64) << 20;
-// Keys per route-and-apply round (the record workspace holds this many).
+// Keys per route-and-apply round.  A batch that passes it by less than an eighth
+// stays one round: a round costs about 100 us however few its keys.
 constexpr uint64_t kPartitionRound = uint64_t(1) << 27;
 
 template <int KB>
@@ -693,16 +641,9 @@ int launch_add_partitioned(b2co_bloom* f, void const* keys, uint8_t const* stenc
 {
     uint32_t const nblocks = uint32_t(f->num_blocks);
     uint32_t const nslices = (nblocks + kSliceBlocks - 1) / kSliceBlocks;
-    uint64_t const want = n < kPartitionRound ? n : kPartitionRound;
-    if (f->recs_cap < want) {
-        if (f->recs) cudaFree(f->recs);
-        f->recs = nullptr;
-        f->recs_cap = 0;
-        B2CO_CUDA(cudaMalloc(&f->recs, want * 8));
-        f->recs_cap = want;
-    }
+    uint64_t const rounds = (n + kPartitionRound / 8 * 9 - 1) / (kPartitionRound / 8 * 9);
+    uint64_t const round = (n + rounds - 1) / rounds;
     auto const route = k_bloom_route<KB>;
-    auto const count = k_bloom_count<KB>;
     size_t const apply_smem = size_t(kSliceBlocks) * 32;
     size_t const rsmem = route_smem(nslices);
     B2CO_CUDA(cudaFuncSetAttribute((void const*)route, cudaFuncAttributeMaxDynamicSharedMemorySize, int(rsmem)));
@@ -710,9 +651,19 @@ int launch_add_partitioned(b2co_bloom* f, void const* keys, uint8_t const* stenc
                                    int(apply_smem)));
     int per_sm = 0;
     B2CO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (void const*)route, kRouteThreads, rsmem));
+    uint64_t const tiles = (round + kRouteTile - 1) / kRouteTile;
     uint32_t const route_cap = uint32_t(per_sm < 1 ? 1 : per_sm) * uint32_t(sm_count());
-    // counts[route CTA][slice], then the slice totals and offsets
-    size_t const part_words = size_t(route_cap) * kMaxSlices + 2 * size_t(kMaxSlices) + 1;
+    uint32_t const nctas = uint32_t(tiles < route_cap ? tiles : route_cap);
+    uint32_t const segment = route_segment(round, nctas, nslices);
+    uint64_t const want = uint64_t(nslices) * nctas * segment;
+    if (f->recs_cap < want) {
+        if (f->recs) cudaFree(f->recs);
+        f->recs = nullptr;
+        f->recs_cap = 0;
+        B2CO_CUDA(cudaMalloc(&f->recs, want * 8));
+        f->recs_cap = want;
+    }
+    size_t const part_words = size_t(route_cap) * kMaxSlices;
     if (f->part_words < part_words) {
         if (f->part) cudaFree(f->part);
         f->part = nullptr;
@@ -720,22 +671,14 @@ int launch_add_partitioned(b2co_bloom* f, void const* keys, uint8_t const* stenc
         B2CO_CUDA(cudaMalloc(&f->part, part_words * 4));
         f->part_words = part_words;
     }
-    uint32_t* counts = f->part;
-    uint32_t* totals = counts + size_t(route_cap) * kMaxSlices;
-    uint32_t* offsets = totals + kMaxSlices;
     if (int st = f->part_order.begin(s)) return st;
-    for (uint64_t at = 0; at < n; at += kPartitionRound) {
-        uint64_t const m = n - at < kPartitionRound ? n - at : kPartitionRound;
+    for (uint64_t at = 0; at < n; at += round) {
+        uint64_t const m = n - at < round ? n - at : round;
         void const* k = static_cast<char const*>(keys) + at * KB;
         uint8_t const* st = stencil ? stencil + at : nullptr;
-        uint64_t const tiles = (m + kRouteTile - 1) / kRouteTile;
-        uint32_t const nctas = uint32_t(tiles < route_cap ? tiles : route_cap);
-        count<<<nctas, 1024, 0, s>>>(nblocks, f->seed, k, st, m, nslices, nctas, counts);
-        k_bloom_colscan<<<(nslices + 255) / 256, 256, 0, s>>>(counts, nslices, nctas, totals);
-        k_bloom_scan<<<1, 1024, 0, s>>>(totals, nslices, offsets);
-        route<<<nctas, kRouteThreads, rsmem, s>>>(nblocks, f->seed, k, st, m, nslices, nctas, counts, offsets,
-                                                      f->recs);
-        k_bloom_apply<<<nslices, kApplyThreads, apply_smem, s>>>(f->words, nblocks, f->recs, offsets);
+        route<<<nctas, kRouteThreads, rsmem, s>>>(f->words, nblocks, f->seed, k, st, m, nslices, nctas, segment, f->part,
+                                                  f->recs);
+        k_bloom_apply<<<nslices, kApplyThreads, apply_smem, s>>>(f->words, nblocks, f->recs, f->part, nctas, segment);
     }
     B2CO_CUDA(cudaGetLastError());
     return f->part_order.end(s);
