@@ -8,8 +8,8 @@
 // B200 design: Add keeps a private copy of the registers in shared memory
 // (p <= 17: 8..128 KiB per CTA of 1024 threads), reads each key once from HBM
 // in 16-byte loads, and raises a shared register with a compare-and-swap loop
-// only when the new rank is larger (after warm-up almost never).  Each CTA then folds its copy into the
-// global registers with a per-byte max (__vmaxu4) CAS on words that changed.
+// only when the new rank is larger (after warm-up almost never).  Each CTA folds its copy into the
+// global registers with a per-byte max (__vmaxu4) CAS on words that changed, large batches early as well.
 // p = 18 (256 KiB) exceeds shared memory and updates the global registers
 // directly, with the same read-before-CAS filter.  Estimate builds the 65-bin
 // rank histogram on the device and finishes with the HLL++ finalizer on the host.
@@ -71,13 +71,16 @@ __device__ __forceinline__ void fold_word(uint32_t* g, uint32_t mine)
 }
 
 // Precision as a compile-time constant: the index and rank shifts become
-// immediates.
+// immediates.  The rank comes from the first 32 bits after the index; only a
+// hash with none of them set (one key in 2^32) needs the rest.
 template <int KB, int P>
 __device__ __forceinline__ void hll_locate_p(uint64_t key, uint32_t& index, uint32_t& rank)
 {
     uint64_t const h = xxh64<KB>(key, 0);
     index = uint32_t(h >> (64 - P));
-    rank = uint32_t(__clzll((long long)((h << P) | (1ull << (P - 1))))) + 1u;
+    uint32_t const top = uint32_t(h >> (32 - P));
+    rank = uint32_t(__clz(int(top))) + 1u;
+    if (top == 0) rank = 33u + uint32_t(__clz(int((uint32_t(h) << P) | (1u << (P - 1)))));
 }
 
 constexpr int kHllBlock = 1024;
@@ -86,29 +89,39 @@ constexpr int kHllBlock = 1024;
 // private register copy (2^P bytes of shared memory), so at p = 16 two CTAs
 // fill an SM's 64 warps.  Keys before the first 16-byte boundary (`head`) and
 // after the last whole vector go one per thread.
+//
+// Bound by instruction issue: xxh64's five 64-bit multiplies, and the raises.
+//  * The loop is the same for all lanes of a warp and ends a round with a warp
+//    barrier: lanes that come out of the compare-and-swap loop one by one would
+//    run the keys that follow one by one as well.  (The same loop without the
+//    barrier: 864 -> 2,456 us for 2^28 keys.)
+//  * A private copy sees only its CTA's share of the keys (2^28 keys over 296 CTAs
+//    at p = 16: 14 per register), so alone it would be raised by a quarter of them.
+//    Batches with a register's worth of keys per CTA or more (`exchanges` > 0)
+//    therefore start from the global registers and exchange with them once a CTA
+//    has taken a quarter of that, and again at the whole of it when four times
+//    that is to come: it folds its copy in and takes the maximum back.  No CTA
+//    waits for another: a register only grows.  None, one, two exchanges: 864, 805
+//    and 742 us; the per-lane loop before them 990.
 template <int KB, int P>
 __global__ void __launch_bounds__(kHllBlock, P <= 16 ? 2 : 1)
-    k_hll_add_vec(uint32_t* regs, void const* keys, uint64_t n, uint64_t head)
+    k_hll_add_vec(uint32_t* regs, void const* keys, uint64_t n, uint64_t head, int exchanges)
 {
     extern __shared__ uint32_t sk[];
-    constexpr uint32_t kWords = (1u << P) / 4;
-    constexpr int V = 16 / KB;        // keys per 16-byte load
+    constexpr uint32_t kRegs = 1u << P, kWords = kRegs / 4;
+    constexpr int V = 16 / KB;          // keys per 16-byte load
     constexpr int U = KB == 8 ? 2 : 1;  // loads in flight per thread
-    for (uint32_t i = threadIdx.x; i < kWords; i += kHllBlock) sk[i] = 0;
+    for (uint32_t i = threadIdx.x; i < kWords; i += kHllBlock)
+        sk[i] = exchanges ? *reinterpret_cast<volatile uint32_t*>(regs + i) : 0u;
     __syncthreads();
     uint64_t const tid = uint64_t(blockIdx.x) * kHllBlock + threadIdx.x;
     uint64_t const stride = uint64_t(gridDim.x) * kHllBlock;
+    uint32_t const lane = threadIdx.x & 31;
     auto add = [&](uint64_t key) {
         uint32_t x, r;
         hll_locate_p<KB, P>(key, x, r);
-        raise_register(sk, x, r);  // a word load decides; a byte load measured 3.5x slower
+        if (reinterpret_cast<volatile uint8_t*>(sk)[x] < r) raise_register(sk, x, r);
     };
-    uint64_t const body = head < n ? n - head : 0;
-    uint64_t const nvec = body / V;
-    uint64_t const tail0 = head + nvec * V;
-    for (uint64_t i = tid; i < head && i < n; i += stride) add(load_key<KB>(keys, i));
-    for (uint64_t i = tail0 + tid; i < n; i += stride) add(load_key<KB>(keys, i));
-    uint4 const* vk = reinterpret_cast<uint4 const*>(static_cast<char const*>(keys) + head * KB);
     auto add_vec = [&](uint4 q) {
         if constexpr (KB == 8) {
             add(uint64_t(q.x) | (uint64_t(q.y) << 32));
@@ -120,17 +133,45 @@ __global__ void __launch_bounds__(kHllBlock, P <= 16 ? 2 : 1)
             add(q.w);
         }
     };
-    uint64_t v = tid;
-    for (; v + (U - 1) * stride < nvec; v += U * stride) {
-        uint4 q[U];
+    uint64_t const body = head < n ? n - head : 0;
+    uint64_t const nvec = body / V;
+    uint64_t const tail0 = head + nvec * V;
+    for (uint64_t i = tid; i < head && i < n; i += stride) add(load_key<KB>(keys, i));
+    for (uint64_t i = tail0 + tid; i < n; i += stride) add(load_key<KB>(keys, i));
+    __syncwarp();
+    uint4 const* vk = reinterpret_cast<uint4 const*>(static_cast<char const*>(keys) + head * KB);
+    uint64_t v = tid - lane;  // the warp's first vector of a round
+    auto run = [&](uint64_t until) {
+        for (; v + 31 + (U - 1) * stride < until; v += U * stride) {
+            uint4 q[U];
 #pragma unroll
-        for (int j = 0; j < U; ++j) q[j] = __ldcs(vk + v + j * stride);
+            for (int j = 0; j < U; ++j) q[j] = __ldcs(vk + v + lane + j * stride);
 #pragma unroll
-        for (int j = 0; j < U; ++j) add_vec(q[j]);
+            for (int j = 0; j < U; ++j) add_vec(q[j]);
+            __syncwarp();
+        }
+    };
+    for (int e = 0; e < exchanges; ++e) {
+        run(uint64_t(gridDim.x) * ((e == 0 ? kRegs / 4 : kRegs) / V));
+        __syncthreads();
+        // every CTA takes the words in another turn, so that they do not all retry on
+        // the same ones
+        for (uint32_t i = threadIdx.x; i < kWords; i += kHllBlock) {
+            uint32_t const w = (i + blockIdx.x * 64) % kWords;
+            fold_word(regs + w, *reinterpret_cast<volatile uint32_t*>(sk + w));
+            fold_word(sk + w, *reinterpret_cast<volatile uint32_t*>(regs + w));
+        }
+        __syncthreads();
     }
-    for (; v < nvec; v += stride) add_vec(__ldcs(vk + v));
+    run(nvec);
+    for (; v < nvec; v += stride) {  // the last rounds; lanes past the end add the last vector again
+        uint64_t const at = v + lane < nvec ? v + lane : nvec - 1;
+        add_vec(__ldcs(vk + at));
+        __syncwarp();
+    }
     __syncthreads();
-    for (uint32_t w = threadIdx.x; w < kWords; w += kHllBlock) {
+    for (uint32_t i = threadIdx.x; i < kWords; i += kHllBlock) {
+        uint32_t const w = (i + blockIdx.x * 64) % kWords;
         uint32_t const mine = sk[w];
         if (mine) fold_word(regs + w, mine);
     }
@@ -293,7 +334,7 @@ int add_launch(b2co_hll* h, void const* keys, uint64_t n, cudaStream_t s)
 {
     uint32_t const p = h->precision;
     if (p <= 17) {
-        using AddFn = void (*)(uint32_t*, void const*, uint64_t, uint64_t);
+        using AddFn = void (*)(uint32_t*, void const*, uint64_t, uint64_t, int);
         static AddFn const fns[2][5] = {
             {k_hll_add_vec<4, 13>, k_hll_add_vec<4, 14>, k_hll_add_vec<4, 15>, k_hll_add_vec<4, 16>,
              k_hll_add_vec<4, 17>},
@@ -319,7 +360,9 @@ int add_launch(b2co_hll* h, void const* keys, uint64_t n, cudaStream_t s)
         // keys up to the first 16-byte boundary go one per thread
         uintptr_t const addr = reinterpret_cast<uintptr_t>(keys);
         uint64_t const head = ((16 - addr % 16) % 16) / h->key_bytes;
-        k<<<grid, kHllBlock, smem, s>>>(h->regs, keys, n, head);
+        uint64_t const per_register = (n / grid) >> p;  // keys of a CTA
+        int const exchanges = grid == 1 || per_register == 0 ? 0 : per_register < 4 ? 1 : 2;
+        k<<<grid, kHllBlock, smem, s>>>(h->regs, keys, n, head, exchanges);
     } else {
         void (*k)(uint32_t*, uint32_t, void const*, uint64_t) =
             h->key_bytes == 8 ? k_hll_add_global<8> : k_hll_add_global<4>;
