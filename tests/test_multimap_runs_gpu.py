@@ -53,3 +53,48 @@ def test_runs_come_back_ascending(kb, vb, name):
     first = torch.zeros(len(q), dtype=torch_dt(vb), device="cuda")
     m.Find(dev(q), first)
     assert np.array_equal(first.cpu().numpy(), np.where(hi > lo, vs[np.minimum(lo, len(vs) - 1)], -1).astype(NP_DT[vb]))
+
+
+def fmix64_inverse(h):
+    """Keys whose MurmurHash3 64-bit finalizer is h (each step of it undone)."""
+    m = (1 << 64) - 1
+    x = h.astype(object)
+    inv1 = pow(0xC4CEB9FE1A85EC53, -1, 1 << 64)
+    inv2 = pow(0xFF51AFD7ED558CCD, -1, 1 << 64)
+    x = x ^ (x >> 33)
+    x = (x * inv1) & m
+    x = x ^ (x >> 33)
+    x = (x * inv2) & m
+    x = x ^ (x >> 33)
+    return np.array([int(v) for v in x], dtype=np.uint64).view(np.int64)
+
+
+@pytest.mark.parametrize("distinct,crowd", [(1500, 0), (1500, 300), (400_000, 0)])
+def test_table_sized_by_the_distinct_keys(distinct, crowd):
+    """Batches large enough for a table of the estimated number of keys; with `crowd` keys that all hash to one place,
+    so that the small table is given up for a full-size one."""
+    import b2co
+    import torch
+    rng = np.random.default_rng(distinct + crowd)
+    n = (1 << 20) + 3
+    keys = np.unique(rng.integers(0, 2**62, size=distinct, dtype=np.int64))
+    if crowd:
+        keys = np.concatenate([keys, fmix64_inverse((np.arange(1, crowd + 1, dtype=np.uint64) << np.uint64(40)) + np.uint64(77))])
+    keys = keys[keys != -1]
+    at = np.concatenate([np.arange(len(keys)), rng.integers(0, len(keys), size=n - len(keys))])
+    v = rng.integers(0, 2**40, size=n, dtype=np.int64)
+    m = b2co.StaticMultimap(n, -1, -1, key_dtype=torch.int64, value_dtype=torch.int64)
+    assert m.Insert(b2co.pack_pairs(dev(keys[at]), dev(v))) == 0
+    q = np.concatenate([keys, keys ^ np.int64(1 << 50)])
+    counts = np.bincount(at, minlength=len(keys))
+    total = int(counts.sum())
+    assert m.Count(dev(keys)) == total
+    ko = torch.zeros(total, dtype=torch.int64, device="cuda")
+    vo = torch.zeros(total, dtype=torch.int64, device="cuda")
+    assert m.Retrieve(dev(keys), ko, vo, total) == total
+    order = np.lexsort((v, at))
+    assert np.array_equal(ko.cpu().numpy(), keys[at[order]])
+    assert np.array_equal(vo.cpu().numpy(), v[order])
+    flags = torch.zeros(len(q), dtype=torch.uint8, device="cuda")
+    m.Contains(dev(q), flags)
+    assert np.array_equal(flags.cpu().numpy(), np.isin(q, keys).astype(np.uint8))
