@@ -21,9 +21,12 @@
 // short as a rule, so the values of a tile of runs are sorted in shared memory,
 // where sorting all (value, key) records together takes one pass over memory per
 // byte of both (16.8 M int64 pairs over 4.2 M keys: twelve passes, 4.9 ms, against 125 us
-// for sorting the runs and 800 for scattering the values into them).
+// for sorting the runs).  The pairs of large batches are grouped partition by
+// partition (565 us for those pairs: survey 55, route 274, build 225), others in a
+// table that all blocks share (1,700 us).
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <new>
 
 #include "multi_common.cuh"
@@ -235,6 +238,13 @@ __global__ void __launch_bounds__(256) k_mmap_append(typename SlotT<KB, VB>::Raw
 
 // ---- grouped index ---------------------------------------------------------
 
+template <int KB>
+__device__ __forceinline__ uint64_t run_hash(KeyWord<KB> k)
+{
+    if constexpr (KB == 4) return uint64_t(fmix32(k, 0)) << 32;
+    else return fmix64(k, 0);
+}
+
 // One distinct key: its run is csr[offset, offset + count).  A slot is one
 // 16-byte word, so adding to a key or asking for it touches one sector, not one
 // each for key, count and offset.
@@ -244,11 +254,19 @@ struct alignas(16) RunSlot {
     uint32_t count, offset;
 };
 
+// A key's probing starts at the leading bits of its hash and goes round the
+// region (a power of two of slots) that it starts in: the whole table, or the
+// part of it that one block builds in shared memory.
 template <int KB>
 struct RunTable {
     RunSlot<KB>* slots;
-    uint64_t mask;  // table size - 1 (a power of two); at most half full
+    uint64_t mask;    // table size - 1 (a power of two); at most half full
+    uint64_t region;  // region size - 1
+    uint32_t shift;   // 64 - log2(table size)
     KeyWord<KB> empty;
+
+    __device__ __forceinline__ uint64_t start(KeyWord<KB> k) const { return run_hash<KB>(k) >> shift; }
+    __device__ __forceinline__ uint64_t next(uint64_t s) const { return (s & ~region) | ((s + 1) & region); }
 };
 
 template <int KB>
@@ -265,7 +283,7 @@ __device__ __forceinline__ bool find_run(RunTable<KB> const& t, KeyWord<KB> k, R
 {
     out.count = 0;
     if (k == t.empty) return false;
-    uint64_t s = table_hash<KB>(k) & t.mask;
+    uint64_t s = t.start(k);
     for (;;) {
         RunSlot<KB> const cur = load_run<KB>(t.slots + s);
         if (cur.key == k) {
@@ -273,7 +291,7 @@ __device__ __forceinline__ bool find_run(RunTable<KB> const& t, KeyWord<KB> k, R
             return true;
         }
         if (cur.key == t.empty) return false;
-        s = (s + 1) & t.mask;
+        s = t.next(s);
     }
 }
 
@@ -284,6 +302,16 @@ __global__ void __launch_bounds__(256) k_run_clear(RunTable<KB> t)
     RunSlot<KB> const e{t.empty, 0u, 0u};
     for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) t.slots[i] = e;
 }
+
+// Counters of one build: runs << 32 | values, then the runs too long for the
+// tile sort, then (found by the long-run sort) the runs left to the radix sort
+// and their values.
+struct RunCounters {
+    unsigned long long cursor;
+    unsigned int nlong, ngiant;
+    unsigned long long giant_values;
+    unsigned int crowded, pad;
+};
 
 constexpr uint32_t kNoPlace = 0xffffffffu;  // no rank in a run: runs have fewer pairs
 constexpr uint32_t kMaxProbes = 128;  // of a table sized by an estimate
@@ -299,13 +327,13 @@ __global__ void __launch_bounds__(256) k_run_count(RunTable<KB> t, typename Slot
     uint64_t const stride = uint64_t(gridDim.x) * blockDim.x;
     for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
         KeyWord<KB> const k = KeyWord<KB>(S::key(dense[i]));
-        uint64_t s = table_hash<KB>(k) & t.mask;
+        uint64_t s = t.start(k);
         uint32_t probes = 0;
         for (;;) {
             KeyWord<KB> cur = t.slots[s].key;
             if (cur == t.empty) cur = atomicCAS(&t.slots[s].key, t.empty, k);
             if (cur == t.empty || cur == k) break;
-            s = (s + 1) & t.mask;
+            s = t.next(s);
             if (crowded && ++probes == kMaxProbes) {
                 *crowded = 1;
                 break;
@@ -372,24 +400,34 @@ __global__ void __launch_bounds__(256) k_run_scatter(RunTable<KB> t, typename Sl
     }
 }
 
-// Estimate of the number of distinct keys (HyperLogLog with 2^11 registers, one
-// pass over the keys, 50 us for 16.8 M pairs): it sizes the table, so a table of
-// few distinct keys stays small, and with it the random accesses of every later
-// pass.  4.2 M keys: clearing 180 -> 46 us, counting 878 -> 588, each probing of 2 M
-// queries 59 -> 44.
+// Survey of a large batch's keys in one pass (55 us for 16.8 M pairs): an estimate of
+// how many are distinct (HyperLogLog with 2^11 registers), which sizes the table,
+// and the sizes of the partitions by the leading bits of the hash.
 constexpr uint32_t kEstimateBits = 11, kEstimateRegs = 1u << kEstimateBits;
+constexpr uint32_t kMaxPartBits = 12, kMaxParts = 1u << kMaxPartBits;
+
+struct Survey {  // device; the host reads regs and counts
+    unsigned int regs[kEstimateRegs];
+    unsigned int counts[kMaxParts];
+    unsigned int cursors[kMaxParts];
+    unsigned int starts[kMaxParts + 1];
+};
 
 template <int KB, int VB>
-__global__ void __launch_bounds__(512) k_run_estimate(typename SlotT<KB, VB>::Raw const* dense, uint64_t n,
-                                                      unsigned int* regs)
+__global__ void __launch_bounds__(512) k_run_survey(typename SlotT<KB, VB>::Raw const* dense, uint64_t n,
+                                                    uint32_t pbits, Survey* out)
 {
     using S = SlotT<KB, VB>;
-    __shared__ unsigned int sk[kEstimateRegs];
+    __shared__ unsigned int sk[kEstimateRegs], hist[kMaxParts];
+    uint32_t const parts = 1u << pbits;
     for (uint32_t i = threadIdx.x; i < kEstimateRegs; i += blockDim.x) sk[i] = 0;
+    for (uint32_t i = threadIdx.x; i < parts; i += blockDim.x) hist[i] = 0;
     __syncthreads();
     uint64_t const stride = uint64_t(gridDim.x) * blockDim.x;
     for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-        uint64_t const h = fmix64(S::key(dense[i]), 0x2545f4914f6cdd1dull);
+        uint64_t const key = S::key(dense[i]);
+        atomicAdd(hist + uint32_t(run_hash<KB>(KeyWord<KB>(key)) >> (64 - pbits)), 1u);
+        uint64_t const h = fmix64(key, 0x2545f4914f6cdd1dull);
         uint32_t const x = uint32_t(h >> (64 - kEstimateBits));
         uint32_t const rank = uint32_t(__clzll((long long)((h << kEstimateBits) | 1ull))) + 1u;
         if (*reinterpret_cast<volatile unsigned int*>(sk + x) < rank) atomicMax(sk + x, rank);
@@ -397,8 +435,174 @@ __global__ void __launch_bounds__(512) k_run_estimate(typename SlotT<KB, VB>::Ra
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < kEstimateRegs; i += blockDim.x) {
         uint32_t const w = (i + blockIdx.x * 64) % kEstimateRegs;
-        if (sk[w]) atomicMax(regs + w, sk[w]);
+        if (sk[w]) atomicMax(out->regs + w, sk[w]);
     }
+    for (uint32_t i = threadIdx.x; i < parts; i += blockDim.x) {
+        uint32_t const w = (i + blockIdx.x * 64) & (parts - 1);
+        if (hist[w]) atomicAdd(out->counts + w, hist[w]);
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) k_part_starts(Survey* s, uint32_t parts)  // one block
+{
+    uint32_t const per = (parts + kThreads - 1) / kThreads, p0 = threadIdx.x * per;
+    uint64_t sum = 0, total;
+    for (uint32_t p = p0; p < p0 + per && p < parts; ++p) sum += s->counts[p];
+    uint64_t at = block_excl_scan(sum, &total);
+    for (uint32_t p = p0; p < p0 + per && p < parts; ++p) {
+        s->starts[p] = s->cursors[p] = uint32_t(at);
+        at += s->counts[p];
+    }
+    if (threadIdx.x == 0) s->starts[parts] = uint32_t(total);
+}
+
+// The pairs of a partition come to lie together, in any order: a block ranks a
+// tile's pairs in their partitions in shared memory, takes the tile's places with
+// one atomic a partition and stores every pair to its place.  The stores of the
+// blocks at work meet in L2 (a partition grows at one end), which puts sectors
+// together, so the pairs need no sorting on the way: 16.8 M pairs of 16 bytes are read
+// and written once, 0.58 GB in 274 us.  Bound by the block's phases, which wait
+// on one another (a load, an atomic in shared memory and one in L2, a store).
+constexpr int kRouteThreads = 1024, kRoutePer = 8;
+template <int KB, int VB>
+__global__ void __launch_bounds__(kRouteThreads, 1)
+    k_part_route(typename SlotT<KB, VB>::Raw const* dense, uint64_t n, uint32_t pbits, Survey* survey,
+                 typename SlotT<KB, VB>::Raw* out)
+{
+    using S = SlotT<KB, VB>;
+    __shared__ uint32_t at[kMaxParts];
+    uint32_t const parts = 1u << pbits;
+    constexpr uint64_t kTileOf = uint64_t(kRouteThreads) * kRoutePer;
+    for (uint64_t base = uint64_t(blockIdx.x) * kTileOf; base < n; base += uint64_t(gridDim.x) * kTileOf) {
+        for (uint32_t p = threadIdx.x; p < parts; p += kRouteThreads) at[p] = 0;
+        typename S::Raw pr[kRoutePer];
+#pragma unroll
+        for (int r = 0; r < kRoutePer; ++r) {
+            uint64_t const i = base + uint64_t(r) * kRouteThreads + threadIdx.x;
+            if (i < n) pr[r] = ld_ro(dense + i);
+        }
+        __syncthreads();
+        uint32_t place[kRoutePer];  // partition | rank in the tile's share of it
+#pragma unroll
+        for (int r = 0; r < kRoutePer; ++r) {
+            uint64_t const i = base + uint64_t(r) * kRouteThreads + threadIdx.x;
+            if (i < n) {
+                uint32_t const p = uint32_t(run_hash<KB>(KeyWord<KB>(S::key(pr[r]))) >> (64 - pbits));
+                place[r] = p | (atomicAdd(at + p, 1u) << kMaxPartBits);
+            }
+        }
+        __syncthreads();
+        for (uint32_t p = threadIdx.x; p < parts; p += kRouteThreads) {
+            uint32_t const c = at[p];
+            if (c) at[p] = atomicAdd(survey->cursors + p, c);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kRoutePer; ++r) {
+            uint64_t const i = base + uint64_t(r) * kRouteThreads + threadIdx.x;
+            if (i < n) out[at[place[r] & (kMaxParts - 1)] + (place[r] >> kMaxPartBits)] = pr[r];
+        }
+        __syncthreads();
+    }
+}
+
+// One block builds one partition's region of the table in shared memory: it
+// counts the keys, scans the counts (a warp its share of the slots), writes the
+// region and the runs, and scatters the values within the partition's stretch
+// of the CSR array.  Every access to memory is a stretch read or written whole, or
+// lands in one that is in L2, where k_run_count, k_run_offsets and k_run_scatter
+// (598, 194 and 821 us for 16.8 M int64 pairs over 4.2 M keys) pay a random access to HBM
+// each.  225 us for them, 0.65 GB; bound by the probing in shared memory.
+constexpr int kPartThreads = 512;
+template <int KB, int VB>
+__global__ void __launch_bounds__(kPartThreads)
+    k_part_build(RunTable<KB> t, typename SlotT<KB, VB>::Raw const* pairs, Survey const* survey, RunCounters* ctr,
+                 uint2* runs, ValueWord<VB>* csr)
+{
+    using S = SlotT<KB, VB>;
+    constexpr int kWarps = kPartThreads / 32, kBatch = 4;
+    extern __shared__ __align__(16) unsigned char region_smem[];
+    __shared__ unsigned long long warp_at[kWarps];
+    uint32_t const region = uint32_t(t.region), slots = region + 1;
+    KeyWord<KB>* const keys = reinterpret_cast<KeyWord<KB>*>(region_smem);
+    uint32_t* const counts = reinterpret_cast<uint32_t*>(keys + slots);
+    uint32_t const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t const begin = survey->starts[blockIdx.x], end = survey->starts[blockIdx.x + 1];
+    for (uint32_t i = threadIdx.x; i < slots; i += kPartThreads) keys[i] = t.empty, counts[i] = 0;
+    __syncthreads();
+    // the slot of a key that is there or finds room; ~0 when the region is crowded
+    auto slot_of = [&](KeyWord<KB> k) {
+        uint32_t s = uint32_t(t.start(k)) & region;
+        for (uint32_t probes = 0; probes < kMaxProbes; ++probes, s = (s + 1) & region) {
+            KeyWord<KB> cur = *reinterpret_cast<KeyWord<KB> volatile*>(keys + s);
+            if (cur == t.empty) cur = atomicCAS(keys + s, t.empty, k);
+            if (cur == t.empty || cur == k) return s;
+        }
+        return ~0u;
+    };
+    // f(pair) for every pair of the partition, whole warps at a time
+    auto each = [&](auto f) {
+        for (uint64_t base = uint64_t(begin) + warp * 32; base < end; base += kBatch * kPartThreads) {
+            typename S::Raw pr[kBatch];
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b)
+                if (base + b * kPartThreads + lane < end) pr[b] = ld_ro(pairs + base + b * kPartThreads + lane);
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b) {
+                if (base + b * kPartThreads + lane < end) f(pr[b]);
+                __syncwarp();  // lanes that probed on longer rejoin
+            }
+        }
+    };
+    each([&](typename S::Raw const& pr) {
+        uint32_t const s = slot_of(KeyWord<KB>(S::key(pr)));
+        if (s == ~0u) ctr->crowded = 1;
+        else atomicAdd(counts + s, 1u);
+    });
+    __syncthreads();
+    uint32_t const share = slots / kWarps, first = warp * share;
+    unsigned long long sum = 0;
+    for (uint32_t i = lane; i < share; i += 32) {
+        uint32_t const c = counts[first + i];
+        sum += c ? (1ull << 32) + c : 0;
+    }
+#pragma unroll
+    for (int d = 16; d; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    if (lane == 0) warp_at[warp] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long total = 0;
+        for (int w = 0; w < kWarps; ++w) total += warp_at[w];
+        unsigned long long at = total ? atomicAdd(&ctr->cursor, total) : 0;
+        for (int w = 0; w < kWarps; ++w) {
+            unsigned long long const v = warp_at[w];
+            warp_at[w] = at;
+            at += v;
+        }
+    }
+    __syncthreads();
+    unsigned long long carry = warp_at[warp];
+    RunSlot<KB>* const out = t.slots + uint64_t(blockIdx.x) * slots;
+    for (uint32_t i = lane; i < share; i += 32) {
+        uint32_t const s = first + i, c = counts[s];
+        unsigned long long const mine = c ? (1ull << 32) + c : 0;
+        unsigned long long incl = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            unsigned long long const o = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= uint32_t(d)) incl += o;
+        }
+        unsigned long long const at = carry + incl - mine;
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+        out[s] = RunSlot<KB>{keys[s], c, c ? uint32_t(at) : 0u};
+        if (c) runs[at >> 32] = make_uint2(uint32_t(at), c);
+        counts[s] = uint32_t(at);
+    }
+    __syncthreads();
+    each([&](typename S::Raw const& pr) {
+        uint32_t const s = slot_of(KeyWord<KB>(S::key(pr)));
+        if (s != ~0u) csr[atomicAdd(counts + s, 1u)] = ValueWord<VB>(S::value(pr));
+    });
 }
 
 // Upper end of what the registers say (standard error 2.3%, linear counting
@@ -416,16 +620,6 @@ uint64_t estimate_distinct(unsigned int const* regs)
     if (e <= 2.5 * m && zeros) e = m * std::log(m / zeros);
     return uint64_t(1.1 * e) + 64;
 }
-
-// Counters of one build: runs << 32 | values, then the runs too long for the
-// tile sort, then (found by the long-run sort) the runs left to the radix sort
-// and their values.
-struct RunCounters {
-    unsigned long long cursor;
-    unsigned int nlong, ngiant;
-    unsigned long long giant_values;
-    unsigned int crowded, pad;
-};
 
 constexpr int kRunTile = 256;            // runs per block of the tile sort, one a thread
 constexpr uint32_t kRunThread = 24;      // longest run that one thread sorts (insertion, in shared memory)
@@ -692,15 +886,17 @@ struct b2co_mmap {
     Scratch scratch, build, hist, records;
     RunCounters* d_ctr = nullptr;
     RunCounters* h_ctr = nullptr;  // pinned
-    unsigned int* d_regs = nullptr;  // distinct-key estimate; made at the first build that wants one
-    unsigned int* h_regs = nullptr;  // pinned
+    uint64_t region = 0;             // slots of a probing region of the table
+    Survey* d_survey = nullptr;      // made at the first build that wants one
+    Survey* h_survey = nullptr;      // pinned
     unsigned int* d_status = nullptr;
     uint64_t* h_word = nullptr;
 
     template <int KB>
     RunTable<KB> table() const
     {
-        return RunTable<KB>{static_cast<RunSlot<KB>*>(tslots), tsize - 1, KeyWord<KB>(ek)};
+        return RunTable<KB>{static_cast<RunSlot<KB>*>(tslots), tsize - 1, region - 1,
+                            uint32_t(64 - __builtin_ctzll(tsize)), KeyWord<KB>(ek)};
     }
     uint32_t slot_bytes() const { return (kb == 4 && vb == 4) ? 8 : 16; }
 };
@@ -876,27 +1072,86 @@ int mmap_sort_giants(b2co_mmap* m, uint2 const* runs, uint32_t const* giants, ui
     return B2CO_OK;
 }
 
-// Pairs from which the table is sized by an estimate of the distinct keys.  Below,
-// the full-size table is in L2 anyway and the estimate's pass and wait (about 20 us) cost more.
-constexpr uint64_t kEstimatePairs = 1ull << 20;
+// Pairs from which the keys are surveyed.  Below, the full-size table is in L2
+// anyway and the survey's pass and wait (about 20 us) cost more.
+constexpr uint64_t kSurveyPairs = 1ull << 20;
+constexpr uint64_t kMinRegion = 512;             // slots; a larger one only for the partitions' size
+constexpr uint64_t kMaxRegionBytes = 200 << 10;  // of shared memory
 
+// The table's size, and the bits of the partition number when the index is to be
+// built by partitions: when a partition's share of the table fits shared memory
+// and no partition is over four times as large as they are on average (one block
+// would be at work on it long after the others).  Whole builds, shared table and
+// partitions, in us, n pairs over n / 4 and n / 256 int64 keys: n = 2^20: 174, 165 and 248, 243;
+// 2^22: 361, 270 and 586, 554; 2^24: 1,907, 750 and 1,959, 1,736; 2^26: 10,260, 3,600 and 8,710, 6,796.
+// 2,048 partitions against 4,096, over n / 4 keys: 2^22: 270 and 284; 2^24: 760 and 750 (over n: 964 and
+// 878); 2^26: only the smaller ones fit.
 template <int KB, int VB>
-int mmap_table_size(b2co_mmap* m, cudaStream_t st, uint64_t* tsize)
+int mmap_plan(b2co_mmap* m, cudaStream_t st, uint64_t* tsize, uint32_t* part_bits)
 {
     uint64_t const n = m->size;
     *tsize = table_size_for(n);
-    if (n < kEstimatePairs) return B2CO_OK;
+    *part_bits = 0;
+    if (n < kSurveyPairs) return B2CO_OK;
     using Raw = typename SlotT<KB, VB>::Raw;
-    if (!m->d_regs) {
-        B2CO_CUDA(cudaMalloc(reinterpret_cast<void**>(&m->d_regs), kEstimateRegs * 4));
-        B2CO_CUDA(cudaMallocHost(reinterpret_cast<void**>(&m->h_regs), kEstimateRegs * 4));
+    if (!m->d_survey) {
+        B2CO_CUDA(cudaMalloc(reinterpret_cast<void**>(&m->d_survey), sizeof(Survey)));
+        B2CO_CUDA(cudaMallocHost(reinterpret_cast<void**>(&m->h_survey), sizeof(Survey)));
     }
-    B2CO_CUDA(cudaMemsetAsync(m->d_regs, 0, kEstimateRegs * 4, st));
-    k_run_estimate<KB, VB><<<uint32_t(sm_count()) * 4, 512, 0, st>>>(static_cast<Raw const*>(m->dense), n, m->d_regs);
+    uint32_t const pbits = n > (1ull << 23) ? kMaxPartBits : kMaxPartBits - 1, parts = 1u << pbits;
+    constexpr size_t kRead = offsetof(Survey, cursors);
+    B2CO_CUDA(cudaMemsetAsync(m->d_survey, 0, kRead, st));
+    k_run_survey<KB, VB><<<uint32_t(sm_count()) * 4, 512, 0, st>>>(static_cast<Raw const*>(m->dense), n, pbits,
+                                                                   m->d_survey);
     B2CO_CUDA(cudaGetLastError());
-    B2CO_CUDA(cudaMemcpyAsync(m->h_regs, m->d_regs, kEstimateRegs * 4, cudaMemcpyDeviceToHost, st));
+    B2CO_CUDA(cudaMemcpyAsync(m->h_survey, m->d_survey, kRead, cudaMemcpyDeviceToHost, st));
     B2CO_CUDA(cudaStreamSynchronize(st));
-    *tsize = std::min(*tsize, table_size_for(estimate_distinct(m->h_regs)));
+    *tsize = std::min(*tsize, table_size_for(estimate_distinct(m->h_survey->regs)));
+    uint64_t const wide = std::max(*tsize, parts * kMinRegion);
+    unsigned int const* const counts = m->h_survey->counts;
+    if ((wide >> pbits) * (KB + 4) <= kMaxRegionBytes &&
+        uint64_t(*std::max_element(counts, counts + parts)) << pbits <= 4 * n) {
+        *tsize = wide;
+        *part_bits = pbits;
+    }
+    return B2CO_OK;
+}
+
+// The index's table, runs and unsorted values by partitions.
+template <int KB, int VB>
+int mmap_group_parts(b2co_mmap* m, cudaStream_t st, uint32_t pbits, void* pairs, uint2* runs)
+{
+    using Raw = typename SlotT<KB, VB>::Raw;
+    uint32_t const parts = 1u << pbits;
+    size_t const smem = size_t(m->region) * (KB + 4);
+    auto* const build = k_part_build<KB, VB>;
+    B2CO_CUDA(cudaFuncSetAttribute((void const*)build, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    k_part_starts<<<1, kThreads, 0, st>>>(m->d_survey, parts);
+    constexpr uint64_t kTileOf = uint64_t(kRouteThreads) * kRoutePer;
+    k_part_route<KB, VB>
+        <<<uint32_t(std::min<uint64_t>((m->size + kTileOf - 1) / kTileOf, uint64_t(sm_count()))), kRouteThreads, 0, st>>>(
+            static_cast<Raw const*>(m->dense), m->size, pbits, m->d_survey, static_cast<Raw*>(pairs));
+    build<<<parts, kPartThreads, smem, st>>>(m->table<KB>(), static_cast<Raw const*>(pairs), m->d_survey, m->d_ctr, runs,
+                                             static_cast<ValueWord<VB>*>(m->csr));
+    B2CO_CUDA(cudaGetLastError());
+    return B2CO_OK;
+}
+
+// The same with random accesses to the whole table.  `place` has room for n places.
+template <int KB, int VB>
+int mmap_group_table(b2co_mmap* m, cudaStream_t st, uint2* place, uint2* runs, bool full)
+{
+    using Raw = typename SlotT<KB, VB>::Raw;
+    auto const* dense = static_cast<Raw const*>(m->dense);
+    uint64_t const n = m->size;
+    RunTable<KB> const t = m->table<KB>();
+    k_run_clear<KB><<<blocks_for(m->tsize), 256, 0, st>>>(t);
+    if (n == 0) return B2CO_OK;
+    k_run_count<KB, VB><<<blocks_for(n), 256, 0, st>>>(t, dense, n, place, full ? nullptr : &m->d_ctr->crowded);
+    k_run_offsets<KB><<<uint32_t(std::min<uint64_t>((n + kTile - 1) / kTile, 148ull * 8)), kThreads, 0, st>>>(
+        t, place, n, &m->d_ctr->cursor, runs);
+    k_run_scatter<KB, VB><<<blocks_for(n), 256, 0, st>>>(t, dense, n, place, static_cast<ValueWord<VB>*>(m->csr));
+    B2CO_CUDA(cudaGetLastError());
     return B2CO_OK;
 }
 
@@ -906,34 +1161,38 @@ template <int KB, int VB>
 int mmap_build(b2co_mmap* m, cudaStream_t st)
 {
     if (!m->dirty) return B2CO_OK;
+    using Raw = typename SlotT<KB, VB>::Raw;
     uint64_t const n = m->size, full = table_size_for(n);
     uint64_t tsize = 0;
-    if (int e = mmap_table_size<KB, VB>(m, st, &tsize)) return e;
-    using Raw = typename SlotT<KB, VB>::Raw;
-    auto const* dense = static_cast<Raw const*>(m->dense);
-    for (;; tsize = full) {  // a table that turns out too small is built again, full-size
+    uint32_t pbits = 0;
+    if (int e = mmap_plan<KB, VB>(m, st, &tsize, &pbits)) return e;
+    // a table that turns out too small is built again, full-size and as a whole
+    for (;; tsize = full, pbits = 0) {
         if (int e = mmap_reserve_index(m, tsize)) return e;
-        RunTable<KB> t = m->table<KB>();
-        auto* csr = static_cast<ValueWord<VB>*>(m->csr);
-        k_run_clear<KB><<<blocks_for(m->tsize), 256, 0, st>>>(t);
-        B2CO_CUDA(cudaGetLastError());
+        m->region = tsize >> pbits;
+        // runs[n] (a key may have one pair only), long runs (of two values or more), giants, and
+        // the partitioned pairs or the pairs' places
+        uint64_t const nlong = n / 2 + 1, ngiant = n / kRunBlock + 1;
+        uint64_t const lists = n * 8 + (nlong + ngiant) * 4 + 8;
+        if (pbits && m->build.reserve(n * sizeof(Raw) + lists)) {
+            cudaGetLastError();  // no room for the partitioned pairs
+            pbits = 0;
+            m->region = tsize;
+        }
+        if (int e = m->build.reserve(n * (pbits ? sizeof(Raw) : sizeof(uint2)) + lists)) return e;
+        auto* const work = m->build.as<unsigned char>();
+        uint2* const runs = reinterpret_cast<uint2*>(work + n * (pbits ? sizeof(Raw) : sizeof(uint2)));
+        uint32_t* const longs = reinterpret_cast<uint32_t*>(runs + n);
+        uint32_t* const giants = longs + nlong;
+        B2CO_CUDA(cudaMemsetAsync(m->d_ctr, 0, sizeof(RunCounters), st));
+        if (int e = pbits ? mmap_group_parts<KB, VB>(m, st, pbits, work, runs)
+                          : mmap_group_table<KB, VB>(m, st, reinterpret_cast<uint2*>(work), runs, tsize == full))
+            return e;
         if (n == 0) {  // an empty table answers every query with a miss
             B2CO_CUDA(cudaStreamSynchronize(st));
             break;
         }
-        // place[n], runs[n] (a key may have one pair only), long runs (of two values or more), giants
-        uint64_t const nlong = n / 2 + 1, ngiant = n / kRunBlock + 1;
-        if (int e = m->build.reserve(n * 16 + (nlong + ngiant) * 4)) return e;
-        uint2* place = m->build.as<uint2>();
-        uint2* runs = place + n;
-        uint32_t* longs = reinterpret_cast<uint32_t*>(runs + n);
-        uint32_t* giants = longs + nlong;
-        B2CO_CUDA(cudaMemsetAsync(m->d_ctr, 0, sizeof(RunCounters), st));
-        k_run_count<KB, VB><<<blocks_for(n), 256, 0, st>>>(t, dense, n, place,
-                                                           tsize < full ? &m->d_ctr->crowded : nullptr);
-        k_run_offsets<KB><<<uint32_t(std::min<uint64_t>((n + kTile - 1) / kTile, 148ull * 8)), kThreads, 0, st>>>(
-            t, place, n, &m->d_ctr->cursor, runs);
-        k_run_scatter<KB, VB><<<blocks_for(n), 256, 0, st>>>(t, dense, n, place, csr);
+        auto* csr = static_cast<ValueWord<VB>*>(m->csr);
         k_run_sort_tile<VB><<<blocks_for(n), kRunTile, 0, st>>>(m->d_ctr, runs, csr, longs);
         k_run_sort_long<VB><<<uint32_t(std::min<uint64_t>((nlong + 7) / 8, 148 * 4)), 256, 0, st>>>(
             m->d_ctr, runs, csr, longs, giants);
@@ -1248,8 +1507,8 @@ int b2co_mmap_destroy(b2co_mmap* m)
     cudaFree(m->d_ctr);
     if (m->h_word) cudaFreeHost(m->h_word);
     if (m->h_ctr) cudaFreeHost(m->h_ctr);
-    cudaFree(m->d_regs);
-    if (m->h_regs) cudaFreeHost(m->h_regs);
+    cudaFree(m->d_survey);
+    if (m->h_survey) cudaFreeHost(m->h_survey);
     m->scratch.release();
     m->build.release();
     m->hist.release();

@@ -69,32 +69,41 @@ def fmix64_inverse(h):
     return np.array([int(v) for v in x], dtype=np.uint64).view(np.int64)
 
 
-@pytest.mark.parametrize("distinct,crowd", [(1500, 0), (1500, 300), (400_000, 0)])
-def test_table_sized_by_the_distinct_keys(distinct, crowd):
-    """Batches large enough for a table of the estimated number of keys; with `crowd` keys that all hash to one place,
-    so that the small table is given up for a full-size one."""
+@pytest.mark.parametrize("kb,vb", [(4, 4), (4, 8), (8, 4), (8, 8)])
+@pytest.mark.parametrize("distinct,crowd,heavy", [
+    (1500, 0, 0),        # too few keys for partitions of like size
+    (1500, 300, 0),      # and too many of them in one place of the small table
+    (400_000, 0, 0),     # by partitions
+    (400_000, 300, 0),   # one partition's part of the table cannot hold its keys
+    (400_000, 0, 1400),  # a key with a large share of its partition
+    (400_000, 0, 9000),  # a partition too large for one block
+    (1_000_000, 0, 0),
+])
+def test_batches_large_enough_to_be_surveyed(distinct, crowd, heavy, kb, vb):
     import b2co
     import torch
-    rng = np.random.default_rng(distinct + crowd)
+    if crowd and kb == 4:
+        pytest.skip("the crowded keys are made for the 64-bit hash")
+    rng = np.random.default_rng(distinct + crowd + heavy)
     n = (1 << 20) + 3
-    keys = np.unique(rng.integers(0, 2**62, size=distinct, dtype=np.int64))
+    ki, vi = np.iinfo(NP_DT[kb]), np.iinfo(NP_DT[vb])
+    keys = np.unique(rng.integers(0, ki.max // 2, size=distinct, dtype=NP_DT[kb]))
     if crowd:
-        keys = np.concatenate([keys, fmix64_inverse((np.arange(1, crowd + 1, dtype=np.uint64) << np.uint64(40)) + np.uint64(77))])
-    keys = keys[keys != -1]
-    at = np.concatenate([np.arange(len(keys)), rng.integers(0, len(keys), size=n - len(keys))])
-    v = rng.integers(0, 2**40, size=n, dtype=np.int64)
-    m = b2co.StaticMultimap(n, -1, -1, key_dtype=torch.int64, value_dtype=torch.int64)
+        keys = np.concatenate([keys, fmix64_inverse((np.uint64(77) << np.uint64(50)) + np.arange(crowd, dtype=np.uint64))])
+        keys = np.unique(keys[keys != -1])
+    at = np.concatenate([np.arange(len(keys)), np.full(heavy, 5), rng.integers(0, len(keys), size=n - len(keys) - heavy)])
+    at = rng.permutation(at)
+    v = rng.integers(0, vi.max, size=n, dtype=NP_DT[vb])
+    m = b2co.StaticMultimap(n, -1, -1, key_dtype=torch_dt(kb), value_dtype=torch_dt(vb))
     assert m.Insert(b2co.pack_pairs(dev(keys[at]), dev(v))) == 0
-    q = np.concatenate([keys, keys ^ np.int64(1 << 50)])
-    counts = np.bincount(at, minlength=len(keys))
-    total = int(counts.sum())
-    assert m.Count(dev(keys)) == total
-    ko = torch.zeros(total, dtype=torch.int64, device="cuda")
-    vo = torch.zeros(total, dtype=torch.int64, device="cuda")
-    assert m.Retrieve(dev(keys), ko, vo, total) == total
+    assert m.Count(dev(keys)) == n
+    ko = torch.zeros(n, dtype=torch_dt(kb), device="cuda")
+    vo = torch.zeros(n, dtype=torch_dt(vb), device="cuda")
+    assert m.Retrieve(dev(keys), ko, vo, n) == n
     order = np.lexsort((v, at))
     assert np.array_equal(ko.cpu().numpy(), keys[at[order]])
     assert np.array_equal(vo.cpu().numpy(), v[order])
+    q = np.concatenate([keys, keys ^ NP_DT[kb](ki.max // 2 + 1)])
     flags = torch.zeros(len(q), dtype=torch.uint8, device="cuda")
     m.Contains(dev(q), flags)
     assert np.array_equal(flags.cpu().numpy(), np.isin(q, keys).astype(np.uint8))
