@@ -30,6 +30,9 @@ int sm_count();
 // items per block, capped at the blocks that can be resident at once.
 uint32_t grid_for(void const* kernel, uint32_t block, uint64_t work, uint64_t per_block);
 
+// Whether the stream is being captured into a graph.
+bool capturing(cudaStream_t s);
+
 // Orders the uses of one piece of library-owned scratch (first-wins
 // InsertAndFind's, the routed Bloom Add's workspace) across the callers'
 // streams: a use waits on the GPU for the previous use to end, so async calls

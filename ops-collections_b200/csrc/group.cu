@@ -23,6 +23,9 @@
 
 using namespace b2co;
 
+constexpr uint32_t kDealers = 16;  // dealt launches of a group that may be in flight side by side; one more waits
+constexpr uint32_t kGroupWords = 2 + kDealers;
+
 struct b2co_oa_group {
     b2co_oa_desc desc{};
     GroupOps const* gops = nullptr;
@@ -33,9 +36,12 @@ struct b2co_oa_group {
     void* slab = nullptr;
     uint64_t total_slots = 0;
     GroupTable* d_tables = nullptr;
-    unsigned long long* d_counters = nullptr;  // [failed, status]
+    unsigned long long* d_counters = nullptr;  // [failed, status], then a chunk counter per dealt launch in flight
     unsigned long long* h_counters = nullptr;
     uint32_t find_shape = 1u | (1u << 8);  // lanes | keys per lane group << 8 | block << 16 (0 = 256)
+    std::mutex deal_mutex;
+    uint32_t next_dealer = 0;
+    ScratchOrder deal_order[kDealers];  // a chunk counter serves one launch at a time
     // one cached graph of the group Find launch
     cudaStream_t capture_stream = nullptr;
     cudaGraphExec_t graph = nullptr;
@@ -68,6 +74,7 @@ GroupArgs group_args(b2co_oa_group const* g, uint64_t const* d_offsets)
 {
     GroupArgs a;
     a.slots = g->slab;
+    a.deal = nullptr;
     a.tables = g->d_tables;
     a.offsets = d_offsets;
     a.count = g->count;
@@ -87,6 +94,22 @@ OaArgs table_args(b2co_oa_group const* g, uint32_t t)
     a.empty_value = g->desc.value_bytes ? g->desc.empty_value_bits : 0;
     a.erased_key = g->desc.empty_key_bits;
     return a;
+}
+
+// Large batches deal their chunks to the warps by a counter (group_kernels.cuh).
+// A captured launch does not: its graph may run beside other launches, whose
+// counters it does not know.
+template <class Launch>
+int dealt(b2co_oa_group* g, GroupArgs a, uint64_t n, cudaStream_t c, Launch launch)
+{
+    if (n < kGroupDealItems || capturing(c)) return launch(a);
+    std::lock_guard<std::mutex> lock(g->deal_mutex);
+    uint32_t const d = g->next_dealer++ % kDealers;
+    if (int st = g->deal_order[d].begin(c)) return st;
+    a.deal = reinterpret_cast<unsigned int*>(g->d_counters + 2 + d);
+    B2CO_CUDA(cudaMemsetAsync(a.deal, 0, sizeof(unsigned int), c));
+    if (int st = launch(a)) return st;
+    return g->deal_order[d].end(c);
 }
 
 int check(b2co_oa_group const* g)
@@ -232,9 +255,9 @@ int b2co_oa_group_create(b2co_oa_desc const* d, uint64_t const* requested, uint3
     B2CO_CUDA(cudaMalloc(&g->slab, (off * g->slot_bytes + 31) / 32 * 32));  // whole sectors (oa_sector.cuh)
     B2CO_CUDA(cudaMalloc(&g->d_tables, sizeof(GroupTable) * count));
     B2CO_CUDA(cudaMemcpy(g->d_tables, g->host_tables.data(), sizeof(GroupTable) * count, cudaMemcpyHostToDevice));
-    B2CO_CUDA(cudaMalloc(&g->d_counters, 2 * sizeof(unsigned long long)));
-    B2CO_CUDA(cudaMemset(g->d_counters, 0, 2 * sizeof(unsigned long long)));
-    B2CO_CUDA(cudaMallocHost(&g->h_counters, 2 * sizeof(unsigned long long)));
+    B2CO_CUDA(cudaMalloc(&g->d_counters, kGroupWords * sizeof(unsigned long long)));
+    B2CO_CUDA(cudaMemset(g->d_counters, 0, kGroupWords * sizeof(unsigned long long)));
+    B2CO_CUDA(cudaMallocHost(&g->h_counters, kGroupWords * sizeof(unsigned long long)));
     B2CO_CUDA(cudaStreamCreateWithFlags(&g->capture_stream, cudaStreamNonBlocking));
     if (int st = b2co_oa_group_clear(g, stream)) return st;
     *out = guard.release();
@@ -246,6 +269,7 @@ int b2co_oa_group_destroy(b2co_oa_group* g)
     if (!g) return B2CO_OK;
     if (g->graph) cudaGraphExecDestroy(g->graph);
     if (g->capture_stream) cudaStreamDestroy(g->capture_stream);
+    for (ScratchOrder& o : g->deal_order) o.release();
     if (g->slab) cudaFree(g->slab);
     if (g->d_tables) cudaFree(g->d_tables);
     if (g->d_counters) cudaFree(g->d_counters);
@@ -307,7 +331,9 @@ int b2co_oa_group_insert(b2co_oa_group* g, void const* pairs, uint64_t const* d_
     if (!d_offsets) return fail(B2CO_EINVAL, "offsets must not be null");
     cudaStream_t c = cs(s);
     if (failed) B2CO_CUDA(cudaMemsetAsync(g->d_counters, 0, sizeof(unsigned long long), c));
-    int st = g->gops->insert(group_args(g, d_offsets), g->desc.bucket_size, pairs, n, failed ? g->d_counters : nullptr, c);
+    int st = dealt(g, group_args(g, d_offsets), n, c, [&](GroupArgs const& a) {
+        return g->gops->insert(a, g->desc.bucket_size, pairs, n, failed ? g->d_counters : nullptr, c);
+    });
     if (st || !failed) return st;
     B2CO_CUDA(cudaMemcpyAsync(g->h_counters, g->d_counters, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c));
     B2CO_CUDA(cudaStreamSynchronize(c));
@@ -321,8 +347,9 @@ int b2co_oa_group_find(b2co_oa_group* g, void const* keys, uint64_t const* d_off
     if (int st = check(g)) return st;
     if (n == 0 || !keys || !out) return B2CO_OK;
     if (!d_offsets) return fail(B2CO_EINVAL, "offsets must not be null");
-    return g->gops->find(group_args(g, d_offsets), g->desc.bucket_size, g->find_shape, contains != 0, keys, out, n,
-                         cs(s));
+    return dealt(g, group_args(g, d_offsets), n, cs(s), [&](GroupArgs const& a) {
+        return g->gops->find(a, g->desc.bucket_size, g->find_shape, contains != 0, keys, out, n, cs(s));
+    });
 }
 
 // The same launch replayed from a CUDA graph captured on first use (and again

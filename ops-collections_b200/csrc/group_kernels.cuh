@@ -4,14 +4,18 @@
 //
 // One launch covers every table: the items of all tables are concatenated
 // (table t owns items [offsets[t], offsets[t+1])) and dealt to the warps in
-// chunks of at most 256 items, chunk c to warp c % warps, so work is balanced by
-// items, not by tables, and the chunks in flight at one time are neighbours:
-// the few tables they touch stay in L2, and the slab crosses HBM about once.
-// (One contiguous span per warp instead keeps the whole slab in play at once, so
-// that every window is a random HBM read.  4,096 tables of 280 M int32 pairs, a
-// 4.5 GB slab, 561 M lookups, with two lanes a window and two windows in flight:
-// Find 23.6 ms with spans, 11.8 with chunks.  With one lane a key reading whole
-// sectors, see below, 7.7 ms, and Insert 11.0 ms against 16.8 slot by slot.)
+// chunks of at most 512 items, so work is balanced by items, not by tables, and
+// the chunks in flight at one time are neighbours: the few tables they touch
+// stay in L2, and the slab crosses HBM about once.  (One contiguous span per warp
+// instead keeps the whole slab in play at once, so that every window is a random
+// HBM read.)  Over many rounds chunk c must not simply go to warp c % warps: warps
+// drift apart, and the tables in play grow past L2 with them.  Large batches deal
+// the chunks by a counter, the next one to whichever warp is free.
+// 4,096 tables of 280 M int32 pairs, a 4.8 GB slab, 561 M lookups, Insert and Find
+// in ms: spans and cooperative windows 16.0 and 23.6; chunks of 256 by warp number,
+// one lane a key (below) 11.0 and 7.7; by the counter 6.8 and 6.3 (7.6 and 7.4 GB
+// read).  Clear, Insert and Find together by chunk size: 64 items 22.4, 128 15.9,
+// 256 14.0, 512 13.8, 1,024 13.5, 2,048 15.8; 512 leaves room for wider slots.
 // The warp searches the table of a chunk's first item together and each lane
 // walks forward from there; the table's probe parameters stay in registers
 // while it does not change.  Per key the algorithms are exactly the
@@ -35,6 +39,26 @@ struct GroupArgs {
     uint32_t probing, hash;  // the same for every table
     uint64_t empty_key;
     uint64_t empty_value;
+    unsigned int* deal;  // chunks dealt after the first of every warp; null: chunk c goes to warp c % warps
+};
+
+__device__ __forceinline__ uint64_t group_warps() { return (uint64_t(gridDim.x) * blockDim.x) >> 5; }
+
+// The chunks of a warp, in ascending order.  The counter's answer is asked for a
+// chunk ahead.
+struct GroupDeal {
+    uint32_t ticket = 0;
+    __device__ __forceinline__ void take(GroupArgs const& g)
+    {
+        if (g.deal && (threadIdx.x & 31) == 0) ticket = atomicAdd(g.deal, 1u);
+    }
+    __device__ __forceinline__ uint64_t next(GroupArgs const& g, uint64_t begin, uint32_t chunk)
+    {
+        if (!g.deal) return begin + group_warps() * chunk;
+        uint64_t const c = group_warps() + __shfl_sync(0xffffffffu, ticket, 0);
+        take(g);
+        return c * chunk;
+    }
 };
 
 // The table of item i (the last t with offsets[t] <= i), searched by the whole
@@ -68,15 +92,29 @@ __device__ __forceinline__ OaArgs group_table_args(GroupArgs const& g, uint32_t 
     return a;
 }
 
+// A pair that is read once: first to leave L2.
+template <class T>
+__device__ __forceinline__ T ld_once(T const* p)
+{
+    return __ldcs(p);
+}
+__device__ __forceinline__ U128 ld_once(U128 const* p)
+{
+    ulonglong2 const v = __ldcs(reinterpret_cast<ulonglong2 const*>(p));
+    return U128{v.x, v.y};
+}
+
 // Items per chunk: a multiple of 32 (every kernel's pass divides it), small
 // enough that a small batch still reaches every warp.
-constexpr uint32_t kGroupChunk = 256;
+constexpr uint32_t kGroupChunk = 512;
+// Items of a batch whose chunks are dealt by the counter.  37 M items: 959 us with
+// and without; 280 M: 13.8 and 18.9 ms.
+constexpr uint64_t kGroupDealItems = 1ull << 25;
 inline uint32_t group_chunk(uint64_t n, uint64_t warps)
 {
     uint64_t const share = ((n + warps - 1) / warps + 31) / 32 * 32;
     return share < kGroupChunk ? uint32_t(share ? share : 32) : kGroupChunk;
 }
-__device__ __forceinline__ uint64_t group_warps() { return (uint64_t(gridDim.x) * blockDim.x) >> 5; }
 __device__ __forceinline__ uint64_t group_warp()
 {
     return (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -109,9 +147,11 @@ struct GroupCursor {
 // One lane per key, its window read as whole sectors (oa_sector.cuh); a key whose
 // window settles nothing is queued in the warp's shared-memory ring with its
 // table and followed a full pass at a time, one window each.  Bound by the L2
-// requests of the windows, as the single-table kernel: 73 Gkeys/s over the 4,096
-// tables above.  Asking L2 for the slab ahead of the chunks with bulk prefetches
-// was slower (10.0 ms).  Blocks of up to 256 threads.
+// requests of the windows, as the single-table kernel: 89 Gkeys/s over the 4,096
+// tables above.  Keys and results leave L2 first (18.7 against 19.2 ms for Clear,
+// Insert and Find).  Asking L2 for the slab ahead of the chunks with bulk prefetches
+// was slower (10.0 against 7.7 ms).  Five blocks an SM: 15.5 against 14.0 ms for
+// all three.  Blocks of up to 256 threads.
 template <class S, int B, bool CONTAINS>
 __global__ void __launch_bounds__(256, 4) k_group_find_lane(__grid_constant__ const GroupArgs g, void const* keys,
                                                             void* out, uint64_t n, uint32_t chunk)
@@ -123,7 +163,8 @@ __global__ void __launch_bounds__(256, 4) k_group_find_lane(__grid_constant__ co
     __shared__ uint32_t qtab[8][kSectorRing], qinit[8][kSectorRing], qidx[8][kSectorRing];
 
     uint32_t const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint64_t const stride = group_warps() * chunk;
+    GroupDeal deal;
+    deal.take(g);
     uint64_t begin = group_warp() * chunk, at = begin, end = begin + chunk < n ? begin + chunk : n;
     Key const* const kin = static_cast<Key const*>(keys);
     uint64_t const empty = S::is_set ? g.empty_key : g.empty_value;
@@ -131,13 +172,13 @@ __global__ void __launch_bounds__(256, 4) k_group_find_lane(__grid_constant__ co
 
     auto store = [&](uint64_t pos, bool hit, uint64_t payload) {
         if constexpr (CONTAINS) reinterpret_cast<uint8_t*>(out)[pos] = hit;
-        else reinterpret_cast<typename Io<S>::Payload*>(out)[pos] = typename Io<S>::Payload(hit ? payload : empty);
+        else __stcs(reinterpret_cast<typename Io<S>::Payload*>(out) + pos, typename Io<S>::Payload(hit ? payload : empty));
     };
     GroupCursor<S, B> cur;
     uint64_t next_key = 0;
     if (begin < n) {
         cur.start(g, begin);
-        next_key = at + lane < end ? uint64_t(__ldg(kin + at + lane)) : 0;
+        next_key = at + lane < end ? uint64_t(__ldcs(kin + at + lane)) : 0;
     }
     for (;;) {
         uint64_t key, pos;
@@ -175,12 +216,12 @@ __global__ void __launch_bounds__(256, 4) k_group_find_lane(__grid_constant__ co
             init = idx = probe_init<S::key_bytes, B>(cur.a.probe, key);
             at += 32;
             if (at >= end) {  // the next chunk
-                begin += stride;
+                begin = deal.next(g, begin, chunk);
                 at = begin;
                 end = begin + chunk < n ? begin + chunk : n;
                 if (begin < n) cur.start(g, begin);
             }
-            next_key = begin < n && at + lane < end ? uint64_t(__ldg(kin + at + lane)) : 0;
+            next_key = begin < n && at + lane < end ? uint64_t(__ldcs(kin + at + lane)) : 0;
         }
         bool open = false;
         if (live) {
@@ -399,7 +440,8 @@ __global__ void __launch_bounds__(256, 4) k_group_insert(__grid_constant__ const
     __shared__ uint32_t qtab[8][kSectorRing], qinit[8][kSectorRing], qidx[8][kSectorRing];
 
     uint32_t const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint64_t const stride = group_warps() * chunk;
+    GroupDeal deal;
+    deal.take(g);
     uint64_t begin = group_warp() * chunk, at = begin, end = begin + chunk < n ? begin + chunk : n;
     Raw const* const pin = static_cast<Raw const*>(pairs);
     uint32_t head = 0, count = 0, failed = 0;
@@ -407,7 +449,7 @@ __global__ void __launch_bounds__(256, 4) k_group_insert(__grid_constant__ const
     Raw next_pair{};
     if (begin < n) {
         cur.start(g, begin);
-        if (at + lane < end) next_pair = ld_ro(pin + at + lane);
+        if (at + lane < end) next_pair = ld_once(pin + at + lane);
     }
     for (;;) {
         Raw pr;
@@ -447,12 +489,12 @@ __global__ void __launch_bounds__(256, 4) k_group_insert(__grid_constant__ const
             }
             at += 32;
             if (at >= end) {
-                begin += stride;
+                begin = deal.next(g, begin, chunk);
                 at = begin;
                 end = begin + chunk < n ? begin + chunk : n;
                 if (begin < n) cur.start(g, begin);
             }
-            if (begin < n && at + lane < end) next_pair = ld_ro(pin + at + lane);
+            if (begin < n && at + lane < end) next_pair = ld_once(pin + at + lane);
         }
         int verdict = kOpen;
         if (live) {

@@ -25,7 +25,6 @@ int cuda_fail(cudaError_t e, char const* what)
                 std::string(what) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")");
 }
 
-namespace {
 bool capturing(cudaStream_t s)
 {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
@@ -35,7 +34,6 @@ bool capturing(cudaStream_t s)
     }
     return st != cudaStreamCaptureStatusNone;
 }
-}  // namespace
 
 int ScratchOrder::begin(cudaStream_t s)
 {
