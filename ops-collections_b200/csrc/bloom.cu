@@ -646,14 +646,13 @@ constexpr uint64_t kPartitionFilterBytes = uint64_t(64) << 20;
 // Keys per route-and-apply round.  A batch that passes it by less than an eighth
 // stays one round: a round costs about 100 us however few its keys.
 constexpr uint64_t kPartitionRound = uint64_t(1) << 27;
+constexpr uint64_t kMinPartitionRound = uint64_t(1) << 20;
 
 template <int KB>
 int launch_add_partitioned(b2co_bloom* f, void const* keys, uint8_t const* stencil, uint64_t n, cudaStream_t s)
 {
     uint32_t const nblocks = uint32_t(f->num_blocks);
     uint32_t const nslices = (nblocks + kSliceBlocks - 1) / kSliceBlocks;
-    uint64_t const rounds = (n + kPartitionRound / 8 * 9 - 1) / (kPartitionRound / 8 * 9);
-    uint64_t const round = (n + rounds - 1) / rounds;
     auto const route = k_bloom_route<KB>;
     size_t const apply_smem = size_t(kSliceBlocks) * 32;
     size_t const rsmem = route_smem(nslices);
@@ -662,17 +661,26 @@ int launch_add_partitioned(b2co_bloom* f, void const* keys, uint8_t const* stenc
                                    int(apply_smem)));
     int per_sm = 0;
     B2CO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (void const*)route, kRouteThreads, rsmem));
-    uint64_t const tiles = (round + kRouteTile - 1) / kRouteTile;
     uint32_t const route_cap = uint32_t(per_sm < 1 ? 1 : per_sm) * uint32_t(sm_count());
-    uint32_t const nctas = uint32_t(tiles < route_cap ? tiles : route_cap);
-    uint32_t const segment = route_segment(round, nctas, nslices);
-    uint64_t const want = uint64_t(nslices) * nctas * segment;
-    if (f->recs_cap < want) {
+    uint64_t rounds = (n + kPartitionRound / 8 * 9 - 1) / (kPartitionRound / 8 * 9), round = 0;
+    uint32_t nctas = 0, segment = 0;
+    for (;; rounds *= 2) {  // shorter rounds where there is no room for the records of the longest
+        round = (n + rounds - 1) / rounds;
+        uint64_t const tiles = (round + kRouteTile - 1) / kRouteTile;
+        nctas = uint32_t(tiles < route_cap ? tiles : route_cap);
+        segment = route_segment(round, nctas, nslices);
+        uint64_t const want = uint64_t(nslices) * nctas * segment;
+        if (f->recs_cap >= want) break;
         if (f->recs) cudaFree(f->recs);
         f->recs = nullptr;
         f->recs_cap = 0;
-        B2CO_CUDA(cudaMalloc(&f->recs, want * 8));
-        f->recs_cap = want;
+        cudaError_t const e = cudaMalloc(&f->recs, want * 8);
+        if (e == cudaSuccess) {
+            f->recs_cap = want;
+            break;
+        }
+        if (e != cudaErrorMemoryAllocation || round <= kMinPartitionRound) return cuda_fail(e, "BloomFilter::Add workspace");
+        cudaGetLastError();
     }
     size_t const part_words = size_t(route_cap) * kMaxSlices;
     if (f->part_words < part_words) {
