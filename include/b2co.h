@@ -231,10 +231,11 @@ int b2co_oa_find_host(b2co_oa_table* table, const void* host_keys, void* host_ou
  * 8) and keys in flight per lane group (1, 2 or 4), optionally OR-ed with
  * B2CO_FIND_SEGMENTED (scan each first bucket window by 64-byte segments and
  * read the second segment only when the first does not end the scan) and the
- * flags below; 0, 0 = library default (4 lanes, 2 windows, B2CO_FIND_DEFERRED;
- * 2 lanes, 1 window for 4-byte slots and for tables of at most 320 MiB, which
- * are served mostly from L2).  No reference counterpart (the reference
- * launches one thread per key). */
+ * flags below; 0, 0 = library default, chosen by table size and batch: one lane
+ * a key for tables of at most 224 MiB (served mostly from L2) with 8- or 16-byte
+ * slots and for batches of at most 98,304 keys; else 2 lanes and 1 window up to
+ * 320 MiB and for 4-byte slots, 4 lanes and 2 windows above, both
+ * B2CO_FIND_DEFERRED.  No reference counterpart. */
 #define B2CO_FIND_SEGMENTED 0x100u
 /* OR-ed into keys_per_lane: fetch every first bucket window with one bulk (TMA)
  * copy into shared memory; tables with 16-byte slots only (others ignore it). */
@@ -247,13 +248,12 @@ int b2co_oa_find_host(b2co_oa_table* table, const void* host_keys, void* host_ou
 int b2co_oa_set_find_shape(b2co_oa_table* table, uint32_t lanes_per_key, uint32_t keys_per_lane);
 /* Kernel shape of the insert family (Insert, InsertIf, InsertOrAssign,
  * InsertAndFind) for this table (no reference counterpart; results do not
- * depend on it).  lanes_per_key 1 runs one lane per key (the reference's scan
- * as written); 2, 4 or 8 lanes share each bucket window with keys_per_tile
- * (1, 2 or 4) keys in flight per lane group.  (0, 0) restores the default:
- * 4 lanes, 1 key (one lane per key for bucket size 1 and for tables of at
- * most 320 MiB, whose windows mostly come from L2).  Layouts with 2-byte
- * or floating-point keys run the default window shape for any request other
- * than one lane per key. */
+ * depend on it).  lanes_per_key 1 reads a key's window with one lane; 2, 4 or 8
+ * read it with a tile of lanes, as many as the window has 32-byte sectors
+ * (keys_per_tile, 1, 2 or 4, is accepted and changes nothing).  (0, 0)
+ * restores the default: one lane for bucket size 1 and for tables of at most
+ * 352 MiB (InsertOrAssign: 256 MiB), whose windows mostly come from L2, a tile
+ * above. */
 int b2co_oa_set_write_shape(b2co_oa_table* table, uint32_t lanes_per_key, uint32_t keys_per_tile);
 
 /* ===================================================================== */
@@ -295,7 +295,7 @@ int b2co_oa_group_insert_per_table(b2co_oa_group* group, const void* pairs, cons
  * keys in flight per lane group (1, 2 or 4, at most the lanes; above 1 the
  * keys whose first window settles nothing are queued and followed a pass at a
  * time) and threads per block (64, 128 or 256; 0 = 256).  Results do not
- * depend on it.  The default is 4 lanes, 2 keys, 256 threads.  The lanes-only
+ * depend on it.  The default is 1 lane, 1 key, 256 threads.  The lanes-only
  * form sets one key per lane group. */
 int b2co_oa_group_set_find_shape(b2co_oa_group* group, uint32_t lanes);
 int b2co_oa_group_set_find_shape_ex(b2co_oa_group* group, uint32_t lanes, uint32_t keys_per_tile, uint32_t block);
@@ -560,7 +560,8 @@ int b2co_bloom_add(b2co_bloom* filter, const void* keys, uint64_t n, b2co_stream
  * four 64-bit atomic ORs per key from the SM.  B2CO_BLOOM_ADD_BULK: one
  * 32-byte TMA bulk reduction (OR) per key from shared memory.
  * B2CO_BLOOM_ADD_PARTITIONED: keys are routed by 128 KiB filter slice into a
- * record workspace (8 bytes per key, at most 2^27 keys per round, allocated on
+ * record workspace (8 bytes per key and room for uneven shares, about a fifth
+ * more for large batches; at most 2^27 keys and an eighth per round, allocated on
  * first use and kept with the filter), then each slice is built in shared
  * memory and ORed into the filter; filters above 2048 slices (256 MiB) use BULK.
  * B2CO_BLOOM_ADD_AUTO (the default): PARTITIONED for filters of at least 64 MiB
