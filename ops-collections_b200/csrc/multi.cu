@@ -22,7 +22,7 @@
 // where sorting all (value, key) records together takes one pass over memory per
 // byte of both (16.8 M int64 pairs over 4.2 M keys: twelve passes, 4.9 ms, against 125 us
 // for sorting the runs).  The pairs of large batches are grouped partition by
-// partition (565 us for those pairs: survey 55, route 274, build 225), others in a
+// partition (475 us for those pairs: survey 55, route 187, build 225), others in a
 // table that all blocks share (1,700 us).
 #include <algorithm>
 #include <cmath>
@@ -457,30 +457,45 @@ __global__ void __launch_bounds__(kThreads) k_part_starts(Survey* s, uint32_t pa
 }
 
 // The pairs of a partition come to lie together, in any order: a block ranks a
-// tile's pairs in their partitions in shared memory, takes the tile's places with
-// one atomic a partition and stores every pair to its place.  The stores of the
-// blocks at work meet in L2 (a partition grows at one end), which puts sectors
-// together, so the pairs need no sorting on the way: 16.8 M pairs of 16 bytes are read
-// and written once, 0.58 GB in 274 us.  Bound by the block's phases, which wait
-// on one another (a load, an atomic in shared memory and one in L2, a store).
+// tile's pairs in their partitions in shared memory, sorts the tile by partition
+// there, takes the tile's places with one atomic a partition and writes run
+// after run, so that the pairs of a run leave in whole sectors.  Bound by the
+// block's phases, which wait on one another: 16.8 M pairs of 16 bytes over 4,096
+// partitions, 0.49 GB in 187 us.  Storing every pair to its place without the sort:
+// 274 us (scattered stores run at about 60 G a second).
 constexpr int kRouteThreads = 1024, kRoutePer = 8;
+constexpr uint32_t kRouteTile = kRouteThreads * kRoutePer;
+template <class Raw>
+constexpr size_t kRouteSmem = size_t(kRouteTile) * (sizeof(Raw) + 4) + kMaxParts * 4 * 2;
+
 template <int KB, int VB>
 __global__ void __launch_bounds__(kRouteThreads, 1)
     k_part_route(typename SlotT<KB, VB>::Raw const* dense, uint64_t n, uint32_t pbits, Survey* survey,
                  typename SlotT<KB, VB>::Raw* out)
 {
     using S = SlotT<KB, VB>;
-    __shared__ uint32_t at[kMaxParts];
-    uint32_t const parts = 1u << pbits;
-    constexpr uint64_t kTileOf = uint64_t(kRouteThreads) * kRoutePer;
-    for (uint64_t base = uint64_t(blockIdx.x) * kTileOf; base < n; base += uint64_t(gridDim.x) * kTileOf) {
-        for (uint32_t p = threadIdx.x; p < parts; p += kRouteThreads) at[p] = 0;
-        typename S::Raw pr[kRoutePer];
+    using Raw = typename S::Raw;
+    constexpr int kWarps = kRouteThreads / 32, kPer = kMaxParts / kRouteThreads;
+    extern __shared__ __align__(16) unsigned char route_smem[];
+    Raw* const stage = reinterpret_cast<Raw*>(route_smem);
+    uint32_t* const stage_at = reinterpret_cast<uint32_t*>(stage + kRouteTile);
+    uint32_t* const first = stage_at + kRouteTile;  // a partition's count, then where its run starts in the tile
+    uint32_t* const delta = first + kMaxParts;      // its place in `out`, less that
+    __shared__ uint32_t warp_tot[kWarps];
+    uint32_t const parts = 1u << pbits, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t const stride = uint64_t(gridDim.x) * kRouteTile;
+    Raw pr[kRoutePer];
+    auto load = [&](uint64_t base) {
 #pragma unroll
         for (int r = 0; r < kRoutePer; ++r) {
             uint64_t const i = base + uint64_t(r) * kRouteThreads + threadIdx.x;
             if (i < n) pr[r] = ld_ro(dense + i);
         }
+    };
+    load(uint64_t(blockIdx.x) * kRouteTile);
+    for (uint64_t base = uint64_t(blockIdx.x) * kRouteTile; base < n; base += stride) {
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) first[threadIdx.x * kPer + q] = 0;
         __syncthreads();
         uint32_t place[kRoutePer];  // partition | rank in the tile's share of it
 #pragma unroll
@@ -488,20 +503,54 @@ __global__ void __launch_bounds__(kRouteThreads, 1)
             uint64_t const i = base + uint64_t(r) * kRouteThreads + threadIdx.x;
             if (i < n) {
                 uint32_t const p = uint32_t(run_hash<KB>(KeyWord<KB>(S::key(pr[r]))) >> (64 - pbits));
-                place[r] = p | (atomicAdd(at + p, 1u) << kMaxPartBits);
+                place[r] = p | (atomicAdd(first + p, 1u) << kMaxPartBits);
             }
         }
         __syncthreads();
-        for (uint32_t p = threadIdx.x; p < parts; p += kRouteThreads) {
-            uint32_t const c = at[p];
-            if (c) at[p] = atomicAdd(survey->cursors + p, c);
+        uint32_t c[kPer], at[kPer], sum = 0;
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            uint32_t const p = threadIdx.x * kPer + q;
+            c[q] = first[p];
+            at[q] = c[q] && p < parts ? atomicAdd(survey->cursors + p, c[q]) : 0u;
+            sum += c[q];
+        }
+        uint32_t incl = sum;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            uint32_t const o = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= uint32_t(d)) incl += o;
+        }
+        if (lane == 31) warp_tot[warp] = incl;
+        __syncthreads();
+        uint32_t run = warp_tot[lane];  // every warp scans the warps' sums for itself
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            uint32_t const o = __shfl_up_sync(0xffffffffu, run, d);
+            if (lane >= uint32_t(d)) run += o;
+        }
+        uint32_t const before = __shfl_sync(0xffffffffu, run, warp ? warp - 1 : 0);
+        run = (warp ? before : 0u) + incl - sum;
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            first[threadIdx.x * kPer + q] = run;
+            delta[threadIdx.x * kPer + q] = at[q] - run;
+            run += c[q];
         }
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < kRoutePer; ++r) {
             uint64_t const i = base + uint64_t(r) * kRouteThreads + threadIdx.x;
-            if (i < n) out[at[place[r] & (kMaxParts - 1)] + (place[r] >> kMaxPartBits)] = pr[r];
+            if (i < n) {
+                uint32_t const p = place[r] & (kMaxParts - 1), to = first[p] + (place[r] >> kMaxPartBits);
+                stage[to] = pr[r];
+                stage_at[to] = to + delta[p];
+            }
         }
+        load(base + stride);  // the next tile, while this one leaves
+        __syncthreads();
+        uint32_t const total = n - base < kRouteTile ? uint32_t(n - base) : kRouteTile;
+        for (uint32_t i = threadIdx.x; i < total; i += kRouteThreads) out[stage_at[i]] = stage[i];
         __syncthreads();
     }
 }
@@ -1083,9 +1132,9 @@ constexpr uint64_t kMaxRegionBytes = 200 << 10;  // of shared memory
 // and no partition is over four times as large as they are on average (one block
 // would be at work on it long after the others).  Whole builds, shared table and
 // partitions, in us, n pairs over n / 4 and n / 256 int64 keys: n = 2^20: 174, 165 and 248, 243;
-// 2^22: 361, 270 and 586, 554; 2^24: 1,907, 750 and 1,959, 1,736; 2^26: 10,260, 3,600 and 8,710, 6,796.
-// 2,048 partitions against 4,096, over n / 4 keys: 2^22: 270 and 284; 2^24: 760 and 750 (over n: 964 and
-// 878); 2^26: only the smaller ones fit.
+// 2^22: 361, 273 and 586, 554; 2^24: 1,907, 655 and 1,959, 1,736; 2^26: 10,260, 2,759 and 8,710, 6,796.
+// 2,048 partitions against 4,096, over n / 4 keys: 2^22: 273 and 284; 2^24: 655 and 654 (over n: 865 and
+// 797); 2^25: 1,386 and 1,233; 2^26: only the smaller ones fit.
 template <int KB, int VB>
 int mmap_plan(b2co_mmap* m, cudaStream_t st, uint64_t* tsize, uint32_t* part_bits)
 {
@@ -1127,10 +1176,11 @@ int mmap_group_parts(b2co_mmap* m, cudaStream_t st, uint32_t pbits, void* pairs,
     auto* const build = k_part_build<KB, VB>;
     B2CO_CUDA(cudaFuncSetAttribute((void const*)build, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     k_part_starts<<<1, kThreads, 0, st>>>(m->d_survey, parts);
-    constexpr uint64_t kTileOf = uint64_t(kRouteThreads) * kRoutePer;
-    k_part_route<KB, VB>
-        <<<uint32_t(std::min<uint64_t>((m->size + kTileOf - 1) / kTileOf, uint64_t(sm_count()))), kRouteThreads, 0, st>>>(
-            static_cast<Raw const*>(m->dense), m->size, pbits, m->d_survey, static_cast<Raw*>(pairs));
+    auto* const route = k_part_route<KB, VB>;
+    B2CO_CUDA(cudaFuncSetAttribute((void const*)route, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kRouteSmem<Raw>)));
+    uint64_t const tiles = (m->size + kRouteTile - 1) / kRouteTile;
+    route<<<uint32_t(std::min<uint64_t>(tiles, uint64_t(sm_count()))), kRouteThreads, kRouteSmem<Raw>, st>>>(
+        static_cast<Raw const*>(m->dense), m->size, pbits, m->d_survey, static_cast<Raw*>(pairs));
     build<<<parts, kPartThreads, smem, st>>>(m->table<KB>(), static_cast<Raw const*>(pairs), m->d_survey, m->d_ctr, runs,
                                              static_cast<ValueWord<VB>*>(m->csr));
     B2CO_CUDA(cudaGetLastError());
