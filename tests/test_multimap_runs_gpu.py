@@ -93,7 +93,8 @@ def test_batches_large_enough_to_be_surveyed(distinct, crowd, heavy, kb, vb):
         keys = np.unique(keys[keys != -1])
     at = np.concatenate([np.arange(len(keys)), np.full(heavy, 5), rng.integers(0, len(keys), size=n - len(keys) - heavy)])
     at = rng.permutation(at)
-    v = rng.integers(0, vi.max, size=n, dtype=NP_DT[vb])
+    v = rng.integers(vi.min + 1, vi.max, size=n, dtype=NP_DT[vb])
+    v[v == -1] = 0
     m = b2co.StaticMultimap(n, -1, -1, key_dtype=torch_dt(kb), value_dtype=torch_dt(vb))
     assert m.Insert(b2co.pack_pairs(dev(keys[at]), dev(v))) == 0
     assert m.Count(dev(keys)) == n
