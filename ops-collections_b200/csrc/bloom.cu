@@ -637,10 +637,12 @@ int launch_contains_policy(b2co_bloom* f, void const* keys, uint8_t const* stenc
 
 // B2CO_BLOOM_ADD_AUTO takes the partitioned Add for filters of at least
 // kPartitionFilterBytes with batches of at least kPartitionKeysPerBlock keys per
-// filter block.  Measured: on a 128 MiB filter routing ties the bulk ORs at 4
-// keys per block (402 vs 412 us) and wins from 8 on (654 vs 842 us); a 2 MiB
-// filter stays in L2, where the bulk ORs win at every batch size (25 vs 94 us
-// at 16 keys per block) and routing's fixed cost of about 45 us dominates.
+// filter block.  Bulk ORs and routing in us at 4, 8 and 16 keys per block: 2 MiB filter
+// 10 and 38, 15 and 46, 23 and 62; 32 MiB: 76 and 89, 141 and 132, 270 and 222; 64 MiB: 148 and
+// 163, 279 and 257, 537 and 443; 128 MiB: 418 and 304, 842 and 505, 1,607 and 898; 256 MiB: 1,210 and
+// 671, 2,396 and 1,140, 4,772 and 2,096.  Filters past L2 would gain from 3 keys per block
+// on, but routing needs a workspace, which the first call allocates and a stream
+// capture cannot, so smaller batches stay without one.
 constexpr uint64_t kPartitionKeysPerBlock = 8;
 constexpr uint64_t kPartitionFilterBytes = uint64_t(64) << 20;
 // Keys per route-and-apply round.  A batch that passes it by less than an eighth
