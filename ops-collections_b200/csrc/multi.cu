@@ -30,6 +30,7 @@
 #include <new>
 
 #include "multi_common.cuh"
+#include "run_probe.h"
 
 using namespace b2co;
 using namespace b2co::multi;
@@ -256,17 +257,19 @@ struct alignas(16) RunSlot {
 
 // A key's probing starts at the leading bits of its hash and goes round the
 // region (a power of two of slots) that it starts in: the whole table, or the
-// part of it that one block builds in shared memory.
+// part of it that one block builds in shared memory.  A table of full size is at
+// most half full; one that was sized by an estimate, and every region that a
+// block built, at most three quarters (region_crowded).
 template <int KB>
 struct RunTable {
     RunSlot<KB>* slots;
-    uint64_t mask;    // table size - 1 (a power of two); at most half full
+    uint64_t mask;    // table size - 1 (a power of two)
     uint64_t region;  // region size - 1
     uint32_t shift;   // 64 - log2(table size)
     KeyWord<KB> empty;
 
     __device__ __forceinline__ uint64_t start(KeyWord<KB> k) const { return run_hash<KB>(k) >> shift; }
-    __device__ __forceinline__ uint64_t next(uint64_t s) const { return (s & ~region) | ((s + 1) & region); }
+    __device__ __forceinline__ uint64_t next(uint64_t s) const { return next_in_region(s, region); }
 };
 
 template <int KB>
@@ -277,22 +280,21 @@ __device__ __forceinline__ RunSlot<KB> load_run(RunSlot<KB> const* p)
     else return RunSlot<KB>{v.x, v.y, v.z};
 }
 
-// The key's slot contents; false (and count 0) when absent.
+// The key's slot contents; false (and count 0) when absent.  Bounded by the
+// region, whatever the table holds.
 template <int KB>
 __device__ __forceinline__ bool find_run(RunTable<KB> const& t, KeyWord<KB> k, RunSlot<KB>& out)
 {
     out.count = 0;
     if (k == t.empty) return false;
-    uint64_t s = t.start(k);
-    for (;;) {
+    return walk_region(t.start(k), t.region, [&](uint64_t s) {
         RunSlot<KB> const cur = load_run<KB>(t.slots + s);
         if (cur.key == k) {
             out = cur;
-            return true;
+            return int(kProbeHit);
         }
-        if (cur.key == t.empty) return false;
-        s = t.next(s);
-    }
+        return int(cur.key == t.empty ? kProbeMiss : kProbeOn);
+    });
 }
 
 template <int KB>
@@ -623,6 +625,7 @@ __global__ void __launch_bounds__(kPartThreads)
         unsigned long long total = 0;
         for (int w = 0; w < kWarps; ++w) total += warp_at[w];
         unsigned long long at = total ? atomicAdd(&ctr->cursor, total) : 0;
+        if (region_crowded(total >> 32, slots)) ctr->crowded = 1;
         for (int w = 0; w < kWarps; ++w) {
             unsigned long long const v = warp_at[w];
             warp_at[w] = at;
@@ -1250,6 +1253,8 @@ int mmap_build(b2co_mmap* m, cudaStream_t st)
         B2CO_CUDA(cudaMemcpyAsync(m->h_ctr, m->d_ctr, sizeof(RunCounters), cudaMemcpyDeviceToHost, st));
         B2CO_CUDA(cudaStreamSynchronize(st));
         if (m->h_ctr->crowded) continue;
+        // a table of full size holds every key that there can be; a smaller one may have been filled up
+        if (tsize != full && region_crowded(m->h_ctr->cursor >> 32, tsize)) continue;
         if (m->h_ctr->ngiant) {
             if (int e = mmap_sort_giants<VB>(m, runs, giants, m->h_ctr->ngiant, m->h_ctr->giant_values, st)) return e;
             B2CO_CUDA(cudaStreamSynchronize(st));
