@@ -8,7 +8,6 @@
 #include <cstring>
 #include <mutex>
 #include <new>
-#include <vector>
 
 #include "b2co_host.h"
 #include "oa_kernels.cuh"
@@ -54,17 +53,29 @@ uint32_t oa_slot_bytes(uint32_t kb, uint32_t vb)
 // Staging slots (and pipeline streams) of the host-buffer Find.
 constexpr int kHostSlots = 3;
 
+// Counters of one synchronous insert call, and the lists they are on.
+struct CounterSet {
+    Counters c{};
+    CounterSet* next_idle = nullptr;
+    CounterSet* next = nullptr;
+};
+constexpr int kCounterSets = 4;  // made with the table: calls on one table side by side that allocate nothing
+constexpr int kSumWords = kCounterWords + 1;
+constexpr int kDeviceWords = 1 + kCounterSets * kSumWords, kHostWords = 2 + kCounterSets * kCounterWords;
+
 struct b2co_oa_table {
     b2co_oa_desc desc{};
     OaArgs args{};
     OaOps const* ops = nullptr;
     uint64_t capacity = 0;
     int device = 0;
-    unsigned long long* d_counters = nullptr;  // [keys not erased / keys counted]
-    unsigned long long* h_counters = nullptr;  // pinned: its mirror, then the status word that kernels write
+    unsigned long long* d_counters = nullptr;  // [keys not erased / keys counted], then the sums of `sets`
+    unsigned long long* h_counters = nullptr;  // pinned: its mirror, the status word that kernels write, then the host
+                                               // words of `sets`
     std::mutex counters_mu;
-    std::vector<Counters> counters;       // of synchronous insert calls; one per call at a time
-    std::vector<Counters> idle_counters;
+    CounterSet sets[kCounterSets];     // of synchronous insert calls; one per call at a time
+    CounterSet* idle = nullptr;        // those in nobody's hands
+    CounterSet* more = nullptr;        // made for calls beyond them, kept
     // first-wins InsertAndFind scratch, grown on demand
     uint32_t* d_pos = nullptr;
     uint64_t pos_cap = 0;
@@ -123,33 +134,42 @@ int check_status(b2co_oa_table* t, cudaStream_t s)
 }
 
 // Counters for one synchronous insert call (concurrent calls on a table each
-// take their own); release() returns them.
-int take_counters(b2co_oa_table* t, Counters& c)
+// take their own); give_counters returns them.  The first few were made with the
+// table.  More callers than those make their own: another thread's stream
+// capture is not disturbed, and the words are cleared on the caller's stream.
+int take_counters(b2co_oa_table* t, CounterSet*& set, cudaStream_t s)
 {
     std::lock_guard<std::mutex> g(t->counters_mu);
-    if (!t->idle_counters.empty()) {
-        c = t->idle_counters.back();
-        t->idle_counters.pop_back();
+    if (t->idle) {
+        set = t->idle;
+        t->idle = set->next_idle;
         return B2CO_OK;
     }
-    c = Counters{};
-    cudaError_t e = cudaMalloc(&c.sum, (kCounterWords + 1) * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMemset(c.sum, 0, (kCounterWords + 1) * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // zero before any stream of the caller's uses it
-    if (e == cudaSuccess) e = cudaMallocHost(&c.host, kCounterWords * sizeof(unsigned long long));
+    auto* n = new (std::nothrow) CounterSet;
+    if (!n) return fail(B2CO_ENOMEM, "host allocation failed");
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    cudaError_t e = cudaMalloc(&n->c.sum, kSumWords * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMallocHost(&n->c.host, kCounterWords * sizeof(unsigned long long));
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e == cudaSuccess) e = cudaMemsetAsync(n->c.sum, 0, kSumWords * sizeof(unsigned long long), s);
     if (e != cudaSuccess) {
-        if (c.sum) cudaFree(c.sum);
+        if (n->c.sum) cudaFree(n->c.sum);
+        if (n->c.host) cudaFreeHost(n->c.host);
+        delete n;
         return cuda_fail(e, "insert counters");
     }
-    t->counters.push_back(c);
-    t->idle_counters.reserve(t->counters.size());  // giving one back never allocates
+    n->next = t->more;
+    t->more = n;
+    set = n;
     return B2CO_OK;
 }
 
-void give_counters(b2co_oa_table* t, Counters const& c)
+void give_counters(b2co_oa_table* t, CounterSet* set)
 {
     std::lock_guard<std::mutex> g(t->counters_mu);
-    t->idle_counters.push_back(c);
+    set->next_idle = t->idle;
+    t->idle = set;
 }
 
 int sync_counters(b2co_oa_table* t, cudaStream_t s, int words)
@@ -215,15 +235,15 @@ int b2co_oa_launch_insert(b2co_oa_table* t, void const* pairs, uint64_t n, bool 
 int b2co_oa_insert_counted(b2co_oa_table* t, void const* pairs, uint8_t const* stencil, uint64_t n, bool assign,
                            cudaStream_t s, uint64_t* counts)
 {
-    Counters c;
-    if (int st = take_counters(t, c)) return st;
-    int st = t->ops->insert(t->args, t->desc.bucket_size, pairs, stencil, uint32_t(n), assign, c, s);
+    CounterSet* set = nullptr;
+    if (int st = take_counters(t, set, s)) return st;
+    int st = t->ops->insert(t->args, t->desc.bucket_size, pairs, stencil, uint32_t(n), assign, set->c, s);
     if (!st) {
         cudaError_t const e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) st = cuda_fail(e, "cudaStreamSynchronize");
     }
-    for (int i = 0; i < kCounterWords; ++i) counts[i] = st ? 0 : static_cast<unsigned long long volatile*>(c.host)[i];
-    give_counters(t, c);
+    for (int i = 0; i < kCounterWords; ++i) counts[i] = st ? 0 : static_cast<unsigned long long volatile*>(set->c.host)[i];
+    give_counters(t, set);
     return st;
 }
 
@@ -250,10 +270,11 @@ int b2co_oa_lookup_over(b2co_oa_table* t, bool contains, void const* keys, void*
                         wait_ctl(status_word(t)), s);
 }
 
-// Device bytes a table holds (slots and counters).
+// Device bytes that an admission by budget counts for a table: its slots and 24
+// for its counters (which share one of the allocator's smallest pieces).
 uint64_t b2co_oa_table_bytes(b2co_oa_table const* t)
 {
-    return t ? t->capacity * slot_bytes(t->desc.key_bytes, t->desc.value_bytes) + sizeof(unsigned long long) : 0;
+    return t ? t->capacity * slot_bytes(t->desc.key_bytes, t->desc.value_bytes) + 3 * sizeof(unsigned long long) : 0;
 }
 
 // Key / payload / pair sizes of a table.
@@ -314,12 +335,18 @@ int b2co_oa_create_ex(b2co_oa_desc const* d, uint64_t requested, bool clear, b2c
 
     // whole 32-byte sectors: kernels read the sectors that a window covers
     cudaError_t e = cudaMalloc(&t->args.slots, (cap * slot_bytes(d->key_bytes, d->value_bytes) + 31) / 32 * 32);
-    if (e == cudaSuccess) e = cudaMalloc(&t->d_counters, sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMallocHost(&t->h_counters, 2 * sizeof(unsigned long long));
-    if (e == cudaSuccess) std::memset(t->h_counters, 0, 2 * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMalloc(&t->d_counters, kDeviceWords * sizeof(unsigned long long));
+    // on the creating call's stream, which the clearing of the slots goes on as well
+    if (e == cudaSuccess) e = cudaMemsetAsync(t->d_counters, 0, kDeviceWords * sizeof(unsigned long long), cs(stream));
+    if (e == cudaSuccess) e = cudaMallocHost(&t->h_counters, kHostWords * sizeof(unsigned long long));
     if (e != cudaSuccess) {
         b2co_oa_destroy(t);
         return cuda_fail(e, "table allocation");
+    }
+    std::memset(t->h_counters, 0, kHostWords * sizeof(unsigned long long));
+    for (int i = 0; i < kCounterSets; ++i) {
+        t->sets[i].c = Counters{t->d_counters + 1 + i * kSumWords, t->h_counters + 2 + i * kCounterWords};
+        give_counters(t, &t->sets[i]);
     }
     if (clear && (st = b2co_oa_clear(t, stream))) {
         b2co_oa_destroy(t);
@@ -428,9 +455,12 @@ int b2co_oa_destroy(b2co_oa_table* t)
     if (t->args.slots) cudaFree(t->args.slots);
     if (t->d_counters) cudaFree(t->d_counters);
     if (t->h_counters) cudaFreeHost(t->h_counters);
-    for (Counters const& c : t->counters) {
-        cudaFree(c.sum);
-        cudaFreeHost(c.host);
+    for (CounterSet* c = t->more; c;) {
+        CounterSet* const next = c->next;
+        cudaFree(c->c.sum);
+        cudaFreeHost(c->c.host);
+        delete c;
+        c = next;
     }
     if (t->d_pos) cudaFree(t->d_pos);
     if (t->d_newbits) cudaFree(t->d_newbits);
