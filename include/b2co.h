@@ -560,10 +560,13 @@ int b2co_bloom_add(b2co_bloom* filter, const void* keys, uint64_t n, b2co_stream
  * four 64-bit atomic ORs per key from the SM.  B2CO_BLOOM_ADD_BULK: one
  * 32-byte TMA bulk reduction (OR) per key from shared memory.
  * B2CO_BLOOM_ADD_PARTITIONED: keys are routed by 128 KiB filter slice into a
- * record workspace (8 bytes per key and room for uneven shares, about a fifth
- * more for large batches; at most 2^27 keys and an eighth per round, allocated on
- * first use and kept with the filter), then each slice is built in shared
- * memory and ORed into the filter; filters above 2048 slices (256 MiB) use BULK.
+ * record workspace (8 bytes per key and room for uneven shares, from a fifth
+ * more for 2^27 keys on a 128 MiB filter to half more at 8 keys per block; at most
+ * 2^27 keys and an eighth per round), then each slice is built in shared memory
+ * and ORed into the filter.  The workspace is allocated on first use, grows with
+ * the largest batch and is kept with the filter; a batch of several rounds settles
+ * it for good, and where memory is short the filter takes shorter rounds from then
+ * on.  An Add that is captured into a graph must find it there; filters above 2048 slices (256 MiB) use BULK.
  * B2CO_BLOOM_ADD_AUTO (the default): PARTITIONED for filters of at least 64 MiB
  * and batches of at least 8 keys per filter block, BULK otherwise -- the
  * reference likewise chooses between

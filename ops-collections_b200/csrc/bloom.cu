@@ -156,8 +156,10 @@ __global__ void __launch_bounds__(256) k_bloom_add_bulk(uint32_t* words, uint32_
 //             copy of the slice and reduces the whole copy into the filter with
 //             TMA bulk ORs (element-wise atomic in L2, so concurrent Adds on
 //             other streams stay correct).
-// Fixed segments take a fifth more workspace than exact ones, and save the pass
-// that counts (and hashes) every key to size them: 0.46 of 2.2 ms for 2^27 keys.
+// Fixed segments take more workspace than exact ones, from a fifth more for 2^27
+// keys on a 128 MiB filter (886 records a segment) to half more at 8 keys per
+// block (221), and save the pass that counts (and hashes) every key to size
+// them: 0.46 of 2.2 ms for 2^27 keys.
 // DRAM traffic per key is the key once and a record written and read back
 // (8 + 8 + 8 bytes), against two scattered 32-byte block transfers per key
 // otherwise.
@@ -376,7 +378,7 @@ __global__ void __launch_bounds__(kApplyThreads) k_bloom_apply(uint32_t* words, 
     for (uint32_t c = threadIdx.x >> 5; c < nctas; c += kApplyThreads / 32) {
         uint32_t const count = counts[uint64_t(sl) * nctas + c];
         unsigned long long const* const seg = recs + uint64_t(sl * nctas + c) * segment;
-                constexpr int kAhead = 4;  // records loaded before any is applied
+        constexpr int kAhead = 4;  // records loaded before any is applied
         for (uint32_t r = lane; r < count; r += 32 * kAhead) {
             unsigned long long rec[kAhead];
 #pragma unroll
@@ -565,6 +567,12 @@ struct b2co_bloom {
     int add_mode = B2CO_BLOOM_ADD_AUTO;  // default-policy Add: see b2co_bloom_add_mode
     unsigned long long* recs = nullptr;  // partitioned Add: record workspace
     uint64_t recs_cap = 0;
+    uint64_t recs_refused = ~0ull;  // records that there was no room for: not asked for again
+    bool recs_in_graph = false;     // a captured Add holds the workspace's address
+    struct Parked {                 // workspaces outgrown, but held by graphs
+        void* p;
+        Parked* next;
+    }* parked = nullptr;
     uint32_t* part = nullptr;  // partitioned Add: records of every segment
     size_t part_words = 0;
     ScratchOrder part_order;  // the workspace serves one partitioned Add at a time
@@ -645,10 +653,72 @@ int launch_contains_policy(b2co_bloom* f, void const* keys, uint8_t const* stenc
 // capture cannot, so smaller batches stay without one.
 constexpr uint64_t kPartitionKeysPerBlock = 8;
 constexpr uint64_t kPartitionFilterBytes = uint64_t(64) << 20;
-// Keys per route-and-apply round.  A batch that passes it by less than an eighth
-// stays one round: a round costs about 100 us however few its keys.
+// Keys per route-and-apply round: a batch that passes kPartitionRound by less
+// than an eighth stays one round, as a round costs about 100 us however few its
+// keys, and a larger one is dealt evenly over rounds.
 constexpr uint64_t kPartitionRound = uint64_t(1) << 27;
+constexpr uint64_t kLongestRound = kPartitionRound / 8 * 9;
 constexpr uint64_t kMinPartitionRound = uint64_t(1) << 20;
+
+struct RoutePlan {
+    uint64_t round;    // keys
+    uint32_t nctas, segment;
+    uint64_t records;  // of the workspace; never falls with the round's keys
+};
+
+RoutePlan route_plan(uint64_t n, uint64_t rounds, uint32_t route_cap, uint32_t nslices)
+{
+    RoutePlan p;
+    p.round = (n + rounds - 1) / rounds;
+    uint64_t const tiles = (p.round + kRouteTile - 1) / kRouteTile;
+    p.nctas = uint32_t(tiles < route_cap ? tiles : route_cap);
+    p.segment = route_segment(p.round, p.nctas, nslices);
+    p.records = uint64_t(nslices) * p.nctas * p.segment;
+    return p;
+}
+
+// Asks for a workspace of so many records; the one there is serves until the
+// larger one is in hand, and stays when there is no room for that.
+int grow_records(b2co_bloom* f, uint64_t records)
+{
+    if (records >= f->recs_refused) return B2CO_OK;
+    unsigned long long* p = nullptr;
+    cudaError_t const e = cudaMalloc(&p, records * 8);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        f->recs_refused = records;
+        return B2CO_OK;
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "BloomFilter::Add workspace");
+    if (f->recs_in_graph) {  // a graph may be replayed at any time
+        if (auto* node = new (std::nothrow) b2co_bloom::Parked{f->recs, f->parked}) f->parked = node;
+    } else if (f->recs) {
+        cudaFree(f->recs);
+    }
+    f->recs = p;
+    f->recs_cap = records;
+    f->recs_in_graph = false;
+    return B2CO_OK;
+}
+
+// The rounds of a batch, with a workspace for them.  A batch of several rounds
+// settles it for good: it is made for the longest round that there is, so no
+// later batch asks for more.  Where there is no room for a round's records the
+// rounds are shorter, for this and for later batches.
+int plan_partitioned(b2co_bloom* f, uint64_t n, uint32_t route_cap, uint32_t nslices, RoutePlan& plan)
+{
+    uint64_t rounds = (n + kLongestRound - 1) / kLongestRound;
+    plan = route_plan(n, rounds, route_cap, nslices);
+    if (f->recs_cap < plan.records && rounds > 1)
+        if (int st = grow_records(f, route_plan(kLongestRound, 1, route_cap, nslices).records)) return st;
+    for (;;) {
+        if (f->recs_cap < plan.records)
+            if (int st = grow_records(f, plan.records)) return st;
+        if (f->recs_cap >= plan.records) return B2CO_OK;
+        if (plan.round <= kMinPartitionRound) return cuda_fail(cudaErrorMemoryAllocation, "BloomFilter::Add workspace");
+        plan = route_plan(n, rounds *= 2, route_cap, nslices);
+    }
+}
 
 template <int KB>
 int launch_add_partitioned(b2co_bloom* f, void const* keys, uint8_t const* stencil, uint64_t n, cudaStream_t s)
@@ -664,26 +734,8 @@ int launch_add_partitioned(b2co_bloom* f, void const* keys, uint8_t const* stenc
     int per_sm = 0;
     B2CO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (void const*)route, kRouteThreads, rsmem));
     uint32_t const route_cap = uint32_t(per_sm < 1 ? 1 : per_sm) * uint32_t(sm_count());
-    uint64_t rounds = (n + kPartitionRound / 8 * 9 - 1) / (kPartitionRound / 8 * 9), round = 0;
-    uint32_t nctas = 0, segment = 0;
-    for (;; rounds *= 2) {  // shorter rounds where there is no room for the records of the longest
-        round = (n + rounds - 1) / rounds;
-        uint64_t const tiles = (round + kRouteTile - 1) / kRouteTile;
-        nctas = uint32_t(tiles < route_cap ? tiles : route_cap);
-        segment = route_segment(round, nctas, nslices);
-        uint64_t const want = uint64_t(nslices) * nctas * segment;
-        if (f->recs_cap >= want) break;
-        if (f->recs) cudaFree(f->recs);
-        f->recs = nullptr;
-        f->recs_cap = 0;
-        cudaError_t const e = cudaMalloc(&f->recs, want * 8);
-        if (e == cudaSuccess) {
-            f->recs_cap = want;
-            break;
-        }
-        if (e != cudaErrorMemoryAllocation || round <= kMinPartitionRound) return cuda_fail(e, "BloomFilter::Add workspace");
-        cudaGetLastError();
-    }
+    RoutePlan plan;
+    if (int st = plan_partitioned(f, n, route_cap, nslices, plan)) return st;
     size_t const part_words = size_t(route_cap) * kMaxSlices;
     if (f->part_words < part_words) {
         if (f->part) cudaFree(f->part);
@@ -692,14 +744,16 @@ int launch_add_partitioned(b2co_bloom* f, void const* keys, uint8_t const* stenc
         B2CO_CUDA(cudaMalloc(&f->part, part_words * 4));
         f->part_words = part_words;
     }
+    if (capturing(s)) f->recs_in_graph = true;
     if (int st = f->part_order.begin(s)) return st;
-    for (uint64_t at = 0; at < n; at += round) {
-        uint64_t const m = n - at < round ? n - at : round;
+    for (uint64_t at = 0; at < n; at += plan.round) {
+        uint64_t const m = n - at < plan.round ? n - at : plan.round;
         void const* k = static_cast<char const*>(keys) + at * KB;
         uint8_t const* st = stencil ? stencil + at : nullptr;
-        route<<<nctas, kRouteThreads, rsmem, s>>>(f->words, nblocks, f->seed, k, st, m, nslices, nctas, segment, f->part,
-                                                  f->recs);
-        k_bloom_apply<<<nslices, kApplyThreads, apply_smem, s>>>(f->words, nblocks, f->recs, f->part, nctas, segment);
+        route<<<plan.nctas, kRouteThreads, rsmem, s>>>(f->words, nblocks, f->seed, k, st, m, nslices, plan.nctas,
+                                                       plan.segment, f->part, f->recs);
+        k_bloom_apply<<<nslices, kApplyThreads, apply_smem, s>>>(f->words, nblocks, f->recs, f->part, plan.nctas,
+                                                                 plan.segment);
     }
     B2CO_CUDA(cudaGetLastError());
     return f->part_order.end(s);
@@ -829,6 +883,12 @@ int b2co_bloom_destroy(b2co_bloom* f)
     if (f->words) cudaFree(f->words);
     if (f->recs) cudaFree(f->recs);
     if (f->part) cudaFree(f->part);
+    while (f->parked) {
+        b2co_bloom::Parked* const next = f->parked->next;
+        cudaFree(f->parked->p);
+        delete f->parked;
+        f->parked = next;
+    }
     f->part_order.release();
     delete f;
     return B2CO_OK;
