@@ -428,7 +428,8 @@ def measure_e2e(t, q, out, stream, world, args):
 def host_find_chunks(n, full=1 << 22):
     """Chunks (one Find launch each) of the host-buffer Find of n keys: batches
     of 16 Mi keys or more ramp up with 1 and 2 Mi chunks and down with 2 and 1 Mi.
-    (Below, this counts whole chunks; the library deals such a batch over four.)"""
+    Below, this counts the whole chunks of a batch in pageable memory; one in
+    pinned memory is dealt over four.  (The step timed here has 2^27 keys.)"""
     q, h, off, count = full // 4, full // 2, 0, 0
     while off < n:
         left = n - off

@@ -764,15 +764,26 @@ int b2co_oa_set_write_shape(b2co_oa_table* t, uint32_t lanes, uint32_t keys_per_
 // evenly over kHostChunks chunks, down to kHostChunkMin keys each (int64 pairs,
 // 1 / 2 / 4 / 8 chunks: 4.2 Mi keys 1,379 / 1,085 / 1,025 / 1,100 us, 10 M keys
 // 2,450 / 2,377 / 2,240 / 2,225, 1 Mi keys 365 / 320 / 312 / 320).
-// Pinned host buffers give full overlap.
+// Pinned host buffers give full overlap.  A copy from or to pageable memory keeps
+// the calling thread until it is done, so nothing overlaps and a chunk more only
+// costs: such a batch goes in whole chunks (0.3 and 1 Mi keys, one chunk and four:
+// 355 and 456, 968 and 1,168 us).
 constexpr uint64_t kHostChunk = 1ull << 22;     // keys per full chunk
 constexpr uint64_t kHostChunks = 4;             // chunks of a batch below 4 full ones
 constexpr uint64_t kHostChunkMin = 1ull << 17;  // a batch of one chunk needs no pipeline
 
-static uint64_t host_chunk_at(uint64_t off, uint64_t n)
+static bool is_pageable(void const* p)
+{
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) cudaGetLastError();
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
+static uint64_t host_chunk_at(uint64_t off, uint64_t n, bool pageable)
 {
     uint64_t const q = kHostChunk / 4, h = kHostChunk / 2, left = n - off;
     if (n < 4 * kHostChunk) {
+        if (pageable) return left < kHostChunk ? left : kHostChunk;
         uint64_t const even = (n + kHostChunks - 1) / kHostChunks;
         uint64_t const chunk = std::min(std::max((even + 63) / 64 * 64, kHostChunkMin), kHostChunk);
         return left < chunk ? left : chunk;
@@ -799,13 +810,14 @@ int b2co_oa_find_host(b2co_oa_table* t, void const* host_keys, void* host_out, u
     }
     cudaStream_t c = cs(s);
     char* base = static_cast<char*>(t->stage);
-    bool const piped = host_chunk_at(0, n) < n;  // one chunk stays on the caller's stream
+    bool const pageable = n > kHostChunkMin && n < 4 * kHostChunk && (is_pageable(host_keys) || is_pageable(host_out));
+    bool const piped = host_chunk_at(0, n, pageable) < n;  // one chunk stays on the caller's stream
     if (piped) {
         B2CO_CUDA(cudaEventRecord(t->ev[kHostSlots], c));
         for (auto& p : t->pipe) B2CO_CUDA(cudaStreamWaitEvent(p, t->ev[kHostSlots], 0));
     }
     for (uint64_t off = 0, c_i = 0, m = 0; off < n; off += m, ++c_i) {
-        m = host_chunk_at(off, n);
+        m = host_chunk_at(off, n, pageable);
         int slot = int(c_i % kHostSlots);
         cudaStream_t p = piped ? t->pipe[slot] : c;
         char* dk = base + uint64_t(slot) * chunk * (kb + ob);
