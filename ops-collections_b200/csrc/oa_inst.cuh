@@ -34,6 +34,9 @@ constexpr uint64_t kNarrowFindBytes = uint64_t(320) << 20;
 // present keys 220 MB 22.5 / 19.4, 300 MB 17.9 / 18.8.
 constexpr uint64_t kSectorInsertBytes = uint64_t(352) << 20;
 constexpr uint64_t kSectorAssignBytes = uint64_t(256) << 20;
+// A small batch, as with the lookups: on a 1.2 GB table, sector / tiled, InsertOrAssign of 8,192 /
+// 32,768 / 65,536 / 131,072 present keys takes 5.4 / 8.2, 6.8 / 8.5, 10.1 / 10.2 and 16.9 / 13.3 us.
+constexpr uint32_t kSectorWriteKeys = 1u << 16;
 // Threads per block of the sector kernels: a batch that does not fill the GPU is
 // spread over more SMs in smaller blocks (an SM takes its windows' requests one
 // after the other): 1,000 keys take 3.8 us in blocks of 64 and 4.8 in blocks of 256.
@@ -79,13 +82,14 @@ struct OaImpl {
 
     // Whether the insert family runs one key per lane (oa_sector.cuh) instead of
     // a tile per window (oa_insert.cuh).
-    static bool sector_writes(OaArgs const& a, int B, int mode)
+    static bool sector_writes(OaArgs const& a, int B, int mode, uint32_t n)
     {
         uint32_t const lanes = a.write_shape >> 8;
         return B == 1 || lanes == 1 ||
-               (lanes == 0 && table_bytes(a) <= (mode == kInsAssign ? kSectorAssignBytes
-                                              : mode >= kInsMark  ? kSectorFindBytes
-                                                                  : kSectorInsertBytes));
+               (lanes == 0 && (n <= kSectorWriteKeys ||
+                               table_bytes(a) <= (mode == kInsAssign ? kSectorAssignBytes
+                                                  : mode >= kInsMark  ? kSectorFindBytes
+                                                                      : kSectorInsertBytes)));
     }
 
     // A write of one mode.
@@ -94,9 +98,10 @@ struct OaImpl {
                      cudaStream_t s)
     {
         if constexpr (B > 1) {
-            if (!sector_writes(a, B, MODE)) {
+            if (!sector_writes(a, B, MODE, n)) {
                 auto k = k_insert_tile<S, B, MODE>;
-                k<<<grid_for((void const*)k, kBlock, n, kBlock), kBlock, 0, s>>>(a, pairs, stencil, n, o);
+                uint32_t const block = sector_block(n);
+                k<<<grid_for((void const*)k, block, n, block), block, 0, s>>>(a, pairs, stencil, n, o);
                 return check_launch("insert kernel");
             }
         }
