@@ -20,6 +20,10 @@
 // one ballot (the lowest lane holding a deciding slot), and the owner gets the
 // slot's place by one shuffle.
 //
+// InsertAndFind (race) of slots up to 8 bytes takes the present slot from the tile
+// by one more shuffle; reading it again is an access to HBM (16 M pairs, 1.1 GB of
+// 8-byte slots: 884 to 519 us).  A wider slot is read again.
+//
 // The window is a snapshot, and that is safe: during these kernels slots only
 // go from empty to occupied, so a slot seen occupied by another key stays so,
 // and a slot seen empty is re-checked by the CAS itself.
@@ -49,6 +53,7 @@ __global__ void __launch_bounds__(256, B2CO_TILE_WRITE_MINB((kTileLanes<S, B>)))
 {
     using Raw = typename S::Raw;
     constexpr int G = kTileLanes<S, B>;
+    constexpr bool kCarry = MODE == kInsIafRace && S::bytes <= 8;  // the owner gets the slot itself
     static_assert(SectorWindow<S, B>::NS <= G && G * (32 / S::bytes) <= 32, "tile shape");
     constexpr uint32_t TILES = 32 / G, TM = (1u << G) - 1u, N = 32 / S::bytes;
     constexpr uint32_t RING = kSectorRing - 1;
@@ -119,9 +124,11 @@ __global__ void __launch_bounds__(256, B2CO_TILE_WRITE_MINB((kTileLanes<S, B>)))
         }
         // each owner learns where its window's first deciding slot is and whether it is empty
         uint32_t mine = 0;  // slot among the window's sectors | 32: empty | 64: found
+        Raw carried{};
 #pragma unroll
         for (int q = 0; q < G; ++q) {
             uint32_t info = 0;
+            Raw stop{};
             if (valid[q]) {
                 uint32_t stops = 0, empties = 0;
 #pragma unroll
@@ -134,20 +141,30 @@ __global__ void __launch_bounds__(256, B2CO_TILE_WRITE_MINB((kTileLanes<S, B>)))
                 if (stops) {
                     uint32_t const i = uint32_t(__ffs(stops) - 1);
                     info = i | (((empties >> i) & 1u) ? 96u : 64u);
+                    if constexpr (kCarry) {
+#pragma unroll
+                        for (int j = 0; j < int(N); ++j)
+                            if (i == uint32_t(j)) stop = sector_slot<S>(w[q], j);
+                    }
                 }
             }
             uint32_t const m = (__ballot_sync(0xffffffffu, info != 0) >> own_shift) & TM;
             uint32_t const first = m ? uint32_t(__ffs(m) - 1) : 0u;
             uint32_t const got = __shfl_sync(0xffffffffu, info, own_shift + first);
             if (uint32_t(q) == own_q && m) mine = got + first * N;
+            if constexpr (kCarry) {
+                using Word = typename std::conditional<S::bytes == 8, unsigned long long, uint32_t>::type;
+                Raw const at = Raw(__shfl_sync(0xffffffffu, Word(stop), own_shift + first));
+                if (uint32_t(q) == own_q) carried = at;
+            }
         }
         int verdict = kOpen;
         if (live && mine) {
             Raw* const win = slots + idx;
             int j = int(mine & 31u) - int(uint32_t(reinterpret_cast<uintptr_t>(win) & 31) / S::bytes);
-            // the slot itself stayed with the tile: a present one is read again where its payload is wanted
+            // a 16-byte slot stayed with the tile: a present one is read again where its payload is wanted
             Raw cur = S::make(a.empty_key, a.empty_value);
-            if (!(mine & 32u)) cur = MODE == kInsIafRace ? ld_rw(win + j) : S::make(~a.empty_key, 0);
+            if (!(mine & 32u)) cur = kCarry ? carried : MODE == kInsIafRace ? ld_rw(win + j) : S::make(~a.empty_key, 0);
             uint64_t found = 0;
             verdict = sector_decide<S, B, MODE>(a, win, j, cur, key, S::value(pr), found);
             if (verdict != kOpen) record(a, o, pos, verdict, idx + uint32_t(j), found);
