@@ -26,6 +26,14 @@ namespace b2co {
 // 16,384 keys, 8.9 / 10.1 for 65,536 and 13.6 / 12.1 for 131,072.
 constexpr uint64_t kSectorFindBytes = uint64_t(224) << 20;
 constexpr uint32_t kSectorFindKeys = 3u << 15;
+// Tables inside the line all the same take the tiled lookup in large batches where
+// the sector kernel is bound by instructions, sector / tiled in Gkeys/s (16 M queries,
+// 16-byte slots): windows of four sectors (eight slots), 24 / 150 / 220 MB 46 / 46 / 39 and
+// 56 / 49 / 46; and of three for a Contains, which needs the keys only, with the table
+// well inside L2 (five slots), 24 / 60 / 150 MB 72 / 71 / 51 and 80 / 63 / 40.  Smaller
+// batches and fuller tables would lose: 1 Mi queries at load 0.95, 24 MB, 69 us and 91.
+constexpr uint64_t kTiledContainsBytes = uint64_t(40) << 20;
+constexpr uint32_t kTiledFourKeys = 1u << 20, kTiledContainsKeys = 1u << 22;
 // Two lanes and one window in flight against four and two: 34 / 31 at 220 MB,
 // 33 / 30 at 300 MB, 27 / 29 at 520 MB.
 constexpr uint64_t kNarrowFindBytes = uint64_t(320) << 20;
@@ -246,7 +254,9 @@ struct OaImpl {
     {
         DeferFn const even = a.keep_misses ? k_find_wdefer<S, B, G, Q, C, true, true> : k_find_wdefer<S, B, G, Q, C, true>;
         uint64_t const share = (n + defer_warps(even) - 1) / defer_warps(even);
-        if (share >= kWarpStageKeys && !a.keep_misses)
+        // (the even deal's kernel for windows of four sectors is the slower one: 1 Mi keys, 300 MB, 29 us against 40)
+        uint64_t const whole = SectorWindow<S, B>::NS >= 4 ? kWarpStageKeys / 2 : kWarpStageKeys;
+        if (share >= whole && !a.keep_misses)
             return launch_wdefer(k_find_wdefer<S, B, G, Q, C>, C, a, keys, out, n, kWarpStageKeys, wc, s);
         uint64_t const rounds = (share + kWarpStageKeys - 1) / kWarpStageKeys;
         return launch_wdefer(even, C, a, keys, out, n, ((share + rounds - 1) / rounds + 31) / 32 * 32, wc, s);
@@ -280,7 +290,11 @@ struct OaImpl {
                          cudaStream_t s)
     {
         if constexpr (B > 1) {
-            if ((table_bytes(a) > kSectorFindBytes || S::bytes <= 4) && n > kSectorFindKeys) {
+            constexpr int kSectors = SectorWindow<S, B>::NS;
+            bool const tiled = table_bytes(a) > kSectorFindBytes || S::bytes <= 4 || (kSectors >= 4 && n >= kTiledFourKeys) ||
+                               (C && kSectors == 3 && !a.keep_misses && table_bytes(a) <= kTiledContainsBytes &&
+                                n >= kTiledContainsKeys);
+            if (tiled && n > kSectorFindKeys) {
                 bool const narrow = S::bytes <= 4 || table_bytes(a) <= kNarrowFindBytes;
                 if (stencil || (reinterpret_cast<uintptr_t>(keys) & 15))  // keys cannot be staged
                     return find_shape<B, C>(a, narrow ? 2 : 4, 1, keys, stencil, out, n, wc, s);
