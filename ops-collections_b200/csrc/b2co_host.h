@@ -114,7 +114,8 @@ struct GroupOps {
     // shape: lanes | keys per lane group << 8 | threads per block << 16
     int (*find)(GroupArgs const& g, uint32_t b, uint32_t shape, bool contains, void const* keys, void* out,
                 uint64_t n, cudaStream_t s);
-    int (*insert)(GroupArgs const& g, uint32_t b, void const* pairs, uint64_t n, unsigned long long* failed,
+    // tiled: a window is read by a tile of lanes, not by one (large tables)
+    int (*insert)(GroupArgs const& g, uint32_t b, bool tiled, void const* pairs, uint64_t n, unsigned long long* failed,
                   cudaStream_t s);
 };
 

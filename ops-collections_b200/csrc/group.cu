@@ -39,6 +39,7 @@ struct b2co_oa_group {
     unsigned long long* d_counters = nullptr;  // [failed, status], then a chunk counter per dealt launch in flight
     unsigned long long* h_counters = nullptr;
     uint32_t find_shape = 1u | (1u << 8);  // lanes | keys per lane group << 8 | block << 16 (0 = 256)
+    bool tiled_writes = false;
     std::mutex deal_mutex;
     uint32_t next_dealer = 0;
     ScratchOrder deal_order[kDealers];  // a chunk counter serves one launch at a time
@@ -94,6 +95,35 @@ OaArgs table_args(b2co_oa_group const* g, uint32_t t)
     a.empty_value = g->desc.value_bytes ? g->desc.empty_value_bits : 0;
     a.erased_key = g->desc.empty_key_bits;
     return a;
+}
+
+// Groups of few large tables: an item's table is far larger than L2, and neighbouring
+// items share no more of it than others do, so a window wants to be asked for in as
+// few requests as it takes (oa_insert.cuh), as in a single large table.  Mean table of an
+// item, one lane a key / tiled, us for 3.4 M and 33.6 M items (16-byte slots): Insert
+// 256 MB 206 / 186 and 1,483 / 1,491, 512 MB 301 / 189 and 2,122 / 1,633, 1 GB 355 / 202 and
+// 2,573 / 1,736; Find 256 MB 165 / 156 and 902 / 1,412, 384 MB 247 / 200 and 1,622 / 1,624,
+// 1 GB 272 / 161 and 2,070 / 1,476.  8-byte slots have their lines in the same place.
+constexpr double kTiledTableBytes = double(320 << 20);
+// An Insert of few items into a slab past L2, whatever its tables, finds no sector that a
+// neighbour has asked for either: 1 GB of 16-byte slots, items a slot, one lane a key / tiled:
+// 32 tables 1/100 60 / 54 us, 1/20 211 / 188, 1/2 1,062 / 1,226; 8-byte slots 1/20 321 / 308, 1/2 1,697 / 1,654.
+constexpr uint64_t kTiledSlabBytes = uint64_t(352) << 20;
+bool tiled_insert(b2co_oa_group const* g, uint64_t n)
+{
+    return g->tiled_writes || (n < g->total_slots / 12 && g->total_slots * g->slot_bytes > kTiledSlabBytes);
+}
+
+void default_shapes(b2co_oa_group* g)
+{
+    double squares = 0;  // a table is met in proportion to its size
+    for (GroupTable const& t : g->host_tables) {
+        double const bytes = double(t.probe.capacity) * g->slot_bytes;
+        squares += bytes * bytes;
+    }
+    g->tiled_writes = squares >= kTiledTableBytes * double(g->total_slots) * g->slot_bytes;
+    if (g->tiled_writes && g->desc.bucket_size > 1)
+        g->find_shape = 2u | ((g->desc.bucket_size == 5 ? 2u : 1u) << 8);  // the deferred 2-lane kernel is for five slots
 }
 
 // Large batches deal their chunks to the warps by a counter (group_kernels.cuh).
@@ -252,6 +282,7 @@ int b2co_oa_group_create(b2co_oa_desc const* d, uint64_t const* requested, uint3
         off += cap;
     }
     g->total_slots = off;
+    default_shapes(g);
     B2CO_CUDA(cudaMalloc(&g->slab, (off * g->slot_bytes + 31) / 32 * 32));  // whole sectors (oa_sector.cuh)
     B2CO_CUDA(cudaMalloc(&g->d_tables, sizeof(GroupTable) * count));
     B2CO_CUDA(cudaMemcpy(g->d_tables, g->host_tables.data(), sizeof(GroupTable) * count, cudaMemcpyHostToDevice));
@@ -332,7 +363,7 @@ int b2co_oa_group_insert(b2co_oa_group* g, void const* pairs, uint64_t const* d_
     cudaStream_t c = cs(s);
     if (failed) B2CO_CUDA(cudaMemsetAsync(g->d_counters, 0, sizeof(unsigned long long), c));
     int st = dealt(g, group_args(g, d_offsets), n, c, [&](GroupArgs const& a) {
-        return g->gops->insert(a, g->desc.bucket_size, pairs, n, failed ? g->d_counters : nullptr, c);
+        return g->gops->insert(a, g->desc.bucket_size, tiled_insert(g, n), pairs, n, failed ? g->d_counters : nullptr, c);
     });
     if (st || !failed) return st;
     B2CO_CUDA(cudaMemcpyAsync(g->h_counters, g->d_counters, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c));

@@ -22,7 +22,7 @@
 // single-table ones.
 #pragma once
 
-#include "oa_sector.cuh"
+#include "oa_insert.cuh"
 
 namespace b2co {
 
@@ -429,10 +429,64 @@ __global__ void __launch_bounds__(256) k_group_find_q(__grid_constant__ const Gr
     while (count > 0) follow();
 }
 
-// Insert into every table: k_insert_sector's pass with the item's own table.
+// Every lane learns where the first deciding slot of its window is (the slot among
+// the window's sectors | 32: empty | 64: found; 0: none), the warp reading its 32
+// windows a sector a lane as k_insert_tile does.
 template <class S, int B>
-__global__ void __launch_bounds__(256, 4) k_group_insert(__grid_constant__ const GroupArgs g, void const* pairs, uint64_t n,
-                                                         uint32_t chunk, unsigned long long* failed_counter)
+__device__ __forceinline__ uint32_t tile_first_slot(bool live, uint64_t key, uint64_t empty_key,
+                                                    typename S::Raw const* window)
+{
+    constexpr int G = kTileLanes<S, B>;
+    constexpr uint32_t TILES = 32 / G, TM = (1u << G) - 1u, N = 32 / S::bytes;
+    static_assert(SectorWindow<S, B>::NS <= G && G * N <= 32, "tile shape");
+    uint32_t const lane = threadIdx.x & 31, r = lane % G, tile = lane / G;
+    uint32_t const own_q = lane / TILES, own_shift = (lane % TILES) * G;  // who reads this lane's window
+    uint32_t const live_mask = __ballot_sync(0xffffffffu, live);
+    Sector w[G];
+    uint64_t k[G];
+    uint32_t valid[G];  // the slots of this lane's sector that lie in the window
+#pragma unroll
+    for (int q = 0; q < G; ++q) {
+        uint32_t const src = q * TILES + tile;
+        k[q] = S::key_bytes <= 4 ? uint64_t(__shfl_sync(0xffffffffu, uint32_t(key), src))
+                                 : __shfl_sync(0xffffffffu, (unsigned long long)key, src);
+        uintptr_t const addr = __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(window), src);
+        valid[q] = ((((1u << B) - 1u) << (uint32_t(addr & 31) / S::bytes)) >> (r * N)) & ((1u << N) - 1u);
+        if (!((live_mask >> src) & 1u)) valid[q] = 0;
+        if (valid[q]) w[q] = ld_sector<true, false>(reinterpret_cast<void const*>((addr & ~uintptr_t(31)) + r * 32));
+    }
+    uint32_t mine = 0;
+#pragma unroll
+    for (int q = 0; q < G; ++q) {
+        uint32_t info = 0;
+        if (valid[q]) {
+            uint32_t stops = 0, empties = 0;
+#pragma unroll
+            for (int i = 0; i < int(N); ++i) {
+                uint64_t const sk = S::key(sector_slot<S>(w[q], i));
+                if (sk == empty_key) empties |= 1u << i;
+                else if (S::key_eq(sk, k[q])) stops |= 1u << i;
+            }
+            stops = (stops | empties) & valid[q];
+            if (stops) {
+                uint32_t const i = uint32_t(__ffs(stops) - 1);
+                info = i | (((empties >> i) & 1u) ? 96u : 64u);
+            }
+        }
+        uint32_t const m = (__ballot_sync(0xffffffffu, info != 0) >> own_shift) & TM;
+        uint32_t const first = m ? uint32_t(__ffs(m) - 1) : 0u;
+        uint32_t const got = __shfl_sync(0xffffffffu, info, own_shift + first);
+        if (uint32_t(q) == own_q && m) mine = got + first * N;
+    }
+    return mine;
+}
+
+// Insert into every table: k_insert_sector's pass with the item's own table, or with
+// TILED k_insert_tile's, the window's address handed to its tile.
+template <class S, int B, bool TILED>
+__global__ void __launch_bounds__(256, TILED ? 3 : 4)
+    k_group_insert(__grid_constant__ const GroupArgs g, void const* pairs, uint64_t n, uint32_t chunk,
+                   unsigned long long* failed_counter)
 {
     using Raw = typename S::Raw;
     constexpr uint32_t RING = kSectorRing - 1;
@@ -497,23 +551,31 @@ __global__ void __launch_bounds__(256, 4) k_group_insert(__grid_constant__ const
             if (begin < n && at + lane < end) next_pair = ld_once(pin + at + lane);
         }
         int verdict = kOpen;
-        if (live) {
-            uint64_t const key = S::key(pr);
+        uint64_t const key = S::key(pr);
+        // the window's first deciding slot: its place in the window, and the slot (TILED: only whether it is empty)
+        int j = -1;
+        Raw cur{};
+        if constexpr (TILED) {
+            uint32_t const at = tile_first_slot<S, B>(live, key, g.empty_key, slots + idx);
+            if (live && at) {
+                j = int(at & 31u) - int(uint32_t(reinterpret_cast<uintptr_t>(slots + idx) & 31) / S::bytes);
+                cur = S::make((at & 32u) ? g.empty_key : ~g.empty_key, 0);
+            }
+        } else if (live) {
             SectorWindow<S, B> w;
             w.template load<true, true>(slots + idx);
-            int j = w.first_stop(key, g.empty_key);
-            if (j >= 0) {
-                Raw old = w.pick(j);
-                verdict = kDuplicate;
-                if (S::key(old) == g.empty_key) {
-                    OaArgs a{};
-                    a.empty_key = g.empty_key;
-                    a.empty_value = g.empty_value;
-                    j -= int(w.off);
-                    verdict = sector_claim<S, B>(a, slots + idx, key, S::value(pr), j, old);
-                }
-                failed += verdict == kDuplicate;
+            int const at = w.first_stop(key, g.empty_key);
+            if (at >= 0) cur = w.pick(at), j = at - int(w.off);
+        }
+        if (j >= 0) {
+            verdict = kDuplicate;
+            if (S::key(cur) == g.empty_key) {
+                OaArgs a{};
+                a.empty_key = g.empty_key;
+                a.empty_value = g.empty_value;
+                verdict = sector_claim<S, B>(a, slots + idx, key, S::value(pr), j, cur);
             }
+            failed += verdict == kDuplicate;
         }
         bool const open = live && verdict == kOpen;
         uint32_t const m = __ballot_sync(0xffffffffu, open);

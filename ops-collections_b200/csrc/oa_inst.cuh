@@ -496,12 +496,14 @@ struct GroupImpl {
         });
     }
 
-    static int insert(GroupArgs const& g, uint32_t b, void const* pairs, uint64_t n, unsigned long long* failed,
-                      cudaStream_t s)
+    static int insert(GroupArgs const& g, uint32_t b, bool tiled, void const* pairs, uint64_t n,
+                      unsigned long long* failed, cudaStream_t s)
     {
         return OaImpl<S>::with_b(b, [&](auto bc) {
             constexpr int B = decltype(bc)::value;
-            auto k = k_group_insert<S, B>;
+            auto k = k_group_insert<S, B, false>;
+            if constexpr (B > 1)
+                if (tiled) k = k_group_insert<S, B, true>;
             uint32_t const grid = grid_for((void const*)k, kBlock, n, kBlock);
             k<<<grid, kBlock, 0, s>>>(g, pairs, n, group_chunk(n, uint64_t(grid) * kBlock / 32), failed);
             return OaImpl<S>::check_launch("group insert kernel");
