@@ -1147,8 +1147,8 @@ int mmap_plan(b2co_mmap* m, cudaStream_t st, uint64_t* tsize, uint32_t* part_bit
     if (n < kSurveyPairs) return B2CO_OK;
     using Raw = typename SlotT<KB, VB>::Raw;
     if (!m->d_survey) {
+        if (!m->h_survey) B2CO_CUDA(cudaMallocHost(reinterpret_cast<void**>(&m->h_survey), sizeof(Survey)));
         B2CO_CUDA(cudaMalloc(reinterpret_cast<void**>(&m->d_survey), sizeof(Survey)));
-        B2CO_CUDA(cudaMallocHost(reinterpret_cast<void**>(&m->h_survey), sizeof(Survey)));
     }
     uint32_t const pbits = n > (1ull << 23) ? kMaxPartBits : kMaxPartBits - 1, parts = 1u << pbits;
     constexpr size_t kRead = offsetof(Survey, cursors);
