@@ -246,9 +246,7 @@ __device__ __forceinline__ uint64_t run_hash(KeyWord<KB> k)
     else return fmix64(k, 0);
 }
 
-// One distinct key: its run is csr[offset, offset + count).  A slot is one
-// 16-byte word, so adding to a key or asking for it touches one sector, not one
-// each for key, count and offset.
+// One distinct key: its run is csr[offset, offset + count).
 template <int KB>
 struct alignas(16) RunSlot {
     KeyWord<KB> key;
@@ -260,25 +258,40 @@ struct alignas(16) RunSlot {
 // part of it that one block builds in shared memory.  A table of full size is at
 // most half full; one that was sized by an estimate, and every region that a
 // block built, at most three quarters (region_crowded).
+// Slots of 8-byte keys are one 16-byte word: adding to a key or asking for it
+// touches one sector, not one each for key and run.  4-byte keys lie apart from
+// their runs: a quarter of the bytes serve Contains, and every miss (2 M queries of
+// 16.8 M distinct keys: Contains 46 us against 74, Count 77 against 90).
 template <int KB>
 struct RunTable {
-    RunSlot<KB>* slots;
+    unsigned char* slots;  // kSlotBytes a slot
     uint64_t mask;    // table size - 1 (a power of two)
     uint64_t region;  // region size - 1
     uint32_t shift;   // 64 - log2(table size)
     KeyWord<KB> empty;
 
+    __device__ __forceinline__ KeyWord<KB>* key(uint64_t s) const
+    {
+        return reinterpret_cast<KeyWord<KB>*>(slots + s * (KB == 8 ? 16 : 4));
+    }
+    __device__ __forceinline__ uint32_t* count(uint64_t s) const  // its offset follows
+    {
+        return reinterpret_cast<uint32_t*>(KB == 8 ? slots + s * 16 + 8 : slots + (mask + 1) * 4 + s * 8);
+    }
+    __device__ __forceinline__ void put(uint64_t s, KeyWord<KB> k, uint32_t c, uint32_t offset) const
+    {
+        if constexpr (KB == 8) {
+            *reinterpret_cast<RunSlot<KB>*>(slots + s * 16) = RunSlot<KB>{k, c, offset};
+        } else {
+            *key(s) = k;
+            *reinterpret_cast<uint2*>(count(s)) = make_uint2(c, offset);
+        }
+    }
     __device__ __forceinline__ uint64_t start(KeyWord<KB> k) const { return run_hash<KB>(k) >> shift; }
     __device__ __forceinline__ uint64_t next(uint64_t s) const { return next_in_region(s, region); }
 };
-
 template <int KB>
-__device__ __forceinline__ RunSlot<KB> load_run(RunSlot<KB> const* p)
-{
-    uint4 const v = __ldg(reinterpret_cast<uint4 const*>(p));
-    if constexpr (KB == 8) return RunSlot<KB>{v.x | ((unsigned long long)v.y << 32), v.z, v.w};
-    else return RunSlot<KB>{v.x, v.y, v.z};
-}
+constexpr uint64_t kSlotBytes = KB == 8 ? 16 : 12;
 
 // The key's slot contents; false (and count 0) when absent.  Bounded by the
 // region, whatever the table holds.
@@ -288,12 +301,21 @@ __device__ __forceinline__ bool find_run(RunTable<KB> const& t, KeyWord<KB> k, R
     out.count = 0;
     if (k == t.empty) return false;
     return walk_region(t.start(k), t.region, [&](uint64_t s) {
-        RunSlot<KB> const cur = load_run<KB>(t.slots + s);
-        if (cur.key == k) {
-            out = cur;
+        KeyWord<KB> found;
+        uint2 run;
+        if constexpr (KB == 8) {
+            uint4 const v = __ldg(reinterpret_cast<uint4 const*>(t.key(s)));
+            found = v.x | ((unsigned long long)v.y << 32);
+            run = make_uint2(v.z, v.w);
+        } else {
+            found = __ldg(t.key(s));
+            if (found == k) run = __ldg(reinterpret_cast<uint2 const*>(t.count(s)));
+        }
+        if (found == k) {
+            out = RunSlot<KB>{k, run.x, run.y};
             return int(kProbeHit);
         }
-        return int(cur.key == t.empty ? kProbeMiss : kProbeOn);
+        return int(found == t.empty ? kProbeMiss : kProbeOn);
     });
 }
 
@@ -301,8 +323,7 @@ template <int KB>
 __global__ void __launch_bounds__(256) k_run_clear(RunTable<KB> t)
 {
     uint64_t const n = t.mask + 1, stride = uint64_t(gridDim.x) * blockDim.x;
-    RunSlot<KB> const e{t.empty, 0u, 0u};
-    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) t.slots[i] = e;
+    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) t.put(i, t.empty, 0u, 0u);
 }
 
 // Counters of one build: runs << 32 | values, then the runs too long for the
@@ -332,8 +353,8 @@ __global__ void __launch_bounds__(256) k_run_count(RunTable<KB> t, typename Slot
         uint64_t s = t.start(k);
         uint32_t probes = 0;
         for (;;) {
-            KeyWord<KB> cur = t.slots[s].key;
-            if (cur == t.empty) cur = atomicCAS(&t.slots[s].key, t.empty, k);
+            KeyWord<KB> cur = *t.key(s);
+            if (cur == t.empty) cur = atomicCAS(t.key(s), t.empty, k);
             if (cur == t.empty || cur == k) break;
             s = t.next(s);
             if (crowded && ++probes == kMaxProbes) {
@@ -342,7 +363,7 @@ __global__ void __launch_bounds__(256) k_run_count(RunTable<KB> t, typename Slot
             }
         }
         bool const placed = !crowded || probes < kMaxProbes;
-        place[i] = placed ? make_uint2(uint32_t(s), atomicAdd(&t.slots[s].count, 1u)) : make_uint2(0u, kNoPlace);
+        place[i] = placed ? make_uint2(uint32_t(s), atomicAdd(t.count(s), 1u)) : make_uint2(0u, kNoPlace);
     }
 }
 
@@ -367,7 +388,7 @@ __global__ void __launch_bounds__(kThreads) k_run_offsets(RunTable<KB> t, uint2 
         }
 #pragma unroll
         for (int r = 0; r < kRounds; ++r) {
-            count[r] = p[r].y == 0 ? t.slots[p[r].x].count : 0u;
+            count[r] = p[r].y == 0 ? *t.count(p[r].x) : 0u;
             if (count[r]) mine += (1ull << 32) + count[r];
         }
         uint64_t total;
@@ -378,7 +399,7 @@ __global__ void __launch_bounds__(kThreads) k_run_offsets(RunTable<KB> t, uint2 
 #pragma unroll
         for (int r = 0; r < kRounds; ++r) {
             if (!count[r]) continue;
-            t.slots[p[r].x].offset = uint32_t(at);
+            t.count(p[r].x)[1] = uint32_t(at);
             runs[at >> 32] = make_uint2(uint32_t(at), count[r]);
             at += (1ull << 32) + count[r];
         }
@@ -398,7 +419,7 @@ __global__ void __launch_bounds__(256) k_run_scatter(RunTable<KB> t, typename Sl
     for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
         uint2 const p = place[i];
         if (p.y == kNoPlace) continue;
-        csr[uint64_t(__ldg(&t.slots[p.x].offset)) + p.y] = ValueWord<VB>(S::value(dense[i]));
+        csr[uint64_t(__ldg(t.count(p.x) + 1)) + p.y] = ValueWord<VB>(S::value(dense[i]));
     }
 }
 
@@ -634,7 +655,8 @@ __global__ void __launch_bounds__(kPartThreads)
     }
     __syncthreads();
     unsigned long long carry = warp_at[warp];
-    RunSlot<KB>* const out = t.slots + uint64_t(blockIdx.x) * slots;
+    uint64_t const out = uint64_t(blockIdx.x) * slots;
+    RunSlot<KB>* const out8 = reinterpret_cast<RunSlot<KB>*>(t.slots) + out;  // put() here costs 8-byte keys 18% of the kernel
     for (uint32_t i = lane; i < share; i += 32) {
         uint32_t const s = first + i, c = counts[s];
         unsigned long long const mine = c ? (1ull << 32) + c : 0;
@@ -646,7 +668,8 @@ __global__ void __launch_bounds__(kPartThreads)
         }
         unsigned long long const at = carry + incl - mine;
         carry += __shfl_sync(0xffffffffu, incl, 31);
-        out[s] = RunSlot<KB>{keys[s], c, c ? uint32_t(at) : 0u};
+        if constexpr (KB == 8) out8[s] = RunSlot<KB>{keys[s], c, c ? uint32_t(at) : 0u};
+        else t.put(out + s, keys[s], c, c ? uint32_t(at) : 0u);
         if (c) runs[at >> 32] = make_uint2(uint32_t(at), c);
         counts[s] = uint32_t(at);
     }
@@ -931,8 +954,8 @@ struct b2co_mmap {
     void* dense = nullptr;
     bool dirty = false;
     // grouped index
-    void* tslots = nullptr;  // RunSlot[tsize]
-    uint64_t tsize = 0, tsize_alloc = 0;
+    void* tslots = nullptr;  // of a RunTable
+    uint64_t tsize = 0, tslots_bytes = 0;
     void* csr = nullptr;
     uint64_t csr_cap = 0;
     Scratch scratch, build, hist, records;
@@ -947,7 +970,7 @@ struct b2co_mmap {
     template <int KB>
     RunTable<KB> table() const
     {
-        return RunTable<KB>{static_cast<RunSlot<KB>*>(tslots), tsize - 1, region - 1,
+        return RunTable<KB>{static_cast<unsigned char*>(tslots), tsize - 1, region - 1,
                             uint32_t(64 - __builtin_ctzll(tsize)), KeyWord<KB>(ek)};
     }
     uint32_t slot_bytes() const { return (kb == 4 && vb == 4) ? 8 : 16; }
@@ -1075,12 +1098,13 @@ int mmap_insert(b2co_mmap* m, void const* pairs, uint8_t const* stencil, uint64_
 
 int mmap_reserve_index(b2co_mmap* m, uint64_t tsize)
 {
-    if (tsize > m->tsize_alloc) {
+    uint64_t const bytes = tsize * (m->kb == 8 ? kSlotBytes<8> : kSlotBytes<4>);
+    if (bytes > m->tslots_bytes) {
         cudaFree(m->tslots);
         m->tslots = nullptr;
-        m->tsize_alloc = 0;
-        B2CO_CUDA(cudaMalloc(&m->tslots, tsize * 16));
-        m->tsize_alloc = tsize;
+        m->tslots_bytes = 0;
+        B2CO_CUDA(cudaMalloc(&m->tslots, bytes));
+        m->tslots_bytes = bytes;
     }
     m->tsize = tsize;
     if (m->size > m->csr_cap) {
