@@ -339,7 +339,8 @@ struct RunCounters {
 constexpr uint32_t kNoPlace = 0xffffffffu;  // no rank in a run: runs have fewer pairs
 constexpr uint32_t kMaxProbes = 128;  // of a table sized by an estimate
 
-// Every pair joins its key's slot; place[i] = (slot, rank of the pair in its run).
+// Every pair joins its key's slot (a warp's pairs of one key with one atomic: 1 M pairs
+// under Zipf(1.1) keys 146 us without that); place[i] = (slot, rank of the pair in its run).
 // A key that finds no place within kMaxProbes slots sets *crowded: the table is
 // too small for the keys, and the host builds again with a full-size one.
 template <int KB, int VB>
@@ -348,22 +349,34 @@ __global__ void __launch_bounds__(256) k_run_count(RunTable<KB> t, typename Slot
 {
     using S = SlotT<KB, VB>;
     uint64_t const stride = uint64_t(gridDim.x) * blockDim.x;
-    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-        KeyWord<KB> const k = KeyWord<KB>(S::key(dense[i]));
-        uint64_t s = t.start(k);
-        uint32_t probes = 0;
-        for (;;) {
-            KeyWord<KB> cur = *t.key(s);
-            if (cur == t.empty) cur = atomicCAS(t.key(s), t.empty, k);
-            if (cur == t.empty || cur == k) break;
-            s = t.next(s);
-            if (crowded && ++probes == kMaxProbes) {
-                *crowded = 1;
-                break;
+    uint32_t const lane = threadIdx.x & 31;
+    for (uint64_t base = uint64_t(blockIdx.x) * blockDim.x + (threadIdx.x & ~31u); base < n; base += stride) {
+        uint64_t const i = base + lane;
+        uint64_t s = 0;
+        bool placed = false;
+        if (i < n) {
+            KeyWord<KB> const k = KeyWord<KB>(S::key(dense[i]));
+            s = t.start(k);
+            for (uint32_t probes = 0;;) {
+                KeyWord<KB> cur = *t.key(s);
+                if (cur == t.empty) cur = atomicCAS(t.key(s), t.empty, k);
+                placed = cur == t.empty || cur == k;
+                if (placed) break;
+                s = t.next(s);
+                if (crowded && ++probes == kMaxProbes) {
+                    *crowded = 1;
+                    break;
+                }
             }
         }
-        bool const placed = !crowded || probes < kMaxProbes;
-        place[i] = placed ? make_uint2(uint32_t(s), atomicAdd(t.count(s), 1u)) : make_uint2(0u, kNoPlace);
+        __syncwarp();
+        // lanes of one key add together; what is not placed has a number of its own
+        uint32_t const peers = __match_any_sync(0xffffffffu, placed ? (unsigned long long)s : ~(unsigned long long)lane);
+        uint32_t const first = uint32_t(__ffs(peers) - 1);
+        uint32_t rank = 0;
+        if (placed && lane == first) rank = atomicAdd(t.count(s), uint32_t(__popc(peers)));
+        rank = __shfl_sync(0xffffffffu, rank, first) + __popc(peers & ((1u << lane) - 1u));
+        if (i < n) place[i] = placed ? make_uint2(uint32_t(s), rank) : make_uint2(0u, kNoPlace);
     }
 }
 
@@ -747,7 +760,7 @@ __device__ __forceinline__ void bitonic_sort(V* v, uint32_t size, uint32_t t, ui
     for (uint32_t k = 2; k <= size; k <<= 1) {
         for (uint32_t j = k >> 1; j > 0; j >>= 1) {
             for (uint32_t p = t; p < size / 2; p += threads) {
-                uint32_t const a = (p / j) * 2 * j + p % j, b = a + j;
+                uint32_t const a = 2 * p - (p & (j - 1)), b = a + j;  // j is a power of two
                 V const x = v[a], y = v[b];
                 bool const up = (a & k) == 0;
                 if ((x > y) == up) v[a] = y, v[b] = x;
