@@ -682,10 +682,7 @@ def fill_measurements(stream, reps=3):
     return res
 
 
-INSERT_SHAPES = [(1, 1), (2, 1), (2, 2), (4, 1), (4, 2), (4, 4), (8, 2), (8, 4)]
-
-
-def insert_measurements(stream, capacity_log2=28, reps=3, shapes=None):
+def insert_measurements(stream, capacity_log2=28, reps=3, shapes=False):
     """The write side of the headline table on its own: StaticMap<int64,int64>,
     DoubleHashing<xxhash_32>, bucket 5, requested capacity 2^capacity_log2; a
     cleared table filled to LF 0.5 by Insert (unique keys), by InsertAndFind in
@@ -729,11 +726,11 @@ def insert_measurements(stream, capacity_log2=28, reps=3, shapes=None):
     res["first_wins_exact"] = bool(int(ins.sum().item()) == unique) and bool(torch.equal(found, vals))
     ms = best(lambda: t.InsertOrAssignAsync(pairs, stream=stream), clear=False)
     res["insert_or_assign_dup_gkeys"] = round(unique / ms / 1e6, 3)
-    if shapes:  # Insert with every write-kernel shape (lanes per window x keys per lane group)
+    if shapes:  # Insert with both write kernels
         sweep = {}
-        for lanes, items in shapes:
-            t.set_write_shape(lanes, items)
-            sweep[f"{lanes}x{items}"] = round(unique / best(lambda: t.InsertAsync(pairs, stream=stream)) / 1e6, 3)
+        for name, lanes in (("one_lane", 1), ("tile", 4)):
+            t.set_write_shape(lanes, 1)
+            sweep[name] = round(unique / best(lambda: t.InsertAsync(pairs, stream=stream)) / 1e6, 3)
         t.set_write_shape(0, 0)
         res["insert_shape_sweep_gkeys"] = sweep
     del t
@@ -1502,7 +1499,7 @@ def main():
               "multi": multi_measurements, "roaring": roaring_measurements,
               "small_map": small_map_measurements, "dmap": dynamic_map_measurements, "fill": fill_measurements,
               "insert": lambda st: insert_measurements(st, capacity_log2=args.capacity_log2,
-                                                       shapes=INSERT_SHAPES if args.sweep else None)}[args.only]
+                                                       shapes=args.sweep)}[args.only]
         print(json.dumps(fn(torch.cuda.current_stream())), flush=True)
     elif args.impl == "reference":
         run_reference(args)
