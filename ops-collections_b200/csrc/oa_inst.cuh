@@ -134,13 +134,17 @@ struct OaImpl {
     static int mark(OaArgs const& a, uint32_t b, void const* pairs, uint32_t n, bool assign, uint8_t* absent,
                     cudaStream_t s)
     {
-        return with_b(b, [&](auto bc) {
-            constexpr int B = decltype(bc)::value;
-            InsOut o{};
-            o.inserted = absent;
-            return assign ? write<B, kInsMarkAssign>(a, pairs, nullptr, n, o, s)
-                          : write<B, kInsMark>(a, pairs, nullptr, n, o, s);
-        });
+        if constexpr (S::is_set) {
+            return fail(B2CO_ELOGIC, "marking is for maps (DynamicMap's submaps)");
+        } else {
+            return with_b(b, [&](auto bc) {
+                constexpr int B = decltype(bc)::value;
+                InsOut o{};
+                o.inserted = absent;
+                return assign ? write<B, kInsMarkAssign>(a, pairs, nullptr, n, o, s)
+                              : write<B, kInsMark>(a, pairs, nullptr, n, o, s);
+            });
+        }
     }
 
     static int assign_if(OaArgs const& a, uint32_t b, void const* pairs, uint8_t const* stencil, uint32_t n,
@@ -252,7 +256,9 @@ struct OaImpl {
     template <int B, int G, int Q, bool C>
     static int find_defer_auto(OaArgs const& a, void const* keys, void* out, uint32_t n, WaitCtl wc, cudaStream_t s)
     {
-        DeferFn const even = a.keep_misses ? k_find_wdefer<S, B, G, Q, C, true, true> : k_find_wdefer<S, B, G, Q, C, true>;
+        DeferFn even = k_find_wdefer<S, B, G, Q, C, true>;
+        if constexpr (!S::is_set)  // DynamicMap's lookups
+            if (a.keep_misses) even = k_find_wdefer<S, B, G, Q, C, true, true>;
         uint64_t const share = (n + defer_warps(even) - 1) / defer_warps(even);
         // (the even deal's kernel for windows of four sectors is the slower one: 1 Mi keys, 300 MB, 29 us against 40)
         uint64_t const whole = SectorWindow<S, B>::NS >= 4 ? kWarpStageKeys / 2 : kWarpStageKeys;
@@ -277,7 +283,9 @@ struct OaImpl {
     static int find_sector(OaArgs const& a, void const* keys, uint8_t const* stencil, void* out, uint32_t n,
                            cudaStream_t s)
     {
-        auto k = a.keep_misses ? k_find_sector<S, B, C, true> : k_find_sector<S, B, C, false>;
+        auto k = k_find_sector<S, B, C, false>;
+        if constexpr (!S::is_set)  // DynamicMap's lookups
+            if (a.keep_misses) k = k_find_sector<S, B, C, true>;
         uint32_t const block = sector_block(n);
         k<<<grid_for((void const*)k, block, n, block), block, 0, s>>>(a, keys, stencil, out, n);
         return check_launch(C ? "contains kernel" : "find kernel");
