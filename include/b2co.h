@@ -233,9 +233,10 @@ int b2co_oa_find_host(b2co_oa_table* table, const void* host_keys, void* host_ou
  * read the second segment only when the first does not end the scan) and the
  * flags below; 0, 0 = library default, chosen by table size and batch: one lane
  * a key for tables of at most 224 MiB (served mostly from L2) with 8- or 16-byte
- * slots and for batches of at most 98,304 keys; else 2 lanes and 1 window up to
- * 320 MiB and for 4-byte slots, 4 lanes and 2 windows above, both
- * B2CO_FIND_DEFERRED.  No reference counterpart. */
+ * slots, for batches of at most 98,304 keys and for bucket size 1; else 2 lanes
+ * and 1 window up to 320 MiB, for 4-byte slots and for large batches on windows
+ * of eight 16-byte slots (Contains on small tables: five), 4 lanes and 2 windows
+ * above, all B2CO_FIND_DEFERRED.  No reference counterpart. */
 #define B2CO_FIND_SEGMENTED 0x100u
 /* OR-ed into keys_per_lane: fetch every first bucket window with one bulk (TMA)
  * copy into shared memory; tables with 16-byte slots only (others ignore it). */
@@ -251,9 +252,9 @@ int b2co_oa_set_find_shape(b2co_oa_table* table, uint32_t lanes_per_key, uint32_
  * depend on it).  lanes_per_key 1 reads a key's window with one lane; 2, 4 or 8
  * read it with a tile of lanes, as many as the window has 32-byte sectors
  * (keys_per_tile, 1, 2 or 4, is accepted and changes nothing).  (0, 0)
- * restores the default: one lane for bucket size 1 and for tables of at most
- * 352 MiB (InsertOrAssign: 256 MiB), whose windows mostly come from L2, a tile
- * above. */
+ * restores the default: one lane for bucket size 1, for batches of at most 65,536
+ * pairs and for tables of at most 352 MiB (InsertOrAssign: 256 MiB), whose windows
+ * mostly come from L2, a tile otherwise. */
 int b2co_oa_set_write_shape(b2co_oa_table* table, uint32_t lanes_per_key, uint32_t keys_per_tile);
 
 /* ===================================================================== */
@@ -295,8 +296,9 @@ int b2co_oa_group_insert_per_table(b2co_oa_group* group, const void* pairs, cons
  * keys in flight per lane group (1, 2 or 4, at most the lanes; above 1 the
  * keys whose first window settles nothing are queued and followed a pass at a
  * time) and threads per block (64, 128 or 256; 0 = 256).  Results do not
- * depend on it.  The default is 1 lane, 1 key, 256 threads.  The lanes-only
- * form sets one key per lane group. */
+ * depend on it.  The default is 1 lane, 1 key, 256 threads; groups of tables of
+ * 320 MB or more (their mean over slots) start with 2 lanes.  The lanes-only form
+ * sets one key per lane group. */
 int b2co_oa_group_set_find_shape(b2co_oa_group* group, uint32_t lanes);
 int b2co_oa_group_set_find_shape_ex(b2co_oa_group* group, uint32_t lanes, uint32_t keys_per_tile, uint32_t block);
 int b2co_oa_group_get_find_shape(const b2co_oa_group* group, uint32_t* lanes, uint32_t* keys_per_tile,

@@ -90,7 +90,8 @@ constexpr int kHllBlock = 1024;
 // fill an SM's 64 warps.  Keys before the first 16-byte boundary (`head`) and
 // after the last whole vector go one per thread.
 //
-// Bound by instruction issue: xxh64's five 64-bit multiplies, and the raises.
+// Issue slots are 66% busy (xxh64's five 64-bit multiplies, and the raises); a warp
+// waits about as long for its keys as for the integer pipes.
 //  * The loop is the same for all lanes of a warp and ends a round with a warp
 //    barrier: lanes that come out of the compare-and-swap loop one by one would
 //    run the keys that follow one by one as well.  (The same loop without the

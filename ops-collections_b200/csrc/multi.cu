@@ -496,8 +496,8 @@ __global__ void __launch_bounds__(kThreads) k_part_starts(Survey* s, uint32_t pa
 // tile's pairs in their partitions in shared memory, sorts the tile by partition
 // there, takes the tile's places with one atomic a partition and writes run
 // after run, so that the pairs of a run leave in whole sectors.  Bound by the
-// block's phases, which wait on one another: 16.8 M pairs of 16 bytes over 4,096
-// partitions, 0.49 GB in 187 us.  Storing every pair to its place without the sort:
+// latency of shared memory within the block's phases (issue slots 22% busy): 16.8 M
+// pairs of 16 bytes over 4,096 partitions, 0.49 GB in 187 us.  Storing every pair to its place without the sort:
 // 274 us (scattered stores run at about 60 G a second).
 constexpr int kRouteThreads = 1024, kRoutePer = 8;
 constexpr uint32_t kRouteTile = kRouteThreads * kRoutePer;
@@ -597,7 +597,7 @@ __global__ void __launch_bounds__(kRouteThreads, 1)
 // of the CSR array.  Every access to memory is a stretch read or written whole, or
 // lands in one that is in L2, where k_run_count, k_run_offsets and k_run_scatter
 // (598, 194 and 821 us for 16.8 M int64 pairs over 4.2 M keys) pay a random access to HBM
-// each.  225 us for them, 0.65 GB; bound by the probing in shared memory.
+// each.  225 us for them, 0.65 GB; bound by the probing in shared memory (L1 82% busy).
 constexpr int kPartThreads = 512;
 template <int KB, int VB>
 __global__ void __launch_bounds__(kPartThreads)
