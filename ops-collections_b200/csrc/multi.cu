@@ -497,8 +497,8 @@ __global__ void __launch_bounds__(kThreads) k_part_starts(Survey* s, uint32_t pa
 // there, takes the tile's places with one atomic a partition and writes run
 // after run, so that the pairs of a run leave in whole sectors.  Bound by the
 // latency of shared memory within the block's phases (issue slots 22% busy): 16.8 M
-// pairs of 16 bytes over 4,096 partitions, 0.49 GB in 187 us.  Storing every pair to its place without the sort:
-// 274 us (scattered stores run at about 60 G a second).
+// pairs of 16 bytes over 4,096 partitions, 0.49 GB in 187 us.  Storing every pair to
+// its place without the sort: 274 us (scattered stores run at about 60 G a second).
 constexpr int kRouteThreads = 1024, kRoutePer = 8;
 constexpr uint32_t kRouteTile = kRouteThreads * kRoutePer;
 template <class Raw>
@@ -669,7 +669,8 @@ __global__ void __launch_bounds__(kPartThreads)
     __syncthreads();
     unsigned long long carry = warp_at[warp];
     uint64_t const out = uint64_t(blockIdx.x) * slots;
-    RunSlot<KB>* const out8 = reinterpret_cast<RunSlot<KB>*>(t.slots) + out;  // put() here costs 8-byte keys 18% of the kernel
+    // 8-byte keys: with put() the compiler keeps fewer registers, and the kernel takes 266 us, not 225
+    RunSlot<KB>* const out8 = reinterpret_cast<RunSlot<KB>*>(t.slots) + out;
     for (uint32_t i = lane; i < share; i += 32) {
         uint32_t const s = first + i, c = counts[s];
         unsigned long long const mine = c ? (1ull << 32) + c : 0;
