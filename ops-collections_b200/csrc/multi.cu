@@ -300,7 +300,7 @@ __device__ __forceinline__ bool find_run(RunTable<KB> const& t, KeyWord<KB> k, R
 {
     out.count = 0;
     if (k == t.empty) return false;
-    return walk_region(t.start(k), t.region, [&](uint64_t s) {
+    return walk_region(uint32_t(t.start(k)), uint32_t(t.region), [&](uint32_t s) {  // at most 2^32 slots
         KeyWord<KB> found;
         uint2 run;
         if constexpr (KB == 8) {

@@ -15,7 +15,11 @@ namespace multi {
 
 // A key's probing goes round the region (a power of two of slots) that it
 // starts in; `region` is the region's size - 1.
-B2CO_PROBE_HD uint64_t next_in_region(uint64_t s, uint64_t region) { return (s & ~region) | ((s + 1) & region); }
+template <class Index>
+B2CO_PROBE_HD Index next_in_region(Index s, Index region)
+{
+    return (s & ~region) | ((s + 1) & region);
+}
 
 // Whether a region with this many keys is too full to be asked: what a build
 // that sized its table by an estimate, or dealt it out by the hash's leading
@@ -28,14 +32,15 @@ enum { kProbeOn = 0, kProbeHit = 1, kProbeMiss = 2 };
 
 // Walks from slot s until look(s) says hit or miss, at most once round the
 // region; whether it was a hit.
-template <class Look>
-B2CO_PROBE_HD bool walk_region(uint64_t s, uint64_t region, Look look)
+template <class Index, class Look>
+B2CO_PROBE_HD bool walk_region(Index start, Index region, Look look)
 {
-    for (uint64_t left = region + 1; left; --left) {
+    Index s = start;
+    do {
         int const what = look(s);
         if (what != kProbeOn) return what == kProbeHit;
         s = next_in_region(s, region);
-    }
+    } while (s != start);
     return false;
 }
 
